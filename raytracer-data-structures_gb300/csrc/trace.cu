@@ -61,48 +61,53 @@ __global__ void __launch_bounds__(kThreads, 10) k_trace_fast(Bvh2View bvh, const
 }
 
 // The FAST walk as persistent warps: a grid that fits on the GPU at once,
-// each warp taking the next 32 rays from a counter (list[1]) until none are
-// left, so no warp idles while the slowest warp of its block finishes.
-// Secondary rays of the 998k-triangle terrain: 3.52 ms against 3.72 ms for
-// one thread per ray in blocks of 128 (blocks of 64: 3.66 ms).  Rays that
+// each warp taking the next rays from a counter (list[1]) until none are
+// left, so no warp idles while the slowest warp of its block finishes.  The
+// rays of a warp share its lanes (walk_warp, trace_device.cuh).  Rays that
 // need the exact box test (a direction component zero or too small for the
 // fused form) are not walked here but appended to list[2..] (count in
 // list[0]) for k_trace_exact, so this kernel carries only the fused walk.
 // UNIT: the LBVH's one-primitive leaves (4-byte stack entries).
+// grab: rays a warp takes at a time (at most 32).
 template <int KIND, bool ANY, bool UNIT>
-__global__ void __launch_bounds__(kThreads, 10) k_trace_warps(Bvh2View bvh, const float4* __restrict__ rays,
+__global__ void __launch_bounds__(kThreads, kWalkBlocks) k_trace_warps(Bvh2View bvh, const float4* __restrict__ rays,
                                                           uint32_t n, float4* __restrict__ hits,
                                                           uint32_t* __restrict__ occ, uint32_t* err,
                                                           const uint32_t* __restrict__ perm,
-                                                          uint32_t* __restrict__ list) {
+                                                          uint32_t* __restrict__ list, uint32_t grab) {
+  __shared__ WarpShare<ANY, false> share[kThreads / 32];
+  WarpShare<ANY, false>& sh = share[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31;
   for (;;) {
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(list + 1, 32u);
+    if (lane == 0) base = atomicAdd(list + 1, grab);
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= n) break;
     const uint32_t i = base + lane;
-    const uint32_t r = (perm && i < n) ? __ldg(perm + i) : i;
-    bool occluded = false;
-    uint32_t visits = 0, tests = 0;
-    if (i < n) {
-      Ray ray = load_ray(rays, r);
-      Closest c = {ray.tmax, kMiss, 0.f, 0.f};
-      const SlabRay sr = slab_ray(ray.o, ray.d);
+    const bool live = lane < grab && i < n;
+    Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
+    SlabRay sr = {};
+    bool walk = live;
+    if (live) {
+      const uint32_t r = perm ? __ldg(perm + i) : i;
+      ray = load_ray(rays, r);
+      sr = slab_ray(ray.o, ray.d);
       if (zero_dir(sr)) {
         list[2 + atomicAdd(list, 1u)] = r;
-      } else {
-        occluded = walk_bvh2_form<KIND, ANY, false, kStackSize, false, UNIT>(bvh, ray, sr, c, visits, tests, err);
-        if (!ANY) store_hit(hits, r, c);
+        walk = false;
       }
     }
-    if (ANY) {
-      if (perm) {
-        if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
-      } else {
-        const uint32_t bits = __ballot_sync(0xffffffffu, occluded);
-        if (lane == 0) occ[base >> 5] = bits;
-      }
+    const bool own = walk;  // this lane's ray is walked here
+    Closest c = {ray.tmax, kMiss, 0.f, 0.f};
+    const bool occluded = walk_warp<KIND, ANY, UNIT, kStackSize, false>(bvh, ray, sr, walk, grab < 32u, c, sh, err);
+    const uint32_t r = (perm && live) ? __ldg(perm + i) : i;
+    if (!ANY) {
+      if (own) store_hit(hits, r, c);
+    } else if (perm || grab < 32u) {
+      if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
+    } else {
+      const uint32_t bits = __ballot_sync(0xffffffffu, occluded);
+      if (lane == 0) occ[base >> 5] = bits;
     }
   }
 }
@@ -880,7 +885,15 @@ void dispatch_bvh2(int traversal, const Bvh2View& v, const float4* rays, uint32_
   } else if (exact) {
     cudaMemsetAsync(exact, 0, 8, s);  // exact-ray count and work counter
     const auto k = v.unit_leaves ? k_trace_warps<KIND, ANY, true> : k_trace_warps<KIND, ANY, false>;
-    k<<<std::min(g, resident_blocks(k)), kThreads, 0, s>>>(v, rays, n, hits, occ, err, perm, exact);
+    // Fewer rays than the resident warps' lanes: fewer rays a warp, halved
+    // while every ray still has a warp to go to, so idle lanes share the work
+    // of few rays at once (1k random rays: 32 a warp 75 us, one a warp 37).
+    const uint32_t blocks = resident_blocks(k);
+    uint32_t grab = 32u;
+    while (grab > 1u && (uint64_t)blocks * (kThreads / 32) * (grab / 2) >= n) grab /= 2;
+    g = (n + grab * (kThreads / 32) - 1) / (grab * (kThreads / 32));
+    if (ANY && !perm && grab < 32u) cudaMemsetAsync(occ, 0, (size_t)((n + 31) / 32) * 4, s);
+    k<<<std::min(g, blocks), kThreads, 0, s>>>(v, rays, n, hits, occ, err, perm, exact, grab);
     count_launch();
     k_trace_exact<KIND, ANY><<<kExactBlocks, kThreads, 0, s>>>(v, rays, exact, hits, occ, err);
   } else {

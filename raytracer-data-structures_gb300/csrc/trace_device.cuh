@@ -377,4 +377,256 @@ __device__ __forceinline__ bool walk_bvh8(const Bvh8View& bvh, const Ray& ray, C
                                           : walk_bvh8_form<KIND, ANY, COUNT, STACK, false>(bvh, ray, c, visits, tests, err);
 }
 
+// ------------------------------------------------- shared lanes of a warp
+// One warp's rays walked by all of its lanes.  Every lane starts with its own
+// ray; a round is at most kWalkChunk node steps a lane, then one leaf test
+// for the lanes that reached a leaf, then a meeting of the warp: lanes whose
+// ray is finished take over the oldest (largest) stacked subtree of lanes
+// that still have some, with a copy of the ray.  The closest-hit rule
+// (smallest t, ties to the smallest id) makes a ray's result independent of
+// which lane tests which subtree and when, so the results are those of the
+// one-lane walk, as long as no box is culled whose primitive is hit at a
+// smaller t than the box is entered at: the slab test's widening covers the
+// rounding of a triangle's t (113M bounce, camera, scanner and random rays
+// walked without any culling gave the culled walk's hits, bit for bit), not
+// that of a small distant sphere's, whose t cancels.  So closest hits on
+// spheres stay with their lane; its order is the one-lane walk's.
+//
+// What it is for: with one lane a ray the warp waits for its longest ray
+// (8.5 of 32 lanes busy on bounce rays), and a ray is one chain of dependent
+// fetches (a launch of few rays lasts as long as its longest chain).  With
+// shared lanes 17 of 32 are busy and the walk is bound by L1 wavefronts (77%
+// of peak; the one-lane walk 48%).  Testing leaves once a round instead of
+// at every step matters as much: a tenth of the visits are leaves, so nearly
+// every step of a full warp paid for a leaf test of one or two lanes.
+// Measured on a GB300 against the one-lane walk (us): 8.3M bounce rays
+// 4371 -> 2631 (in octant order 3332 -> 2738), 1M random rays 620 -> 385
+// (any hit 417 -> 317), 2M bounce rays on a median BVH 1421 -> 768, 115k
+// scanner rays 250 -> 168, 1k random rays 82 -> 37; coherent rays gain
+// nothing: 8.3M camera rays 997 -> 1034, shadow rays 999 -> 1003.
+//
+// kWalkChunk: 2 / 3 / 4 / 6 / 8 node steps a round give 2915 / 2838 / 2853 /
+// 2922 / 3016 us on the ordered bounce rays, and camera rays want 4 or more
+// (1181 / 1087 / 1071 / 1065 / 1067).  kWalkIdle(Any): lanes idle before
+// subtrees move (a move is some 40 instructions of the whole warp, and a far
+// subtree taken early may be one that the nearer hit would have culled):
+// closest hit 1 / 8 / 12 / 16 / 24 give 417 / 397 / 387 / 385 / 397 us on the
+// random rays and 2853 / 2826 / 2833 / 2875 / 3076 on the bounce rays; any
+// hit, where every taken subtree of a ray that is hit is wasted, 452 / 432 /
+// 419 / 403 / 374.  Rays kept in shared memory, a sentinel entry instead of
+// the two stack bounds and a forced convergence at every step were all
+// slower (up to 1.4x).
+constexpr int kWalkChunk = 4;
+constexpr int kWalkIdle = 12;
+constexpr int kWalkIdleAny = 20;
+constexpr int kWalkBlocks = 10;  // blocks of 128 per SM (48 registers); 8 / 9 / 10: 2920 / 2817 / 2738 us (bounce)
+
+template <bool ANY, bool MANY>
+struct WarpShare {
+  uint32_t give[32];           // a meeting's donors, by rank
+  const float4* prims[MANY ? 32 : 1];    // MANY: the structure of each ray
+  const uint32_t* order[MANY ? 32 : 1];
+  unsigned long long key[ANY ? 1 : 32];  // best hit per ray: (order-preserving bits of t + 0, prim)
+  float t[ANY ? 1 : 32];
+  float2 uv[ANY ? 1 : 32];
+};
+
+__device__ __forceinline__ float from_order_key(uint32_t u) {
+  return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
+}
+__device__ __forceinline__ unsigned long long hit_key(const Closest& c) {
+  return ((unsigned long long)order_key(__fadd_rn(c.t, 0.f)) << 32) | c.prim;  // -0 and +0 tie
+}
+
+// slab_box<false> with each axis' two plane distances from one packed
+// multiply-add (camera rays 1073 -> 1034 us, bounce rays 2769 -> 2738).
+__device__ __forceinline__ void plane_pair(float lo, float hi, float inv, float noi, float& t0, float& t1) {
+  asm("{\n\t.reg .b64 p, i, n, r;\n\t"
+      "mov.b64 p, {%2, %3};\n\tmov.b64 i, {%4, %4};\n\tmov.b64 n, {%5, %5};\n\t"
+      "fma.rn.f32x2 r, p, i, n;\n\tmov.b64 {%0, %1}, r;\n\t}"
+      : "=f"(t0), "=f"(t1)
+      : "f"(lo), "f"(hi), "f"(inv), "f"(noi));
+}
+__device__ __forceinline__ bool slab_pairs(const SlabRay& r, float lx, float hx, float ly, float hy, float lz, float hz,
+                                           float tmin, float tfar, float& tnear) {
+  float tx0, tx1, ty0, ty1, tz0, tz1;
+  plane_pair(lx, hx, r.inv.x, r.noi.x, tx0, tx1);
+  plane_pair(ly, hy, r.inv.y, r.noi.y, ty0, ty1);
+  plane_pair(lz, hz, r.inv.z, r.noi.z, tz0, tz1);
+  tnear = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), tmin));
+  const float tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fminf(fmaxf(tz0, tz1), tfar));
+  return tnear <= __fmaf_rn(tf, kWiden, r.eps);
+}
+
+// The warp's 32 lanes call it together, each with its ray (walk: it has one,
+// and not one for the exact box test).  c starts as the ray's (tmax, miss)
+// and returns its closest hit; any hit returns whether the lane's ray is
+// occluded.  eager: lanes start without a ray (fewer than 32 rays), so
+// subtrees move as soon as a lane is idle.  MANY: the lanes' rays may belong
+// to different structures (bvh is the lane's own).
+template <int KIND, bool ANY, bool UNIT, int STACK, bool MANY>
+__device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay sr, bool walk, bool eager, Closest& c,
+                                          WarpShare<ANY, MANY>& sh, uint32_t* err) {
+  constexpr bool kShare = ANY || KIND == kTriangles;
+  const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  typename std::conditional<UNIT, int, int2>::type stack[STACK];
+  int sp = 0, bot = 0;  // entries [bot, sp): lanes that take over work take the entry at bot
+  int cur = bvh.n_internal ? 0 : -1;
+  int cnt = bvh.n_internal ? 0 : (int)bvh.n_slots;
+  const float4* nodes = bvh.nodes;
+  uint32_t home = lane;  // the lane whose ray this lane works on
+  uint32_t found = 0;    // any hit: the rays that are done (one bit each)
+  bool shared = false;   // some lane has taken over another's subtree (warp-uniform)
+  // A ray's walk visits every node and leaf at most once, and a lane that
+  // takes over a subtree continues its donor's walk: whatever lane is busy at
+  // a meeting, at least one node or leaf of its ray lies behind it for every
+  // meeting so far.
+  uint32_t max_meetings = 2u * (bvh.n_internal + bvh.n_slots) + 8u;
+  if (MANY) {
+    max_meetings = __reduce_max_sync(0xffffffffu, walk ? max_meetings : 0u);
+    sh.prims[MANY ? lane : 0] = bvh.prims;
+    sh.order[MANY ? lane : 0] = bvh.order;
+    __syncwarp();
+  }
+  uint32_t meetings = 0;
+  if (walk) {
+    float tn;
+    const float* rb = bvh.root;
+    walk = slab_box<false>(sr, ray.o, rb[0], rb[3], rb[1], rb[4], rb[2], rb[5], ray.tmin, ray.tmax, tn);
+  }
+  auto pop = [&]() {
+    if (sp == bot) {
+      walk = false;
+    } else if constexpr (UNIT) {
+      cur = stack[--sp];
+    } else {
+      const int2 e = stack[--sp];
+      cur = e.x;
+      cnt = e.y;
+    }
+  };
+  for (;;) {
+#pragma unroll 1
+    for (int k = 0; k < kWalkChunk && walk && cur >= 0; ++k) {
+      float4 a, b, z;
+      int4 l;
+      load_node(nodes + 4 * (size_t)cur, a, b, z, l);
+      const float tfar = ANY ? ray.tmax : c.t;
+      float tl, tr;
+      const bool hl = slab_pairs(sr, a.x, a.y, a.z, a.w, z.x, z.y, ray.tmin, tfar, tl);
+      const bool hr = slab_pairs(sr, b.x, b.y, b.z, b.w, z.z, z.w, ray.tmin, tfar, tr);
+      if (hl || hr) {
+        const bool left = hl && !(hr && tr < tl);
+        cur = left ? l.x : l.y;
+        if (!UNIT) cnt = left ? l.z : l.w;
+        if (hl && hr) {
+          if (sp >= STACK) {
+            atomicOr(err, kErrStackOverflow);
+            walk = false;
+            break;
+          }
+          if constexpr (UNIT) stack[sp++] = left ? l.y : l.x;
+          else stack[sp++] = left ? make_int2(l.y, l.w) : make_int2(l.x, l.z);
+        }
+      } else {
+        pop();
+      }
+    }
+    bool hit = false;  // any hit: the ray is occluded; closest hit: c is a new one
+    if (walk && cur < 0) {
+      if (UNIT) cnt = 1;
+      const uint32_t had = c.prim;
+      const float had_t = c.t;
+      hit = test_leaf<KIND, ANY, false>(MANY ? sh.prims[MANY ? home : 0] : bvh.prims,
+                                        MANY ? sh.order[MANY ? home : 0] : bvh.order, (uint32_t)(~cur), cnt, ray, c);
+      if (!ANY) hit = c.prim != had || c.t != had_t;
+      pop();
+    }
+    __syncwarp();
+    if (__any_sync(0xffffffffu, hit)) {
+      if constexpr (ANY) {
+        found |= __reduce_or_sync(0xffffffffu, hit ? 1u << home : 0u);
+        if ((found >> home) & 1u) walk = false;
+      } else if (shared) {
+        const unsigned long long mine = hit_key(c);
+        if (hit) atomicMin(&sh.key[home], mine);
+        __syncwarp();
+        const unsigned long long best = sh.key[home];
+        if (hit && best == mine) {  // equal keys: the same primitive, so the same t, u, v
+          sh.t[home] = c.t;
+          sh.uv[home] = make_float2(c.u, c.v);
+        }
+        c.t = from_order_key((uint32_t)(best >> 32));
+        c.prim = (uint32_t)best;
+      }
+    }
+    const uint32_t busy = __ballot_sync(0xffffffffu, walk);
+    if (busy == 0u) break;
+    if (++meetings > max_meetings) {
+      if (lane == 0) atomicOr(err, kErrCorrupt);
+      break;
+    }
+    if (!kShare || 32 - __popc(busy) < (eager ? 1 : ANY ? kWalkIdleAny : kWalkIdle)) continue;
+    const uint32_t donors = __ballot_sync(0xffffffffu, walk && sp > bot);
+    if (donors == 0u) continue;
+    if constexpr (!ANY) {
+      if (!shared) {  // every lane still holds its own ray
+        sh.key[lane] = hit_key(c);
+        sh.t[lane] = c.t;
+        sh.uv[lane] = make_float2(c.u, c.v);
+      }
+    }
+    shared = true;
+    const int pairs = min(__popc(donors), 32 - __popc(busy));
+    const int rank = __popc((walk ? donors : ~busy) & below);
+    int give = 0, give_cnt = 0;
+    if (walk && sp > bot && rank < pairs) {
+      if constexpr (UNIT) {
+        give = stack[bot++];
+      } else {
+        const int2 e = stack[bot++];
+        give = e.x;
+        give_cnt = e.y;
+      }
+      sh.give[rank] = lane;
+    }
+    __syncwarp();
+    const bool take = !walk && rank < pairs;
+    const int src = take ? (int)sh.give[rank] : (int)lane;
+    auto from = [&](float& x) { x = __shfl_sync(0xffffffffu, x, src); };
+    from(ray.o.x); from(ray.o.y); from(ray.o.z);
+    from(ray.d.x); from(ray.d.y); from(ray.d.z);
+    from(ray.tmin);
+    from(sr.inv.x); from(sr.inv.y); from(sr.inv.z);
+    from(sr.noi.x); from(sr.noi.y); from(sr.noi.z);
+    from(sr.eps);
+    home = __shfl_sync(0xffffffffu, home, src);
+    if (ANY) {
+      from(ray.tmax);
+    } else {
+      from(c.t);
+      c.prim = __shfl_sync(0xffffffffu, c.prim, src);
+    }
+    if (MANY)
+      nodes = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(nodes), src));
+    give = __shfl_sync(0xffffffffu, give, src);
+    if (!UNIT) give_cnt = __shfl_sync(0xffffffffu, give_cnt, src);
+    if (take) {
+      walk = true;
+      cur = give;
+      cnt = give_cnt;
+      sp = bot = 0;
+    }
+    __syncwarp();
+  }
+  if constexpr (!ANY) {
+    if (shared) {
+      const float2 uv = sh.uv[lane];  // written before the last meeting's ballot
+      c = {sh.t[lane], (uint32_t)sh.key[lane], uv.x, uv.y};
+      __syncwarp();
+    }
+  }
+  return (found >> lane) & 1u;
+}
+
 }  // namespace rq
