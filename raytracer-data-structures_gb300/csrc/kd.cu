@@ -27,7 +27,7 @@
 #include <vector>
 
 #include "rq_build.hpp"
-#include "rq_device.cuh"
+#include "trace_device.cuh"
 
 namespace rq {
 namespace {
@@ -766,6 +766,286 @@ __global__ void __launch_bounds__(128) k_trace_kd_warps(KdView kd, uint32_t n_no
   }
 }
 
+// The FAST walk as persistent warps whose rays share the warp's lanes, as
+// walk_warp (trace_device.cuh) does for the BVH: a round is at most kKdChunk
+// interior nodes a lane, then the leaves that lanes reached, then a meeting
+// where idle lanes take over the last todo entry (the farthest subtree) of
+// busy ones.
+//
+// kdtreeIntersect's answer depends on its order (the first closest hit wins,
+// and the walk ends at the first entry that begins behind the best hit), so
+// the shared walk keeps track of it:
+//  * every piece of a ray's walk carries its place in that order: a piece
+//    owns [lo, hi] of the numbers, what is taken from it gets the upper half
+//    (it comes later, but before what was taken earlier), and equal t go to
+//    the smaller lo (sh.key = (t, lo));
+//  * a hit found before its leaf's interval begins (t < tMin: a primitive
+//    that reaches into nearer leaves) belongs to an earlier leaf.  The
+//    one-lane walk finds it there, or ends before it gets here, unless
+//    rounding made it skip the earlier leaf.  The shared walk only notes the
+//    smallest such t (sh.doubt), and a ray whose noted t is smaller than its
+//    best hit is walked again by its own lane alone.
+// Every other hit lies in its own interval, so the one-lane walk reaches it
+// whenever it is the answer, and what a best hit prunes here begins behind
+// it in the one-lane walk's order too.
+//
+// Rays sit in shared memory (a piece moves without its ray; the split axis
+// indexes them), todo entries are 8 bytes (an entry ends where the one below
+// it begins, the last one at t_end).  The node loop converges at every step:
+// left to itself (a loop a lane leaves at its leaf) it took 2080-3200 us
+// where this takes 1950.
+// Measured against the one-lane walk (us): 1023 random rays 194 -> 60, 300k
+// random rays 377 -> 279 (any hit 347 -> 209), 307k camera rays 260 -> 215,
+// their shadow rays 348 -> 257, 2M bounce rays 2020 -> 1950 (lanes per
+// instruction 5.4 -> 10.9, but leaves of unequal length now take most of the
+// issue slots); 2M coherent shadow rays lose, 697 -> 778 (300k: 260 -> 219),
+// so any-hit launches over a million rays walk one ray a lane.
+constexpr int kKdChunk = 8;  // 2 / 3 / 4 / 8 / 16: 2352 / 2126 / 2025 / 1960 / 2031 us
+constexpr int kKdIdle = 8;   // lanes idle before pieces move
+constexpr uint32_t kKdSharedAnyMax = 1u << 20;  // longer any-hit launches walk one ray a lane (dispatch_kd)
+
+__device__ __forceinline__ int2 load_kd(const int4* __restrict__ nodes, int node) {
+  return __ldg(reinterpret_cast<const int2*>(nodes + node));
+}
+
+template <bool ANY>
+struct KdShare {
+  float o[3][32], inv[3][32], d[3][32], tmin[32], tmax[32];
+  uint32_t give[32];
+  unsigned long long key[ANY ? 1 : 32];  // best hit per ray: (order-preserving bits of t + 0, place)
+  uint32_t doubt[ANY ? 1 : 32];          // smallest t found before its leaf, order-preserving bits
+  uint32_t prim[ANY ? 1 : 32];
+  float t[ANY ? 1 : 32];
+  float2 uv[ANY ? 1 : 32];
+};
+
+template <int KIND, bool ANY>
+__global__ void __launch_bounds__(128, ANY ? 9 : 8) k_trace_kd_shared(KdView kd, uint32_t n_nodes,
+                                                                   const float4* __restrict__ rays, uint32_t n,
+                                                                   float4* __restrict__ hits,
+                                                                   uint32_t* __restrict__ occ, uint32_t* err,
+                                                                   uint32_t* work, uint32_t grab) {
+  __shared__ KdShare<ANY> share[4];
+  KdShare<ANY>& sh = share[threadIdx.x >> 5];
+  const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  const uint32_t limit = 2u * n_nodes + 8u;  // meetings: a piece has a node of its ray behind it for every one
+  int2 todo[kStackSize];                     // (node, bits of tMin)
+  for (;;) {
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(work, grab);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (base >= n) break;
+    const uint32_t r = base + lane;
+    const bool own = lane < grab && r < n;
+    float first = 0.f, last = 0.f;  // the ray's interval in the root box
+    bool start = false;
+    __syncwarp();
+    if (own) {
+      const float4 ra = __ldcs(rays + 2 * (size_t)r), rb = __ldcs(rays + 2 * (size_t)r + 1);
+      const F3 o = {ra.x, ra.y, ra.z}, d = {rb.x, rb.y, rb.z};
+      const SlabRay sr = slab_ray(o, d);
+      const float* R = kd.root;
+      if (zero_dir(sr)) {  // the exact box test (rq_device.cuh)
+        start = slab_box<true>(sr, o, R[0], R[3], R[1], R[4], R[2], R[5], ra.w, rb.w, first);
+        last = __fmaf_rn(slab_exit<true>(sr, o, R[0], R[3], R[1], R[4], R[2], R[5], rb.w), kWidenExact, sr.eps);
+      } else {
+        start = slab_box<false>(sr, o, R[0], R[3], R[1], R[4], R[2], R[5], ra.w, rb.w, first);
+        last = __fmaf_rn(slab_exit<false>(sr, o, R[0], R[3], R[1], R[4], R[2], R[5], rb.w), kWiden, sr.eps);
+      }
+      sh.o[0][lane] = o.x; sh.o[1][lane] = o.y; sh.o[2][lane] = o.z;
+      sh.inv[0][lane] = sr.inv.x; sh.inv[1][lane] = sr.inv.y; sh.inv[2][lane] = sr.inv.z;
+      sh.d[0][lane] = d.x; sh.d[1][lane] = d.y; sh.d[2][lane] = d.z;
+      sh.tmin[lane] = ra.w;
+      sh.tmax[lane] = rb.w;
+    }
+    __syncwarp();
+    uint32_t found = 0;
+    bool open = own;  // the ray's answer is not stored yet
+    for (int pass = 0; pass < 2; ++pass) {  // second pass: rays in doubt, one lane each
+      uint32_t home = lane, lo = 1u, hi = 0xFFFFFFFFu, place = 0u;  // place: the best hit's
+      int node = 0, tp = 0, bot = 0;
+      int2 w = load_kd(kd.nodes, 0);  // the node's first two words
+      float tMin = first, tMax = last, t_end = last;
+      bool walk = start, shared = false;
+      uint32_t meetings = 0;
+      float best = own ? sh.tmax[lane] : 0.f, bu = 0.f, bv = 0.f;  // any hit: best stays the ray's end
+      uint32_t bprim = kMiss;
+      if (best < tMin) walk = false;
+      for (;;) {
+#pragma unroll 1
+        for (int k = 0; k < kKdChunk; ++k) {
+          if (walk && (w.y & 3) != 3) {
+          const int axis = w.y & 3;
+          const float split = __int_as_float(w.x), oa = sh.o[axis][home];
+          const float tPlane = __fmul_rn(__fsub_rn(split, oa), sh.inv[axis][home]);
+          const bool belowFirst = (oa < split) || (oa == split && sh.d[axis][home] <= 0.f);
+          const int above = w.y >> 2;
+          const int near = belowFirst ? node + 1 : above, far = belowFirst ? above : node + 1;
+          const bool skip_far = tPlane > tMax || tPlane <= 0.f, skip_near = !skip_far && tPlane < tMin;
+          node = skip_near ? far : near;
+          if (!skip_far && !skip_near) {
+            if (tp >= kStackSize) {
+              atomicOr(err, kErrStackOverflow);
+              walk = false;
+            } else {
+              todo[tp++] = make_int2(far, __float_as_int(tPlane));
+              tMax = tPlane;
+            }
+          }
+          w = load_kd(kd.nodes, node);
+          }
+          __syncwarp();
+        }
+        bool hit = false, doubt = false;
+        float doubt_t = 0.f;
+        if (walk && (w.y & 3) == 3) {
+          const int leaf_n = w.y >> 2;
+          const F3 o = {sh.o[0][home], sh.o[1][home], sh.o[2][home]}, d = {sh.d[0][home], sh.d[1][home], sh.d[2][home]};
+          const float rtmin = sh.tmin[home];
+          for (int i = 0; i < leaf_n; ++i) {
+            const uint32_t id = (uint32_t)(leaf_n == 1 ? w.x : __ldg(kd.prim_idx + w.x + i));
+            // equal t: only over a hit from later in the order
+            const float bound = !ANY && place > lo ? nextafterf(best, __int_as_float(0x7F800000)) : best;
+            float t, u = 0.f, v = 0.f;
+            bool ok;
+            if (KIND == kTriangles) {
+              const float4* q = kd.prims + 3 * (size_t)id;
+              ok = tri_mt(__ldg(q), __ldg(q + 1), __ldg(q + 2), o, d, rtmin, bound, t, u, v);
+            } else {
+              ok = sphere_closest(__ldg(kd.prims + id), o, d, rtmin, bound, false, t);
+            }
+            if (!ok) continue;
+            if (ANY) {
+              hit = true;
+              break;
+            }
+            if (shared && t < tMin) {  // an earlier leaf's
+              doubt_t = doubt ? fminf(doubt_t, t) : t;
+              doubt = true;
+              continue;
+            }
+            best = t; bprim = id; bu = u; bv = v;
+            place = shared ? lo : 0u;
+            hit = true;
+          }
+          if (tp > bot) {
+            const int2 e = todo[--tp];
+            node = e.x;
+            w = load_kd(kd.nodes, node);
+            tMin = __int_as_float(e.y);
+            tMax = tp > bot ? __int_as_float(todo[tp - 1].y) : t_end;
+            if (best < tMin) walk = false;  // this entry and those below it begin behind the best hit
+          } else {
+            walk = false;
+          }
+        }
+        __syncwarp();
+        if constexpr (ANY) {
+          if (__any_sync(0xffffffffu, hit)) {
+            found |= __reduce_or_sync(0xffffffffu, hit ? 1u << home : 0u);
+            if ((found >> home) & 1u) walk = false;
+          }
+        } else if (shared && __any_sync(0xffffffffu, hit || doubt)) {
+          const unsigned long long mine = ((unsigned long long)order_key(__fadd_rn(best, 0.f)) << 32) | place;
+          if (hit) atomicMin(&sh.key[home], mine);
+          if (doubt) atomicMin(&sh.doubt[home], order_key(doubt_t));
+          __syncwarp();
+          const unsigned long long now = sh.key[home];
+          if (hit && now == mine) {  // one piece, one t: one lane
+            sh.t[home] = best;
+            sh.prim[home] = bprim;
+            sh.uv[home] = make_float2(bu, bv);
+          }
+          best = from_order_key((uint32_t)(now >> 32));
+          place = (uint32_t)now;
+        }
+        const uint32_t busy = __ballot_sync(0xffffffffu, walk);
+        if (busy == 0u) break;
+        if (++meetings > limit) {
+          if (lane == 0) atomicOr(err, kErrCorrupt);
+          break;
+        }
+        if (pass || 32 - __popc(busy) < (grab < 32u ? 1 : kKdIdle)) continue;
+        const bool can = walk && tp > bot && hi - lo >= 2u;
+        const uint32_t donors = __ballot_sync(0xffffffffu, can);
+        if (donors == 0u) continue;
+        if constexpr (!ANY) {
+          if (!shared) {  // every lane still holds its own ray
+            sh.key[lane] = (unsigned long long)order_key(__fadd_rn(best, 0.f)) << 32;  // place 0: before every piece
+            sh.doubt[lane] = 0xFFFFFFFFu;
+            sh.t[lane] = best;
+            sh.prim[lane] = bprim;
+            sh.uv[lane] = make_float2(bu, bv);
+          }
+        }
+        shared = true;
+        const int pairs = min(__popc(donors), 32 - __popc(busy));
+        const int rank = __popc((walk ? donors : ~busy) & below);
+        int2 give = make_int2(0, 0);
+        float give_end = 0.f;
+        uint32_t give_lo = 0, give_hi = 0;
+        if (can && rank < pairs) {
+          give = todo[bot++];
+          give_end = t_end;
+          t_end = __int_as_float(give.y);
+          give_lo = lo + (hi - lo) / 2 + 1u;
+          give_hi = hi;
+          hi = give_lo - 1u;
+          sh.give[rank] = lane;
+        }
+        __syncwarp();
+        const bool take = !walk && rank < pairs;
+        const int src = take ? (int)sh.give[rank] : (int)lane;
+        const uint32_t new_home = __shfl_sync(0xffffffffu, home, src);
+        give.x = __shfl_sync(0xffffffffu, give.x, src);
+        give.y = __shfl_sync(0xffffffffu, give.y, src);
+        give_end = __shfl_sync(0xffffffffu, give_end, src);
+        give_lo = __shfl_sync(0xffffffffu, give_lo, src);
+        give_hi = __shfl_sync(0xffffffffu, give_hi, src);
+        const float new_best = __shfl_sync(0xffffffffu, best, src);
+        const uint32_t new_place = __shfl_sync(0xffffffffu, place, src);
+        if (take) {
+          home = new_home;
+          best = new_best;
+          place = new_place;
+          lo = give_lo;
+          hi = give_hi;
+          node = give.x;
+          tMin = __int_as_float(give.y);
+          tMax = t_end = give_end;
+          tp = bot = 0;
+          w = load_kd(kd.nodes, node);
+          walk = !(best < tMin);
+        }
+        __syncwarp();
+      }
+      if constexpr (!ANY) {
+        bool again = false;
+        if (shared) {
+          const float2 uv = sh.uv[lane];  // written before the last meeting's ballot
+          best = sh.t[lane];
+          bprim = sh.prim[lane];
+          bu = uv.x;
+          bv = uv.y;
+          again = open && sh.doubt[lane] < (uint32_t)(sh.key[lane] >> 32);
+        }
+        if (open && !again) __stcs(hits + r, make_float4(best, __uint_as_float(bprim), bu, bv));
+        open = start = again;
+      }
+      if (ANY || !__any_sync(0xffffffffu, open)) break;
+    }
+    if constexpr (ANY) {
+      const bool occluded = (found >> lane) & 1u;
+      if (grab < 32u) {
+        if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
+      } else {
+        const uint32_t bits = __ballot_sync(0xffffffffu, occluded);
+        if (lane == 0) occ[base >> 5] = bits;
+      }
+    }
+  }
+}
+
 template <typename K>
 uint32_t kd_resident_blocks(K k) {
   int per_sm = 0, dev = 0, sms = 0;
@@ -782,8 +1062,18 @@ void dispatch_kd(int traversal, const KdView& v, uint32_t n_nodes, const float4*
   const unsigned g = (n + 127) / 128;
   if (work) {
     cudaMemsetAsync(work, 0, 4, s);
-    const auto k = traversal == RQ_TRAVERSAL_REFERENCE ? k_trace_kd_warps<KIND, ANY, true> : k_trace_kd_warps<KIND, ANY, false>;
-    k<<<std::min(g, kd_resident_blocks(k)), 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work);
+    if (traversal == RQ_TRAVERSAL_REFERENCE || (ANY && n > kKdSharedAnyMax)) {
+      const auto k = traversal == RQ_TRAVERSAL_REFERENCE ? k_trace_kd_warps<KIND, ANY, true> : k_trace_kd_warps<KIND, ANY, false>;
+      k<<<std::min(g, kd_resident_blocks(k)), 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work);
+      return;
+    }
+    // fewer rays a warp when there are fewer rays than resident lanes, as for the BVH (trace.cu)
+    const auto k = k_trace_kd_shared<KIND, ANY>;
+    const uint32_t blocks = kd_resident_blocks(k);
+    uint32_t grab = 32u;
+    while (grab > 1u && (uint64_t)blocks * 4 * (grab / 2) >= n) grab /= 2;
+    if (ANY && grab < 32u) cudaMemsetAsync(occ, 0, (size_t)((n + 31) / 32) * 4, s);
+    k<<<std::min((n + 4 * grab - 1) / (4 * grab), blocks), 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work, grab);
   } else if (traversal == RQ_TRAVERSAL_REFERENCE) {
     k_trace_kd<KIND, ANY, true><<<g, 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err);
   } else {

@@ -85,3 +85,47 @@ def test_shared_lanes_many_structures(engine, oracle, rqm, terrain):
         occ = oracle.trace_bvh2(oracle.TRIANGLES, oracle.FAST, oracle.ANY, tree, prims, rays[k])
         assert np.array_equal(_u32(hits[offs[k]:offs[k + 1]]), _u32(want)), k
         assert np.array_equal(bits[offs[k]:offs[k + 1]], occ), k
+
+
+def _kd_check(engine, oracle, rqm, kind, scene, prims, rays):
+    acc = engine.build(scene, rqm.KDTREE)
+    nodes, pidx, root, _ = engine.export_kd(acc)
+    kd = oracle.Kd(nodes, pidx, root)
+    want = oracle.trace_kd(kind, oracle.FAST, oracle.CLOSEST, kd, prims, rays)
+    occ = oracle.trace_kd(kind, oracle.FAST, oracle.ANY, kd, prims, rays)
+    assert np.array_equal(_u32(engine.trace_closest(acc, rays)), _u32(want))
+    assert np.array_equal(rqm.unpack_bits(engine.trace_any(acc, rays), len(rays)), occ)
+    return want
+
+
+@pytest.mark.parametrize("n_rays", [1, 33, 900, 50_000, 250_003])
+def test_shared_lanes_kd(engine, oracle, rqm, terrain, n_rays):
+    """The first closest hit in the walk's order, whichever lane finds it."""
+    v, f = terrain
+    prims, _, _ = oracle.tri_prims(v, f)
+    _kd_check(engine, oracle, rqm, oracle.TRIANGLES, engine.scene_triangles(v, f), prims, _grazing(n_rays, 80 + n_rays))
+
+
+def test_shared_lanes_kd_any_hit_over_the_shared_limit(engine, oracle, rqm, terrain):
+    """One ray a lane from 2^20 rays on: the same bits on both sides of the line."""
+    v, f = terrain
+    prims, _, _ = oracle.tri_prims(v, f)
+    acc = engine.build(engine.scene_triangles(v, f), rqm.KDTREE)
+    rays = _grazing((1 << 20) + 33, 7)
+    bits = rqm.unpack_bits(engine.trace_any(acc, rays), len(rays))
+    below = rqm.unpack_bits(engine.trace_any(acc, rays[:1 << 20]), 1 << 20)
+    assert np.array_equal(bits[:1 << 20], below)
+
+
+@pytest.mark.parametrize("n_rays", [700, 100_003])
+def test_shared_lanes_kd_small_distant_spheres(engine, oracle, rqm, n_rays):
+    """Spheres whose hit distances cancel: hits before their leaf's interval, equal distances, rays in doubt."""
+    rng = np.random.default_rng(9)
+    p = rng.normal(size=(5000, 3))
+    p /= np.linalg.norm(p, axis=1, keepdims=True)
+    sph = np.concatenate([p * 3.6 + np.array([-2.0, 5.0, -58.0]), np.full((5000, 1), 0.05)], 1).astype(np.float32)
+    t = p[rng.integers(0, 5000, n_rays)] * rng.uniform(0.2, 1.02, (n_rays, 1)) * 3.6 + np.array([-2.0, 5.0, -58.0])
+    d = t / np.linalg.norm(t, axis=1, keepdims=True)
+    rays = scenes._rays(np.zeros((n_rays, 3), np.float32), d.astype(np.float32))
+    want = _kd_check(engine, oracle, rqm, oracle.SPHERES, engine.scene_spheres(sph), sph, rays)
+    assert (want["prim"] != rqm.MISS).mean() > 0.2
