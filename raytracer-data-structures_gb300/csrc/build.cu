@@ -1,6 +1,7 @@
 // Build orchestration: the dataStructure switch of main() (main.cpp:791-843)
 // over the engine's kernels, the LBVH pipeline, query dispatch and
 // device-side input validation.
+#include <algorithm>
 #include <atomic>
 
 #include "rq_build.hpp"
@@ -54,18 +55,26 @@ static size_t zero_words(uint32_t n, int passes) {
 }
 
 BuildResult sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, int passes, bool compute_hist,
-                       BuildScratch& sc, uint32_t* err, cudaStream_t st) {
-  if (n <= 1) return {};
-  RQ_B(sc.keys_alt.ensure((size_t)n * 4), "sort scratch");
-  RQ_B(sc.vals_alt.ensure((size_t)n * 4), "sort scratch");
+                       BuildScratch& sc, uint32_t* err, cudaStream_t st, uint32_t count, size_t stride, bool identity) {
+  if (n <= 1) {
+    if (n == 1 && identity)
+      for (uint32_t c = 0; c < count; ++c) RQ_B(cudaMemsetAsync(vals + c * stride, 0, 4, st), "memset");
+    return {};
+  }
+  const size_t all = (size_t)(count - 1) * stride + n;
+  RQ_B(sc.keys_alt.ensure(all * 4), "sort scratch");
+  RQ_B(sc.vals_alt.ensure(all * 4), "sort scratch");
+  // [hist][counters][look-back status], each for every sort
+  const size_t head = (size_t)count * (kSortHistWords + kSortCounterWords);
   if (compute_hist) {
-    RQ_B(sc.zero.ensure(zero_words(n, passes) * 4), "sort scratch");
-    RQ_B(cudaMemsetAsync(sc.zero.p, 0, (1024 + 16 + sort_status_words(n, passes)) * 4, st), "memset");
-    launch_histogram(keys, n, passes, sc.zero.as<uint32_t>(), st);
+    const size_t words = head + (size_t)count * sort_status_words(n, passes);
+    RQ_B(sc.zero.ensure(std::max(words, zero_words(n, passes)) * 4), "sort scratch");
+    RQ_B(cudaMemsetAsync(sc.zero.p, 0, words * 4, st), "memset");
+    launch_histogram(keys, n, passes, sc.zero.as<uint32_t>(), st, count, stride);
   }
   uint32_t* z = sc.zero.as<uint32_t>();
-  SortScratch s{sc.keys_alt.as<uint32_t>(), sc.vals_alt.as<uint32_t>(), z, z + 1040, z + 1024, sc.stall};
-  launch_onesweep(keys, vals, n, passes, s, err, st);
+  SortScratch s{sc.keys_alt.as<uint32_t>(), sc.vals_alt.as<uint32_t>(), z, z + head, z + (size_t)count * kSortHistWords, sc.stall};
+  launch_onesweep(keys, vals, n, passes, s, err, st, count, stride, identity);
   RQ_B(cudaGetLastError(), "radix sort launch");
   return {};
 }
@@ -125,9 +134,9 @@ static BuildResult build_lbvh(const SceneView& s, const rq_settings_t& cfg, Acce
   RQ_B(cudaMemsetAsync(z, 0, zero_words(n, kSortPasses) * 4, st), "memset");
   uint32_t* codes = a.codes.as<uint32_t>();
   uint32_t* order = a.order.as<uint32_t>();
-  BuildResult r = morton_codes(s, cfg.morton, codes, order, z, sc, st);
+  BuildResult r = morton_codes(s, cfg.morton, codes, nullptr, z, sc, st);
   if (!r.ok()) return r;
-  r = sort_pairs(codes, order, n, kSortPasses, false, sc, err, st);
+  r = sort_pairs(codes, order, n, kSortPasses, false, sc, err, st, 1, 0, true);
   if (!r.ok()) return r;
   uint32_t* flags = z + 1040 + sort_status_words(n, kSortPasses);
   uint32_t* mk = sc.mark.as<uint32_t>();

@@ -1245,20 +1245,22 @@ BuildResult build_kd_tree(const SceneView& s, int max_depth_cfg, AccelBuffers& a
   // start-first, then by primitive id)
   const uint32_t E0 = 2 * n;
   KD_TRY(sc.keys.ensure((size_t)E0 * kEdgeWords * 4 + 64), "KD edges");
-  KD_TRY(sc.vals.ensure((size_t)E0 * 2 * 4 + 64), "KD edges");
+  KD_TRY(sc.vals.ensure((size_t)E0 * 6 * 4 + 64), "KD edges");
   EdgeLists el{sc.keys.as<uint32_t>(), (size_t)E0};
   {
-    const size_t zwords = 1024 + 16 + sort_status_words(E0, 4);
+    // the three lists in one set of launches
+    const size_t head = 3 * (kSortHistWords + kSortCounterWords), zwords = head + 3 * sort_status_words(E0, 4);
     KD_TRY(sc.m4.ensure(zwords * 4 + 64), "KD sort");
     uint32_t* zero = sc.m4.as<uint32_t>();
-    SortScratch ss{sc.vals.as<uint32_t>(), sc.vals.as<uint32_t>() + E0, zero, zero + 1024 + 16, zero + 1024};
+    uint32_t* alt = sc.vals.as<uint32_t>();
+    SortScratch ss{alt, alt + 3 * (size_t)E0, zero, zero + head, zero + 3 * kSortHistWords};
+    KD_TRY(cudaMemsetAsync(zero, 0, zwords * 4, st), "KD sort");
     for (int ax = 0; ax < 3; ++ax) {
       count_launch();
       k_root_edges<<<grid(n), kThreads, 0, st>>>(aabb, n, ax, el.t(ax), el.v(ax));
-      KD_TRY(cudaMemsetAsync(zero, 0, zwords * 4, st), "KD sort");
-      launch_histogram(el.t(ax), E0, 4, zero, st);
-      launch_onesweep(el.t(ax), el.v(ax), E0, 4, ss, err, st);
     }
+    launch_histogram(el.t(0), E0, 4, zero, st, 3, el.cap);
+    launch_onesweep(el.t(0), el.v(0), E0, 4, ss, err, st, 3, el.cap);
     for (int ax = 0; ax < 3; ++ax) {
       KD_TRY(cudaMemsetAsync(el.n(ax), 0, (size_t)E0 * 4, st), "KD root edges");
       count_launch();

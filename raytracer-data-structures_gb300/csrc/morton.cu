@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kThreads) k_morton_tris(const float4* __restri
     if (live) {
       code = code_scene(tri_centroid(verts, idx, i), lo, ext);
       keys[i] = code;
-      vals[i] = i;
+      if (vals) vals[i] = i;
     }
     if (hist) hist_add(sh, code, live);
   }
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kThreads) k_morton_spheres(const float4* __res
         code = code_scene({s.x, s.y, s.z}, s_lo, s_ext);
       }
       keys[i] = code;
-      vals[i] = i;
+      if (vals) vals[i] = i;
     }
     if (hist) hist_add(sh, code, live);
   }

@@ -94,13 +94,15 @@ struct BuildResult {
 
 BuildResult build_accel(int type, const SceneView& s, const rq_settings_t& settings, AccelBuffers& a,
                         BuildScratch& sc, uint32_t* err, cudaStream_t st);
-// Morton codes in primitive order (vals = identity); hist optional.
+// Morton codes in primitive order; vals (identity) and hist optional.
 BuildResult morton_codes(const SceneView& s, int mode, uint32_t* codes, uint32_t* vals,
                          uint32_t* hist, BuildScratch& sc, cudaStream_t st);
 // In-place stable sort; compute_hist = false when sc.zero's histogram was
-// already filled (fused Morton kernel) and zeroed state is in place.
+// already filled (fused Morton kernel) and zeroed state is in place.  count,
+// stride, identity: as launch_onesweep.
 BuildResult sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, int passes, bool compute_hist,
-                       BuildScratch& sc, uint32_t* err, cudaStream_t st);
+                       BuildScratch& sc, uint32_t* err, cudaStream_t st, uint32_t count = 1, size_t stride = 0,
+                       bool identity = false);
 
 // Builders living in their own translation units.
 BuildResult build_median_bvh(const SceneView& s, AccelBuffers& a, BuildScratch& sc, uint32_t* err,

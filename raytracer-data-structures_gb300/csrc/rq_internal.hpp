@@ -60,15 +60,21 @@ size_t sort_status_words(uint32_t n, int passes);
 // hist must hold the digit histogram of `keys` for every pass (as produced by
 // launch_histogram or the fused Morton kernels).  status/counters must be
 // zero.  Result lands in keys/vals.
-void launch_histogram(const uint32_t* keys, uint32_t n, int passes, uint32_t* hist, cudaStream_t s);
+// count > 1: that many sorts of n pairs in one set of launches, `stride` pairs
+// apart in every buffer, their histograms kSortHistWords, tile counters
+// kSortCounterWords and look-back words sort_status_words(n, passes) apart.
+// identity: the values are 0 .. n - 1 (per sort), vals need not hold them.
+constexpr uint32_t kSortHistWords = 1024, kSortCounterWords = 16;
+void launch_histogram(const uint32_t* keys, uint32_t n, int passes, uint32_t* hist, cudaStream_t s,
+                      uint32_t count = 1, size_t stride = 0);
 void launch_onesweep(uint32_t* keys, uint32_t* vals, uint32_t n, int passes, const SortScratch& sc,
-                     uint32_t* err, cudaStream_t s);
+                     uint32_t* err, cudaStream_t s, uint32_t count = 1, size_t stride = 0, bool identity = false);
 // As launch_onesweep, without copying the result back after an odd number of
 // passes: returns the buffer (vals or sc.vals_alt) that holds the sorted values.
 uint32_t* launch_onesweep_vals(uint32_t* keys, uint32_t* vals, uint32_t n, int passes, const SortScratch& sc,
                                uint32_t* err, cudaStream_t s);
 
-// 64-bit keys, 32-bit values (tiles of 2,560 keys).  hist: 256 words per pass
+// 64-bit keys, 32-bit values.  hist: 256 words per pass
 // (up to 8 passes); status: sort_status_words64 words; counters: one per pass.
 size_t sort_status_words64(uint32_t n, int passes);
 void launch_histogram64(const uint64_t* keys, uint32_t n, int passes, uint32_t* hist, cudaStream_t s);

@@ -23,7 +23,7 @@ namespace {
 //   [.., +kStatus)    look-back words            [+16]     error word and padding
 constexpr uint32_t kMaxPairs = RQ_SORT_NOALLOC_MAX_PAIRS;
 constexpr int kMaxPasses = 4;
-constexpr uint32_t kTileKeys = 3840;  // keys per tile of the onesweep kernel
+constexpr uint32_t kTileKeys = 3840;  // at most the keys per tile of a full-size sort (sort_tiles)
 constexpr size_t kMaxTiles = (kMaxPairs + kTileKeys - 1) / kTileKeys;
 constexpr size_t kStatusWords = (size_t)kMaxPasses * kMaxTiles * 256;
 constexpr size_t kHistOff = 2 * (size_t)kMaxPairs;
