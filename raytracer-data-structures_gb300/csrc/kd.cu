@@ -23,6 +23,16 @@
 //    the split go below, those whose end edge follows it go above (:928-934).
 // Leaves list their primitives by id (the reference's order inside a leaf
 // comes from an unstable sort).
+//
+// A level is five launches: costs; decisions with the numbering of interior
+// nodes and leaf refs; sides of the refs with their ranks (both one-pass
+// prefix sums); side counts of the edges, while the host reads the level's
+// totals; children (nodes, refs) ; and the partition of the edges.  Small
+// trees are bound by launches and the one wait a level, large ones by the
+// partition's and cost pass's edge traffic.  GB300 rebuild, against some
+// twenty launches a level, edges as four arrays and side flags and ranks as
+// four more: 36k spheres 4552 -> 1656 us, 82k triangles 5522 -> 2316, 330k
+// 9164 -> 5401, 998k 13824 -> 9880.
 #include <algorithm>
 #include <vector>
 
@@ -49,88 +59,200 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 
 // Level-local node state.
 struct LevelNodes {
-  float* box;         // 6 per node
-  int32_t* depth;
-  int32_t* bad;       // badRefines
+  float4* lo;         // box minimum, 1 / surface area
+  float4* hi;         // box maximum, first ref (bits)
+  uint32_t* open;     // ref count of a node still undecided, else 0
   uint32_t* rs;       // first ref
   uint32_t* rc;       // ref count
-  int32_t* axis0;     // longest axis of the node box
+  int32_t* depth;
+  int32_t* bad;       // badRefines
   unsigned long long* best;  // 3 per node, one per axis: (cost key << 32) | edge offset in the node
-  int32_t* state;     // 0 undecided, 1 leaf, 2 interior
-  int32_t* best_axis;
-  uint32_t* best_off;
-  float* tsplit;
-  uint32_t* split_key;  // the split edge: ordered t key and (ref << 1 | end)
-  uint32_t* split_v;
-  float4* sa;           // node box extents d[0..2] and 1 / surface area, for the cost
-  uint4* plan;          // interior nodes: (sA[rs], sB[rs], sB[rs + rc], first child) for the partition
+  int32_t* axis;      // interior nodes: the split axis; leaves: 3
+  uint2* split;       // the split edge: ordered t key and (ref << 1 | end)
+  uint32_t* irank;    // interior nodes before it
+  uint32_t* lofs;     // leaf refs before it
+  uint4* plan;        // interior nodes: (sA[rs], sB[rs], sB[rs + rc], first child) for the partition
 };
 
 // Edge lists: one per axis, each holding 2 edges per ref of the level (the
 // node's refs' edges at [2 rs, 2 rs + 2 rc)), sorted inside every node by
 // (t, start before end, ref), the order buildTree's edge sort gives
-// (:872-879) with ties in primitive-id order.  Structure of arrays:
-// t[a] (ordered float keys), v[a] (ref << 1 | end), n[a] (node) and s[a]
-// (the number of start edges before the edge in its node: the nBelow of the
-// cost, carried through the partitions).  A child's lists come
-// from its parent's by a stable partition, so the edges are sorted once, at
-// the root.
+// (:872-879) with ties in primitive-id order.  An edge is 16 bytes: x the
+// ordered float key of t, y ref << 1 | end, z its node, w the number of start
+// edges before it in its node (the nBelow of the cost, carried through the
+// partitions).  A child's lists come from its parent's by a stable partition,
+// so the edges are sorted once, at the root.
 struct EdgeLists {
-  uint32_t* base;
+  uint4* base;
   size_t cap;  // edges per list
-  __host__ __device__ uint32_t* t(int a) const { return base + (size_t)a * cap; }
-  __host__ __device__ uint32_t* v(int a) const { return base + (size_t)(3 + a) * cap; }
-  __host__ __device__ uint32_t* n(int a) const { return base + (size_t)(6 + a) * cap; }  // the edge's node
-  __host__ __device__ uint32_t* s(int a) const { return base + (size_t)(9 + a) * cap; }  // start edges before it in its node
+  __host__ __device__ uint4* list(int a) const { return base + (size_t)a * cap; }
 };
-constexpr int kEdgeWords = 12;  // t, v, node and start-rank arrays of the three lists
 
-// Pre-leaf test and first axis (:843, :860); also clears the level's ref
-// side flags (R + 1 each).
-__global__ void k_node_init(LevelNodes L, uint32_t M, uint32_t* __restrict__ below, uint32_t* __restrict__ above,
-                            uint32_t R) {
-  uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k <= R) {
-    below[k] = 0u;
-    above[k] = 0u;
+// ------------------------------------------------------- one-pass prefix sums
+// A tile's exclusive prefix by decoupled look-back: two sums of at most 31
+// bits each in one word (high and low half), with the state in the top two
+// bits.  The first warp reads 32 earlier tiles a round trip; waits are
+// bounded, and a tile that gives up marks itself so later tiles do too.
+constexpr unsigned long long kTileAgg = 1ull << 62, kTilePrefix = 2ull << 62, kTileAbort = 3ull << 62;
+constexpr unsigned long long kTileValue = (1ull << 62) - 1;
+constexpr uint32_t kTilePolls = 1u << 20;
+
+__device__ __forceinline__ unsigned long long tile_load(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void tile_store(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long pair31(uint32_t hi, uint32_t lo) {
+  return ((unsigned long long)hi << 31) | lo;
+}
+
+// The exclusive prefix of thread v over the grid's tiles in tile order; the
+// whole block (256 threads) calls it.  tmp: 34 words of shared memory.  The
+// total up to and including the block in tmp[33].
+__device__ __forceinline__ unsigned long long grid_prefix(unsigned long long v, uint32_t tile,
+                                                          unsigned long long* status, unsigned long long* tmp,
+                                                          uint32_t* err) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  constexpr uint32_t kW = kThreads / 32;
+  unsigned long long x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= (uint32_t)o) x += y;
   }
-  if (k >= M) return;
-  const float* b = L.box + 6 * (size_t)k;
-  for (int a = 0; a < 3; ++a) L.best[3 * (size_t)k + a] = kNone;
-  L.best_axis[k] = -1;
-  if ((int)L.rc[k] <= kMaxPrims || L.depth[k] == 0) {
-    L.state[k] = 1;
-    return;
+  if (lane == 31) tmp[warp] = x;
+  __syncthreads();
+  if (warp == 0) {
+    unsigned long long total = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kW; ++w) total += tmp[w];
+    unsigned long long excl = 0;
+    if (tile == 0) {
+      if (lane == 0) tile_store(status, kTilePrefix | total);
+    } else {
+      if (lane == 0) tile_store(status + tile, kTileAgg | total);
+      uint32_t polls = 0;
+      for (int64_t j = (int64_t)tile - 1;;) {
+        const int64_t at = j - lane;
+        const unsigned long long s = at >= 0 ? tile_load(status + at) : kTilePrefix;
+        const uint32_t flag = (uint32_t)(s >> 62);
+        const uint32_t prefix = __ballot_sync(0xffffffffu, flag >= 2u);  // prefix or abort
+        const uint32_t empty = __ballot_sync(0xffffffffu, flag == 0u);
+        const uint32_t use = prefix ? (prefix & (0u - prefix)) * 2u - 1u : 0xffffffffu;  // up to the nearest prefix
+        const bool aborted = __any_sync(0xffffffffu, flag == 3u && ((use >> lane) & 1u));
+        if (aborted || polls > kTilePolls) {
+          if (lane == 0) {
+            atomicOr(err, kErrTimeout);
+            tile_store(status + tile, kTileAbort);
+          }
+          excl = 0;
+          total = 0;
+          break;
+        }
+        if (empty & use) {
+          if (++polls > 64u) __nanosleep(100);
+          continue;
+        }
+        unsigned long long part = ((use >> lane) & 1u) ? s & kTileValue : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        excl += part;
+        if (prefix) {
+          if (lane == 0) tile_store(status + tile, kTilePrefix | ((excl + total) & kTileValue));
+          break;
+        }
+        j -= 32;
+      }
+    }
+    if (lane == 0) {
+      tmp[32] = excl;
+      tmp[33] = excl + total;
+    }
   }
-  float ax = __fsub_rn(b[3], b[0]), ay = __fsub_rn(b[4], b[1]), az = __fsub_rn(b[5], b[2]);
-  L.state[k] = 0;
-  L.axis0[k] = (ax > ay && ax > az) ? 0 : (ay > az ? 1 : 2);
-  // totalSA and its inverse as buildTree computes them (:855-857)
+  __syncthreads();
+  unsigned long long before = tmp[32];
+#pragma unroll
+  for (uint32_t w = 0; w < kW; ++w) before += w < warp ? tmp[w] : 0ull;
+  return before + x - v;
+}
+
+// Node k's first state: a leaf by the pre-leaf test (:843), or undecided with
+// its box's surface (:855-857).
+__device__ __forceinline__ void init_node(const LevelNodes& L, uint32_t k, F3 lo, F3 hi, uint32_t rs, uint32_t rc,
+                                          int depth, int bad) {
+  const float ax = __fsub_rn(hi.x, lo.x), ay = __fsub_rn(hi.y, lo.y), az = __fsub_rn(hi.z, lo.z);
   const float totalSA = __fmul_rn(2.f, __fadd_rn(__fadd_rn(__fmul_rn(ax, ay), __fmul_rn(ax, az)), __fmul_rn(ay, az)));
-  L.sa[k] = make_float4(ax, ay, az, __fdiv_rn(1.f, totalSA));
+  L.lo[k] = make_float4(lo.x, lo.y, lo.z, __fdiv_rn(1.f, totalSA));
+  L.hi[k] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(rs));
+  L.open[k] = ((int)rc <= kMaxPrims || depth == 0) ? 0u : rc;
+  L.rs[k] = rs;
+  L.rc[k] = rc;
+  L.depth[k] = depth;
+  L.bad[k] = bad;
+  for (int a = 0; a < 3; ++a) L.best[3 * (size_t)k + a] = kNone;
+}
+
+__global__ void k_root_node(LevelNodes L, const int32_t* lohi, float* root, uint32_t n, int depth) {
+  if (threadIdx.x != 0) return;
+  float b[6];
+  for (int q = 0; q < 6; ++q) root[q] = b[q] = ordered_to_float(lohi[q]);
+  init_node(L, 0, {b[0], b[1], b[2]}, {b[3], b[4], b[5]}, 0, n, depth, 0);
 }
 
 // Root edge lists before the sort: starts of refs 0..n-1, then their ends,
-// so a stable sort by t alone orders equal t start-first and by ref.
-__global__ void k_root_edges(const float* __restrict__ aabb, uint32_t n, int a, uint32_t* __restrict__ t,
-                             uint32_t* __restrict__ v) {
+// so a stable sort by t alone orders equal t start-first and by ref.  Also
+// the root's refs.
+__global__ void k_root_edges(const float* __restrict__ aabb, uint32_t n, uint32_t* __restrict__ t,
+                             uint32_t* __restrict__ v, uint32_t* __restrict__ ref_prim, uint32_t* __restrict__ ref_node) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
+  ref_prim[p] = p;
+  ref_node[p] = 0u;
   const float* q = aabb + 6 * (size_t)p;
-  t[p] = float_key(__ldg(q + a));
-  v[p] = p << 1;
-  t[n + p] = float_key(__ldg(q + 3 + a));
-  v[n + p] = (p << 1) | 1u;
+  for (int a = 0; a < 3; ++a) {
+    const size_t at = (size_t)a * 2 * n;
+    t[at + p] = float_key(__ldg(q + a));
+    v[at + p] = p << 1;
+    t[at + n + p] = float_key(__ldg(q + 3 + a));
+    v[at + n + p] = (p << 1) | 1u;
+  }
 }
 
-__global__ void k_start_flags(const uint32_t* __restrict__ v, uint32_t E, uint32_t* __restrict__ f) {
-  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < E) f[e] = (v[e] & 1u) ? 0u : 1u;
+// The sorted root lists as edges (blockIdx.y: the axis): the start ranks are
+// a prefix sum of the start flags.
+constexpr int kRootItems = 8;
+__global__ void __launch_bounds__(kThreads) k_root_lists(const uint32_t* __restrict__ t, const uint32_t* __restrict__ v,
+                                                         uint32_t E, EdgeLists el, unsigned long long* status,
+                                                         uint32_t* ticket, uint32_t tiles, uint32_t* err) {
+  __shared__ unsigned long long tmp[34];
+  __shared__ uint32_t s_tile;
+  const int a = blockIdx.y;
+  if (threadIdx.x == 0) s_tile = atomicAdd(ticket + a, 1u);
+  __syncthreads();
+  const uint32_t tile = s_tile, e0 = (tile * kThreads + threadIdx.x) * kRootItems;
+  uint32_t vv[kRootItems], starts = 0;
+#pragma unroll
+  for (int j = 0; j < kRootItems; ++j) {
+    vv[j] = e0 + j < E ? __ldg(v + (size_t)a * E + e0 + j) : 1u;
+    starts += (vv[j] & 1u) ^ 1u;
+  }
+  uint32_t rank = (uint32_t)grid_prefix(starts, tile, status + (size_t)a * tiles, tmp, err);
+#pragma unroll
+  for (int j = 0; j < kRootItems; ++j)
+    if (e0 + j < E) {
+      el.list(a)[e0 + j] = make_uint4(__ldg(t + (size_t)a * E + e0 + j), vv[j], 0u, rank);
+      rank += (vv[j] & 1u) ^ 1u;
+    }
 }
 
 constexpr int kEdgeItems = 8;
 constexpr uint32_t kEdgeRun = 32 * kEdgeItems;               // edges per warp: lane l takes 32 j + l in round j
 constexpr uint32_t kEdgeTile = kEdgeRun * (kThreads / 32);  // edges per block of the partition passes
+constexpr int kCostItems = 4;
+constexpr uint32_t kCostRun = 32 * kCostItems;               // edges per warp of the cost pass
 
 // SAH cost of splitting at every edge of every undecided node, on all three
 // axes at once (buildTree :883-912, same float operations).  buildTree tries
@@ -138,51 +260,61 @@ constexpr uint32_t kEdgeTile = kEdgeRun * (kThreads / 32);  // edges per block o
 // (:915-919); every axis's minimum is kept and k_decide takes the first axis
 // in that order that has a candidate, which is the same choice.
 //
-// One warp per run of 256 consecutive edges of one list, lane l taking edge
-// 32 j + l in round j.  The lanes that share a node are consecutive, so each
-// round takes every node's minimum by a segmented shuffle reduction; the
-// run that reaches lane 31 is carried into the next round, and only runs
-// that end issue an atomicMin (near the root a level has a few nodes of
-// millions of edges, and one atomic per edge on one address serialises in
-// L2).
+// One warp per run of 128 consecutive edges of one list, lane l taking edge
+// 32 j + l in round j.  A round whose lanes share a node takes its minimum by
+// one warp reduction; otherwise a segmented shuffle reduction finds every
+// node's.  The run that reaches lane 31 is carried into the next round, and
+// only runs that end issue an atomicMin (near the root a level has a few
+// nodes of millions of edges, and one atomic per edge on one address
+// serialises in L2).  The first blocks also clear the level's look-back words.
 __device__ __forceinline__ void flush_best(LevelNodes L, uint32_t k, int a, unsigned long long ck) {
   if (ck != kNone) atomicMin(L.best + 3 * (size_t)k + a, ck);
 }
 
 __global__ void __launch_bounds__(kThreads) k_cost(EdgeLists el, uint32_t E2, uint32_t runs_per_list, uint32_t M,
-                                                   LevelNodes L, uint32_t* err) {
+                                                   LevelNodes L, unsigned long long* clear, uint32_t clear_words,
+                                                   uint32_t* err) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < clear_words; i += gridDim.x * blockDim.x) clear[i] = 0ull;
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (gw >= 3 * runs_per_list) return;  // whole warps
   const int lane = threadIdx.x & 31;
   const int a = (int)(gw / runs_per_list);
-  const uint32_t run0 = (gw - (uint32_t)a * runs_per_list) * kEdgeRun;
-  const uint32_t* __restrict__ tl = el.t(a);
-  const uint32_t* __restrict__ vl = el.v(a);
-  const uint32_t* __restrict__ nl = el.n(a);
-  const uint32_t* __restrict__ sl = el.s(a);
+  const uint32_t run0 = (gw - (uint32_t)a * runs_per_list) * kCostRun;
+  const uint4* __restrict__ list = el.list(a);
   uint32_t carry_k = 0xFFFFFFFFu;  // the open run from the previous round (warp-uniform)
   unsigned long long carry = kNone;
-#pragma unroll 2
-  for (int j = 0; j < kEdgeItems; ++j) {
+  uint4 edge[kCostItems];
+  uint32_t open[kCostItems];
+#pragma unroll
+  for (int j = 0; j < kCostItems; ++j) {
     const uint32_t e = run0 + 32 * j + lane;
-    const bool in = e < E2;
-    uint32_t k = in ? __ldg(nl + e) : 0xFFFFFFFFu;
-    if (in && k >= M) { atomicOr(err, kErrCorrupt); k = 0xFFFFFFFFu; }
+    edge[j] = e < E2 ? __ldg(list + e) : make_uint4(0u, 0u, 0xFFFFFFFFu, 0u);
+  }
+#pragma unroll
+  for (int j = 0; j < kCostItems; ++j) {
+    if (edge[j].z != 0xFFFFFFFFu && edge[j].z >= M) { atomicOr(err, kErrCorrupt); edge[j].z = 0xFFFFFFFFu; }
+    open[j] = edge[j].z != 0xFFFFFFFFu ? __ldg(L.open + edge[j].z) : 0u;
+  }
+#pragma unroll
+  for (int j = 0; j < kCostItems; ++j) {
+    const uint32_t e = run0 + 32 * j + lane, k = edge[j].z;
     unsigned long long ck = kNone;
-    if (k != 0xFFFFFFFFu && L.state[k] == 0) {
-      const float t = key_float(__ldg(tl + e));
-      const float* b = L.box + 6 * (size_t)k;
-      const float lo = b[a], hi = b[3 + a];
+    uint32_t key = 0xFFFFFFFFu, off = 0;
+    bool have = false;
+    if (open[j]) {
+      const float t = key_float(edge[j].x);
+      const float4 bl = __ldg(L.lo + k), bh = __ldg(L.hi + k);
+      const float lo = a == 0 ? bl.x : a == 1 ? bl.y : bl.z, hi = a == 0 ? bh.x : a == 1 ? bh.y : bh.z;
       if (t > lo && t < hi) {
-        const uint32_t rs = L.rs[k], n = L.rc[k];
-        const uint32_t nBelow = __ldg(sl + e);
-        const uint32_t off = e - 2 * rs;
-        const uint32_t nEndIncl = off - nBelow + (__ldg(vl + e) & 1u);
+        const uint32_t rs = __float_as_uint(bh.w), n = open[j];
+        const uint32_t nBelow = edge[j].w;
+        off = e - 2 * rs;
+        const uint32_t nEndIncl = off - nBelow + (edge[j].y & 1u);
         const uint32_t nAbove = n - nEndIncl;
-        const float4 q = L.sa[k];
-        const float invTotalSA = q.w;
-        const float d0 = a == 0 ? q.y : a == 1 ? q.z : q.x;  // the other two axes, (a + 1) % 3 and (a + 2) % 3
-        const float d1 = a == 0 ? q.z : a == 1 ? q.x : q.y;
+        const float invTotalSA = bl.w;
+        const float ex = __fsub_rn(bh.x, bl.x), ey = __fsub_rn(bh.y, bl.y), ez = __fsub_rn(bh.z, bl.z);
+        const float d0 = a == 0 ? ey : a == 1 ? ez : ex;  // the other two axes, (a + 1) % 3 and (a + 2) % 3
+        const float d1 = a == 0 ? ez : a == 1 ? ex : ey;
         float dd = __fmul_rn(d0, d1), ds = __fadd_rn(d0, d1);
         float belowSA = __fmul_rn(2.f, __fadd_rn(dd, __fmul_rn(__fsub_rn(t, lo), ds)));
         float aboveSA = __fmul_rn(2.f, __fadd_rn(dd, __fmul_rn(__fsub_rn(hi, t), ds)));
@@ -191,8 +323,25 @@ __global__ void __launch_bounds__(kThreads) k_cost(EdgeLists el, uint32_t E2, ui
         float cost = __fadd_rn(kTrav, __fmul_rn(__fmul_rn(kIsect, __fsub_rn(1.f, eb)),
                                                 __fadd_rn(__fmul_rn(pB, (float)nBelow),
                                                           __fmul_rn(pA, (float)nAbove))));
-        ck = ((unsigned long long)float_key(cost) << 32) | (unsigned long long)off;
+        key = float_key(cost);
+        ck = ((unsigned long long)key << 32) | (unsigned long long)off;
+        have = true;
       }
+    }
+    const uint32_t k0 = __shfl_sync(0xffffffffu, k, 0);
+    if (__all_sync(0xffffffffu, k == k0)) {  // one node: offsets grow with the lane, so the first lane of the minimum
+      const uint32_t m = __reduce_min_sync(0xffffffffu, key);
+      const uint32_t at = __ballot_sync(0xffffffffu, have && key == m);
+      unsigned long long best = kNone;
+      if (at) best = ((unsigned long long)m << 32) | __shfl_sync(0xffffffffu, off, __ffs(at) - 1);
+      if (carry_k == k0) {
+        if (best < carry) carry = best;
+      } else {
+        if (lane == 0 && carry_k != 0xFFFFFFFFu) flush_best(L, carry_k, a, carry);
+        carry_k = k0;
+        carry = best;
+      }
+      continue;
     }
     // Minimum over the lane's run of equal nodes from this lane on.
 #pragma unroll
@@ -206,7 +355,6 @@ __global__ void __launch_bounds__(kThreads) k_cost(EdgeLists el, uint32_t E2, ui
     const uint32_t heads = __ballot_sync(0xffffffffu, head);
     const int last = 31 - __clz(heads);  // head of the run that reaches lane 31
     // the carried run continues into lane 0's run or ends here
-    const uint32_t k0 = __shfl_sync(0xffffffffu, k, 0);
     if (lane == 0) {
       if (carry_k == k0) { if (carry < ck) ck = carry; }
       else if (carry_k != 0xFFFFFFFFu) flush_best(L, carry_k, a, carry);
@@ -218,95 +366,144 @@ __global__ void __launch_bounds__(kThreads) k_cost(EdgeLists el, uint32_t E2, ui
   if (lane == 0 && carry_k != 0xFFFFFFFFu) flush_best(L, carry_k, a, carry);
 }
 
-// Split decision (:915-925): the first axis from the longest on with a
-// candidate edge; none -> leaf.
-__device__ void decide_node(EdgeLists el, LevelNodes L, uint32_t k, uint32_t E2, uint32_t* err);
-
-// Decides every undecided node, then writes each node's interior flag and
-// leaf ref count (M + 1 entries, the last 0) for the level's scans.
-__global__ void k_decide(EdgeLists el, LevelNodes L, uint32_t M, uint32_t E2, uint32_t* __restrict__ iflag,
-                         uint32_t* __restrict__ lcnt, uint32_t* err) {
-  uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k > M) return;
-  if (k == M) {
-    iflag[k] = 0u;
-    lcnt[k] = 0u;
-    return;
-  }
-  if (L.state[k] == 0) decide_node(el, L, k, E2, err);
-  const int st = L.state[k];
-  iflag[k] = st == 2 ? 1u : 0u;
-  lcnt[k] = st == 1 ? L.rc[k] : 0u;
-}
-
-__device__ void decide_node(EdgeLists el, LevelNodes L, uint32_t k, uint32_t E2, uint32_t* err) {
+// Split decision (:915-925) of an undecided node: the first axis from the
+// longest on with a candidate edge; none -> leaf.  Returns whether it is an
+// interior node.
+__device__ __forceinline__ bool decide_node(EdgeLists el, LevelNodes L, uint32_t k, uint32_t rc, uint32_t E2, uint32_t* err) {
+  const float4 lo = L.lo[k], hi = L.hi[k];
+  const float ax = __fsub_rn(hi.x, lo.x), ay = __fsub_rn(hi.y, lo.y), az = __fsub_rn(hi.z, lo.z);
+  const int axis0 = (ax > ay && ax > az) ? 0 : (ay > az ? 1 : 2);
+  unsigned long long bs[3];
+  for (int a = 0; a < 3; ++a) bs[a] = L.best[3 * (size_t)k + a];
   for (int q = 0; q < 3; ++q) {
-    const int a = (L.axis0[k] + q) % 3;
-    const unsigned long long b = L.best[3 * (size_t)k + a];
+    const int a = (axis0 + q) % 3;
+    const unsigned long long b = a == 0 ? bs[0] : a == 1 ? bs[1] : bs[2];
     if (b == kNone) continue;
     const float bestCost = key_float((uint32_t)(b >> 32));
-    const float oldCost = __fmul_rn(kIsect, (float)L.rc[k]);
+    const float oldCost = __fmul_rn(kIsect, (float)rc);
     const int bad = L.bad[k] + (bestCost > oldCost ? 1 : 0);
     L.bad[k] = bad;
-    const bool leaf = (bestCost > __fmul_rn(4.f, oldCost) && L.rc[k] < 16) || bad == 3;
-    L.state[k] = leaf ? 1 : 2;
-    L.best_axis[k] = a;
-    const uint32_t off = (uint32_t)(b & 0xFFFFFFFFull), e = 2 * L.rs[k] + off;
-    L.best_off[k] = off;
-    if (e >= E2) { atomicOr(err, kErrCorrupt); L.state[k] = 1; return; }
-    const uint32_t key = el.t(a)[e];
-    L.split_key[k] = key;
-    L.split_v[k] = el.v(a)[e];
-    L.tsplit[k] = key_float(key);
-    return;
+    const bool leaf = (bestCost > __fmul_rn(4.f, oldCost) && rc < 16) || bad == 3;
+    if (leaf) return false;
+    const uint32_t e = 2 * L.rs[k] + (uint32_t)(b & 0xFFFFFFFFull);
+    if (e >= E2) { atomicOr(err, kErrCorrupt); return false; }
+    const uint4 edge = el.list(a)[e];
+    L.split[k] = make_uint2(edge.x, edge.y);
+    L.axis[k] = a;
+    return true;
   }
-  L.state[k] = 1;  // no split found on any axis
+  return false;  // no split found on any axis
+}
+
+// Decides every undecided node and numbers the level's interior nodes and
+// leaf refs (totals: [0] interiors, [1] leaf refs).
+__global__ void __launch_bounds__(kThreads) k_decide(EdgeLists el, LevelNodes L, uint32_t M, uint32_t E2,
+                                                     unsigned long long* status, uint32_t* ticket,
+                                                     uint32_t* __restrict__ totals, uint32_t* err) {
+  __shared__ unsigned long long tmp[34];
+  __shared__ uint32_t s_tile;
+  if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+  __syncthreads();
+  const uint32_t tile = s_tile, k = tile * kThreads + threadIdx.x;
+  uint32_t interior = 0, leaf_refs = 0;
+  if (k < M) {
+    const uint32_t rc = L.rc[k], open = L.open[k];
+    if (open && decide_node(el, L, k, open, E2, err)) {
+      interior = 1u;
+    } else {
+      L.axis[k] = 3;
+      leaf_refs = rc;
+    }
+  }
+  const unsigned long long at = grid_prefix(pair31(interior, leaf_refs), tile, status, tmp, err);
+  if (k < M) {
+    L.irank[k] = (uint32_t)(at >> 31);
+    L.lofs[k] = (uint32_t)(at & 0x7FFFFFFFull);
+  }
+  if (tile == gridDim.x - 1 && threadIdx.x == 0) {
+    totals[0] = (uint32_t)((tmp[33] & kTileValue) >> 31);
+    totals[1] = (uint32_t)(tmp[33] & 0x7FFFFFFFull);
+  }
 }
 
 // Below/above sides (:928-934): a ref whose start edge precedes the split
 // edge in the chosen axis's sorted order goes below, one whose end edge
 // follows it goes above.  The order is (t key, start before end, ref), so
 // the comparison needs only the ref's box and the split edge, not the list.
-__global__ void k_classify(const uint32_t* __restrict__ ref_prim, const uint32_t* __restrict__ ref_node,
-                           uint32_t R, uint32_t M, const float* __restrict__ aabb, LevelNodes L,
-                           uint32_t* __restrict__ below, uint32_t* __restrict__ above, uint32_t* err) {
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  const uint32_t k = __ldg(ref_node + r);
-  if (k >= M) { atomicOr(err, kErrCorrupt); return; }
-  if (L.state[k] != 2) return;
-  const int a = L.best_axis[k];
-  const uint32_t sk = L.split_key[k], sv = L.split_v[k], sr = sv >> 1;
-  const float* q = aabb + 6 * (size_t)__ldg(ref_prim + r);
-  const uint32_t lo = float_key(__ldg(q + a)), hi = float_key(__ldg(q + 3 + a));
-  below[r] = (lo < sk || (lo == sk && ((sv & 1u) || r < sr))) ? 1u : 0u;   // (lo, start, r) < split
-  above[r] = (hi > sk || (hi == sk && (!(sv & 1u) || r > sr))) ? 1u : 0u;  // (hi, end, r) > split
+// sides[r] = (below refs before r | below flag << 31, the same for above),
+// r = 0 .. R; totals: [2] below refs, [3] above refs.
+constexpr uint32_t kSideFlag = 0x80000000u, kSideRank = 0x7FFFFFFFu;
+constexpr int kSideItems = 4;
+__global__ void __launch_bounds__(kThreads) k_sides(const uint32_t* __restrict__ ref_prim,
+                                                    const uint32_t* __restrict__ ref_node, uint32_t R, uint32_t M,
+                                                    const float* __restrict__ aabb, LevelNodes L,
+                                                    uint2* __restrict__ sides, unsigned long long* status,
+                                                    uint32_t* ticket, uint32_t* __restrict__ totals, uint32_t* err) {
+  __shared__ unsigned long long tmp[34];
+  __shared__ uint32_t s_tile;
+  if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+  __syncthreads();
+  const uint32_t tile = s_tile, r0 = (tile * kThreads + threadIdx.x) * kSideItems;
+  uint32_t b = 0, ab = 0;  // flags of the thread's refs
+  uint32_t node[kSideItems], axis[kSideItems], prim[kSideItems];
+#pragma unroll
+  for (int j = 0; j < kSideItems; ++j) {
+    node[j] = r0 + j < R ? __ldg(ref_node + r0 + j) : 0xFFFFFFFFu;
+    prim[j] = r0 + j < R ? __ldg(ref_prim + r0 + j) : 0u;
+    if (node[j] != 0xFFFFFFFFu && node[j] >= M) { atomicOr(err, kErrCorrupt); node[j] = 0xFFFFFFFFu; }
+  }
+#pragma unroll
+  for (int j = 0; j < kSideItems; ++j) axis[j] = node[j] != 0xFFFFFFFFu ? (uint32_t)L.axis[node[j]] : 3u;
+#pragma unroll
+  for (int j = 0; j < kSideItems; ++j) {
+    if (axis[j] == 3u) continue;
+    const uint2 sp = L.split[node[j]];
+    const uint32_t sk = sp.x, sv = sp.y, sr = sv >> 1, r = r0 + j;
+    const float* q = aabb + 6 * (size_t)prim[j] + axis[j];
+    const uint32_t lo = float_key(__ldg(q)), hi = float_key(__ldg(q + 3));
+    if (lo < sk || (lo == sk && ((sv & 1u) || r < sr))) b |= 1u << j;    // (lo, start, r) < split
+    if (hi > sk || (hi == sk && (!(sv & 1u) || r > sr))) ab |= 1u << j;  // (hi, end, r) > split
+  }
+  const unsigned long long at = grid_prefix(pair31(__popc(b), __popc(ab)), tile, status, tmp, err);
+  uint32_t sb = (uint32_t)(at >> 31), sa = (uint32_t)(at & 0x7FFFFFFFull);
+#pragma unroll
+  for (int j = 0; j < kSideItems; ++j) {
+    const uint32_t fb = (b >> j) & 1u, fa = (ab >> j) & 1u;
+    if (r0 + j <= R) sides[r0 + j] = make_uint2(sb | (fb ? kSideFlag : 0u), sa | (fa ? kSideFlag : 0u));
+    sb += fb;
+    sa += fa;
+  }
+  if (tile == gridDim.x - 1 && threadIdx.x == 0) {
+    totals[2] = (uint32_t)((tmp[33] & kTileValue) >> 31);
+    totals[3] = (uint32_t)(tmp[33] & 0x7FFFFFFFull);
+  }
 }
 
 // Children's edge lists: a stable partition of every interior node's edges,
-// on each axis, into its below child (refs with below[r]) and above child
-// (refs with above[r]); straddling refs go to both.  With sB / sA the
-// exclusive scans of below / above over the level's refs, and BS, BE, AS, AE
-// the list-wide counts of below-start, below-end, above-start and above-end
+// on each axis, into its below child (refs with the below flag) and above
+// child (refs with the above flag); straddling refs go to both.  With sB / sA
+// the below / above refs before a ref (sides), and BS, BE, AS, AE the
+// list-wide counts of below-start, below-end, above-start and above-end
 // edges before e:
 //   below child: position BS + BE + 2 sA[rs], ref sA[rs] + sB[r],
 //                start rank BS - sB[rs]
 //   above child: position AS + AE + 2 sB[re], ref sB[re] + sA[r],
 //                start rank AS - sA[rs]
 // (re = rs + rc; children are laid out node by node, below before above,
-// and leaf refs count in neither scan), matching k_emit_refs's numbering of
+// and leaf refs count in neither), matching k_spawn_emit's numbering of
 // the refs.  Per node the bases come from plan[k] = (sA[rs], sB[rs], sB[re],
-// first child), written by k_spawn.
+// first child), written by k_spawn_emit.
 //
-// Three passes, none waiting on another block: k_part_count counts each
-// tile's (BS, BE) and (AS, AE), packed 31 bits apiece in two 64-bit words
-// (lists hold fewer than 2^31 edges, so the fields never carry), and keeps
-// the side flags as one ballot word per 32 edges; k_part_scan turns the tile
-// counts of each list into exclusive prefixes; k_partition adds the warp
-// offsets inside the tile and scatters.
+// Passes, none waiting on another block: k_part_count counts each tile's
+// (BS, BE) and (AS, AE), packed 31 bits apiece in two 64-bit words (lists
+// hold fewer than 2^31 edges, so the fields never carry), and keeps the side
+// flags as one ballot word per 32 edges; k_partition adds up the earlier
+// tiles' counts (k_part_scan does when there are more than kPartSelf) and the
+// warp offsets inside the tile, and scatters.
+constexpr uint32_t kPartSelf = 1024;
+
 __global__ void __launch_bounds__(kThreads) k_part_count(EdgeLists el, uint32_t E2, uint32_t tiles_per_list,
-                                                         uint32_t R, uint32_t M, const uint32_t* __restrict__ below,
-                                                         const uint32_t* __restrict__ above,
+                                                         uint32_t R, const uint2* __restrict__ sides,
                                                          uint32_t* __restrict__ sideB, uint32_t* __restrict__ sideA,
                                                          unsigned long long* __restrict__ tile_cnt, uint32_t* err) {
   __shared__ unsigned long long wsum[2][kThreads / 32];
@@ -314,31 +511,34 @@ __global__ void __launch_bounds__(kThreads) k_part_count(EdgeLists el, uint32_t 
   const uint32_t tile = blockIdx.x, a = tile / tiles_per_list;
   const uint32_t run0 = (tile - a * tiles_per_list) * kEdgeTile + (uint32_t)warp * kEdgeRun;
   const size_t words = (size_t)(E2 + 31) / 32;  // ballot words per list
-  unsigned long long t0 = 0, t1 = 0;
+  uint32_t v[kEdgeItems];
+  uint2 sd[kEdgeItems];
 #pragma unroll
   for (int j = 0; j < kEdgeItems; ++j) {
     const uint32_t e = run0 + 32 * j + lane;
-    const bool in = e < E2;
-    const uint32_t v = in ? __ldg(el.v(a) + e) : 0u;
-    bool b = false, ab = false;
-    if (in) {
-      const uint32_t r = v >> 1, k = __ldg(el.n(a) + e);
-      if (r < R && k < M) {
-        b = __ldg(below + r) != 0u;
-        ab = __ldg(above + r) != 0u;
-      } else {
-        atomicOr(err, kErrCorrupt);
-      }
+    v[j] = e < E2 ? __ldg(&el.list(a)[e].y) : 0xFFFFFFFFu;
+  }
+#pragma unroll
+  for (int j = 0; j < kEdgeItems; ++j) {
+    sd[j] = make_uint2(0u, 0u);
+    if (v[j] != 0xFFFFFFFFu) {
+      if ((v[j] >> 1) < R) sd[j] = __ldg(sides + (v[j] >> 1));
+      else atomicOr(err, kErrCorrupt);
     }
-    const uint32_t kb = __ballot_sync(0xffffffffu, b), ka = __ballot_sync(0xffffffffu, ab);
-    const uint32_t em = __ballot_sync(0xffffffffu, (v & 1u) != 0u);
+  }
+  unsigned long long t0 = 0, t1 = 0;
+#pragma unroll
+  for (int j = 0; j < kEdgeItems; ++j) {
+    const uint32_t kb = __ballot_sync(0xffffffffu, (sd[j].x & kSideFlag) != 0u);
+    const uint32_t ka = __ballot_sync(0xffffffffu, (sd[j].y & kSideFlag) != 0u);
+    const uint32_t em = __ballot_sync(0xffffffffu, (v[j] & 1u) != 0u);
     const uint32_t w = (run0 >> 5) + (uint32_t)j;
     if (lane == 0 && w < words) {
       sideB[(size_t)a * words + w] = kb;
       sideA[(size_t)a * words + w] = ka;
     }
-    t0 += ((unsigned long long)__popc(kb & em) << 31) | (unsigned long long)__popc(kb & ~em);
-    t1 += ((unsigned long long)__popc(ka & em) << 31) | (unsigned long long)__popc(ka & ~em);
+    t0 += pair31(__popc(kb & em), __popc(kb & ~em));
+    t1 += pair31(__popc(ka & em), __popc(ka & ~em));
   }
   if (lane == 0) {
     wsum[0][warp] = t0;
@@ -384,43 +584,63 @@ __global__ void __launch_bounds__(1024) k_part_scan(unsigned long long* tile_cnt
   }
 }
 
+template <bool SCANNED>
 __global__ void __launch_bounds__(kThreads) k_partition(EdgeLists el, uint32_t E2, uint32_t tiles_per_list,
                                                         LevelNodes L, const uint32_t* __restrict__ sideB,
                                                         const uint32_t* __restrict__ sideA,
-                                                        const unsigned long long* __restrict__ tile_pre,
-                                                        const uint32_t* __restrict__ sB,
-                                                        const uint32_t* __restrict__ sA, EdgeLists out,
+                                                        const unsigned long long* __restrict__ tile_cnt,
+                                                        const uint2* __restrict__ sides, EdgeLists out,
                                                         uint32_t E2next, uint32_t* err) {
-  __shared__ unsigned long long wpre[2][kThreads / 32];
+  __shared__ unsigned long long wpre[2][kThreads / 32], wsum[2][kThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t tile = blockIdx.x, a = tile / tiles_per_list;
   const uint32_t run0 = (tile - a * tiles_per_list) * kEdgeTile + (uint32_t)warp * kEdgeRun;
   const size_t words = (size_t)(E2 + 31) / 32;
-  // Side-flag words and end-edge ballots of round j (read twice: for the
-  // warp totals, then for the scatter; the second read hits the cache).
-  auto round_flags = [&](int j, uint32_t& kb, uint32_t& ka, uint32_t& em, uint32_t& v) {
-    const uint32_t e = run0 + 32 * j + lane;
-    const uint32_t w = (run0 >> 5) + (uint32_t)j;
-    const bool wv = w < words;
-    kb = wv ? __ldg(sideB + (size_t)a * words + w) : 0u;
-    ka = wv ? __ldg(sideA + (size_t)a * words + w) : 0u;
-    v = e < E2 ? __ldg(el.v(a) + e) : 0u;
-    em = __ballot_sync(0xffffffffu, (v & 1u) != 0u);
-  };
+  uint4 edge[kEdgeItems];
+  uint32_t kb[kEdgeItems], ka[kEdgeItems];
+#pragma unroll
+  for (int j = 0; j < kEdgeItems; ++j) {
+    const uint32_t e = run0 + 32 * j + lane, w = (run0 >> 5) + (uint32_t)j;
+    kb[j] = w < words ? __ldg(sideB + (size_t)a * words + w) : 0u;
+    ka[j] = w < words ? __ldg(sideA + (size_t)a * words + w) : 0u;
+    edge[j] = e < E2 ? __ldg(el.list(a) + e) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  unsigned long long p0 = 0, p1 = 0;
+  if (SCANNED) {
+    p0 = __ldg(tile_cnt + 2 * (size_t)tile);
+    p1 = __ldg(tile_cnt + 2 * (size_t)tile + 1);
+  } else {
+    for (uint32_t t = a * tiles_per_list + threadIdx.x; t < tile; t += kThreads) {
+      p0 += __ldg(tile_cnt + 2 * (size_t)t);
+      p1 += __ldg(tile_cnt + 2 * (size_t)t + 1);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      p0 += __shfl_xor_sync(0xffffffffu, p0, o);
+      p1 += __shfl_xor_sync(0xffffffffu, p1, o);
+    }
+  }
   unsigned long long t0 = 0, t1 = 0;
 #pragma unroll
   for (int j = 0; j < kEdgeItems; ++j) {
-    uint32_t kb, ka, em, v;
-    round_flags(j, kb, ka, em, v);
-    t0 += ((unsigned long long)__popc(kb & em) << 31) | (unsigned long long)__popc(kb & ~em);
-    t1 += ((unsigned long long)__popc(ka & em) << 31) | (unsigned long long)__popc(ka & ~em);
+    const uint32_t em = __ballot_sync(0xffffffffu, (edge[j].y & 1u) != 0u);
+    t0 += pair31(__popc(kb[j] & em), __popc(kb[j] & ~em));
+    t1 += pair31(__popc(ka[j] & em), __popc(ka[j] & ~em));
   }
   if (lane == 0) {
     wpre[0][warp] = t0;
     wpre[1][warp] = t1;
+    wsum[0][warp] = p0;
+    wsum[1][warp] = p1;
   }
   __syncthreads();
-  unsigned long long p0 = __ldg(tile_pre + 2 * (size_t)tile), p1 = __ldg(tile_pre + 2 * (size_t)tile + 1);
+  if (!SCANNED) {
+    p0 = p1 = 0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      p0 += wsum[0][w];
+      p1 += wsum[1][w];
+    }
+  }
   for (int w = 0; w < warp; ++w) {
     p0 += wpre[0][w];
     p1 += wpre[1][w];
@@ -428,38 +648,26 @@ __global__ void __launch_bounds__(kThreads) k_partition(EdgeLists el, uint32_t E
   uint32_t cbs = (uint32_t)(p0 & 0x7FFFFFFFull), cbe = (uint32_t)(p0 >> 31);
   uint32_t cas = (uint32_t)(p1 & 0x7FFFFFFFull), cae = (uint32_t)(p1 >> 31);
   const uint32_t lt = (1u << lane) - 1u, me = 1u << lane;
-#pragma unroll 2
+#pragma unroll
   for (int j = 0; j < kEdgeItems; ++j) {
-    uint32_t kb, ka, em, v;
-    round_flags(j, kb, ka, em, v);
-    const uint32_t bs = kb & ~em, be = kb & em, as = ka & ~em, ae = ka & em;
-    const bool b = (kb & me) != 0u, ab = (ka & me) != 0u;
+    const uint32_t em = __ballot_sync(0xffffffffu, (edge[j].y & 1u) != 0u);
+    const uint32_t bs = kb[j] & ~em, be = kb[j] & em, as = ka[j] & ~em, ae = ka[j] & em;
+    const bool b = (kb[j] & me) != 0u, ab = (ka[j] & me) != 0u;
     if (b || ab) {
-      const uint32_t e = run0 + 32 * j + lane;
-      const uint32_t tk = __ldg(el.t(a) + e), k = __ldg(el.n(a) + e);
-      const uint32_t r = v >> 1, end = v & 1u;
-      const uint4 pl = L.plan[k];  // (sA[rs], sB[rs], sB[re], first child)
+      const uint32_t r = edge[j].y >> 1, end = edge[j].y & 1u;
+      const uint4 pl = __ldg(L.plan + edge[j].z);  // (sA[rs], sB[rs], sB[re], first child)
+      const uint2 sd = __ldg(sides + r);
       if (b) {
         const uint32_t nbs = cbs + __popc(bs & lt), nbe = cbe + __popc(be & lt);
         const uint32_t pos = nbs + nbe + 2 * pl.x;
-        if (pos >= E2next) { atomicOr(err, kErrCorrupt); }
-        else {
-          out.t(a)[pos] = tk;
-          out.v(a)[pos] = ((pl.x + __ldg(sB + r)) << 1) | end;
-          out.n(a)[pos] = pl.w;
-          out.s(a)[pos] = nbs - pl.y;
-        }
+        if (pos >= E2next) atomicOr(err, kErrCorrupt);
+        else out.list(a)[pos] = make_uint4(edge[j].x, ((pl.x + (sd.x & kSideRank)) << 1) | end, pl.w, nbs - pl.y);
       }
       if (ab) {
         const uint32_t nas = cas + __popc(as & lt), nae = cae + __popc(ae & lt);
         const uint32_t pos = nas + nae + 2 * pl.z;
-        if (pos >= E2next) { atomicOr(err, kErrCorrupt); }
-        else {
-          out.t(a)[pos] = tk;
-          out.v(a)[pos] = ((pl.z + __ldg(sA + r)) << 1) | end;
-          out.n(a)[pos] = pl.w + 1;
-          out.s(a)[pos] = nas - pl.x;
-        }
+        if (pos >= E2next) atomicOr(err, kErrCorrupt);
+        else out.list(a)[pos] = make_uint4(edge[j].x, ((pl.z + (sd.y & kSideRank)) << 1) | end, pl.w + 1, nas - pl.x);
       }
     }
     cbs += __popc(bs);
@@ -468,7 +676,6 @@ __global__ void __launch_bounds__(kThreads) k_partition(EdgeLists el, uint32_t E
     cae += __popc(ae);
   }
 }
-
 
 // Global node table (breadth-first ids).
 struct Table {
@@ -481,104 +688,115 @@ struct Table {
   uint32_t* pool_off;   // leaf primitives in the pool
 };
 
-// Interior nodes spawn their two children; every node fills its table entry.
-__global__ void k_spawn(LevelNodes L, uint32_t M, const uint32_t* __restrict__ irank, const uint32_t* __restrict__ sB,
-                        const uint32_t* __restrict__ sA, const uint32_t* __restrict__ lrank_cnt, uint32_t pool_base,
-                        uint32_t level_base, uint32_t next_base, Table T, LevelNodes N,
-                        uint32_t* __restrict__ child_cnt, uint32_t M2, uint32_t* err) {
-  uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k == 0) child_cnt[M2] = 0u;  // the scan's last entry
-  if (k >= M) return;
-  const uint32_t g = level_base + k;
-  const uint32_t rs = L.rs[k], rc = L.rc[k];
-  if (L.state[k] != 2) {
+// Threads up to M: interior nodes spawn their two children (whose refs'
+// places follow from the sides, see the partition), every node fills its
+// table entry.  Threads up to R: stable filter of every interior node's refs
+// into its children; leaf refs to the pool.
+__global__ void __launch_bounds__(kThreads) k_spawn_emit(LevelNodes L, uint32_t M, const uint2* __restrict__ sides,
+                                                         uint32_t pool_base, uint32_t level_base, uint32_t next_base,
+                                                         Table T, LevelNodes N, uint32_t M2,
+                                                         const uint32_t* __restrict__ ref_prim,
+                                                         const uint32_t* __restrict__ ref_node, uint32_t R,
+                                                         uint32_t* __restrict__ out_prim, uint32_t* __restrict__ out_node,
+                                                         uint32_t* __restrict__ pool, uint32_t R2, uint32_t pool_cap,
+                                                         uint32_t* err) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < R) {
+    const uint32_t r = i, k = __ldg(ref_node + r), p = __ldg(ref_prim + r);
+    const uint2 s = __ldg(sides + r);
+    const uint32_t rs = L.rs[k];
+    if (L.axis[k] == 3) {
+      const uint32_t q = pool_base + L.lofs[k] + (r - rs);
+      if (q >= pool_cap) atomicOr(err, kErrCorrupt);
+      else pool[q] = p;
+    } else {
+      const uint32_t c = 2 * L.irank[k];
+      if (s.x & kSideFlag) {
+        const uint32_t o = (__ldg(&sides[rs].y) & kSideRank) + (s.x & kSideRank);
+        if (o >= R2) atomicOr(err, kErrCorrupt);
+        else { out_prim[o] = p; out_node[o] = c; }
+      }
+      if (s.y & kSideFlag) {
+        const uint32_t o = (__ldg(&sides[rs + L.rc[k]].x) & kSideRank) + (s.y & kSideRank);
+        if (o >= R2) atomicOr(err, kErrCorrupt);
+        else { out_prim[o] = p; out_node[o] = c + 1; }
+      }
+    }
+  }
+  if (i >= M) return;
+  const uint32_t k = i, g = level_base + k, rs = L.rs[k], rc = L.rc[k];
+  const int axis = L.axis[k];
+  if (axis == 3) {
     T.leaf[g] = 1;
     T.count[g] = rc;
-    T.pool_off[g] = pool_base + lrank_cnt[k];
+    T.pool_off[g] = pool_base + L.lofs[k];
     return;
   }
-  const uint32_t c = 2 * irank[k];
-  if (c + 1 >= M2 + 1 || L.best_axis[k] < 0) { atomicOr(err, kErrCorrupt); return; }
-  const int axis = L.best_axis[k];
-  const float ts = L.tsplit[k];
+  const uint32_t c = 2 * L.irank[k];
+  if (c + 1 >= M2) { atomicOr(err, kErrCorrupt); return; }
+  const float ts = key_float(L.split[k].x);
   T.leaf[g] = 0;
   T.axis[g] = axis;
   T.split[g] = ts;
   T.child0[g] = next_base + c;
   T.child1[g] = next_base + c + 1;
-  const float* b = L.box + 6 * (size_t)k;
-  for (int side = 0; side < 2; ++side) {
-    float* nb = N.box + 6 * (size_t)(c + side);
-    for (int q = 0; q < 6; ++q) nb[q] = b[q];
-    if (side == 0) nb[3 + axis] = ts;  // bounds0.max[axis] = tSplit
-    else nb[axis] = ts;                // bounds1.min[axis] = tSplit
-    N.depth[c + side] = L.depth[k] - 1;
-    N.bad[c + side] = L.bad[k];
-  }
-  child_cnt[c] = sB[rs + rc] - sB[rs];
-  child_cnt[c + 1] = sA[rs + rc] - sA[rs];
-  L.plan[k] = make_uint4(sA[rs], sB[rs], sB[rs + rc], c);
+  const uint2 s0 = __ldg(sides + rs), s1 = __ldg(sides + rs + rc);
+  const uint32_t b0 = s0.x & kSideRank, a0 = s0.y & kSideRank, b1 = s1.x & kSideRank, a1 = s1.y & kSideRank;
+  const float4 lo = L.lo[k], hi = L.hi[k];
+  const int depth = L.depth[k] - 1, bad = L.bad[k];
+  F3 cut_hi = {hi.x, hi.y, hi.z}, cut_lo = {lo.x, lo.y, lo.z};
+  if (axis == 0) cut_hi.x = cut_lo.x = ts;  // bounds0.max[axis] = bounds1.min[axis] = tSplit
+  else if (axis == 1) cut_hi.y = cut_lo.y = ts;
+  else cut_hi.z = cut_lo.z = ts;
+  init_node(N, c, {lo.x, lo.y, lo.z}, cut_hi, a0 + b0, b1 - b0, depth, bad);
+  init_node(N, c + 1, cut_lo, {hi.x, hi.y, hi.z}, b1 + a0, a1 - a0, depth, bad);
+  L.plan[k] = make_uint4(a0, b0, b1, c);
 }
 
-__global__ void k_set_ref_starts(LevelNodes N, uint32_t M2, const uint32_t* __restrict__ child_cnt,
-                                 const uint32_t* __restrict__ child_off) {
-  uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= M2) return;
-  N.rs[c] = child_off[c];
-  N.rc[c] = child_cnt[c];
+// Depth-first layout: subtree sizes bottom-up, positions top-down, three
+// levels a launch (a level's node lies below one node of the level two up, so
+// that node's thread serves it: 30 levels took 60 launches one by one).
+constexpr int kLayoutLevels = 3;
+template <int D>
+__device__ uint32_t subtree_size(const Table& T, uint32_t g, uint32_t* __restrict__ size, uint32_t total, uint32_t* err) {
+  uint32_t s = 1;
+  if (!T.leaf[g]) {
+    const uint32_t c0 = T.child0[g], c1 = T.child1[g];
+    if (c0 >= total || c1 >= total) {
+      atomicOr(err, kErrCorrupt);
+    } else if constexpr (D > 1) {
+      s += subtree_size<D - 1>(T, c0, size, total, err) + subtree_size<D - 1>(T, c1, size, total, err);
+    } else {
+      s += size[c0] + size[c1];
+    }
+  }
+  size[g] = s;
+  return s;
+}
+template <int D>
+__global__ void k_sizes(Table T, uint32_t lo, uint32_t hi, uint32_t* __restrict__ size, uint32_t total, uint32_t* err) {
+  const uint32_t g = lo + blockIdx.x * blockDim.x + threadIdx.x;
+  if (g < hi) subtree_size<D>(T, g, size, total, err);
 }
 
-// Stable filter of every interior node's refs into its children; leaf refs to the pool.
-__global__ void k_emit_refs(const uint32_t* __restrict__ ref_prim, const uint32_t* __restrict__ ref_node, uint32_t R,
-                            LevelNodes L, const uint32_t* __restrict__ irank, const uint32_t* __restrict__ below,
-                            const uint32_t* __restrict__ above, const uint32_t* __restrict__ sB,
-                            const uint32_t* __restrict__ sA, LevelNodes N, uint32_t* __restrict__ out_prim,
-                            uint32_t* __restrict__ out_node, const uint32_t* __restrict__ lrank_cnt,
-                            uint32_t pool_base, uint32_t* __restrict__ pool, uint32_t R2, uint32_t pool_cap,
-                            uint32_t* err) {
-  uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R) return;
-  const uint32_t k = ref_node[r];
-  const uint32_t p = ref_prim[r];
-  const uint32_t rs = L.rs[k];
-  if (L.state[k] != 2) {
-    const uint32_t q = pool_base + lrank_cnt[k] + (r - rs);
-    if (q >= pool_cap) { atomicOr(err, kErrCorrupt); return; }
-    pool[q] = p;
-    return;
-  }
-  const uint32_t c = 2 * irank[k];
-  if (below[r]) {
-    const uint32_t o = N.rs[c] + (sB[r] - sB[rs]);
-    if (o >= R2) { atomicOr(err, kErrCorrupt); return; }
-    out_prim[o] = p;
-    out_node[o] = c;
-  }
-  if (above[r]) {
-    const uint32_t o = N.rs[c + 1] + (sA[r] - sA[rs]);
-    if (o >= R2) { atomicOr(err, kErrCorrupt); return; }
-    out_prim[o] = p;
-    out_node[o] = c + 1;
+template <int D>
+__device__ void place_children(const Table& T, uint32_t g, uint32_t p, const uint32_t* __restrict__ size,
+                               uint32_t* __restrict__ pos, uint32_t total) {
+  if (T.leaf[g]) return;
+  const uint32_t c0 = T.child0[g], c1 = T.child1[g];
+  if (c0 >= total || c1 >= total) return;
+  const uint32_t p1 = p + 1 + size[c0];
+  pos[c0] = p + 1;
+  pos[c1] = p1;
+  if constexpr (D > 1) {
+    place_children<D - 1>(T, c0, p + 1, size, pos, total);
+    place_children<D - 1>(T, c1, p1, size, pos, total);
   }
 }
-
-// Depth-first layout: subtree sizes bottom-up, positions top-down.
-__global__ void k_sizes(Table T, uint32_t lo, uint32_t hi, uint32_t* __restrict__ size, uint32_t total,
-                        uint32_t* err) {
-  uint32_t g = lo + blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= hi) return;
-  if (!T.leaf[g] && (T.child0[g] >= total || T.child1[g] >= total)) { atomicOr(err, kErrCorrupt); size[g] = 1; return; }
-  size[g] = T.leaf[g] ? 1u : 1u + size[T.child0[g]] + size[T.child1[g]];
-}
-
 __global__ void k_positions(Table T, uint32_t lo, uint32_t hi, const uint32_t* __restrict__ size,
                             uint32_t* __restrict__ pos, uint32_t total) {
-  uint32_t g = lo + blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= hi || T.leaf[g]) return;
-  if (T.child0[g] >= total || T.child1[g] >= total) return;
-  const uint32_t p = pos[g];
-  pos[T.child0[g]] = p + 1;
-  pos[T.child1[g]] = p + 1 + size[T.child0[g]];
+  const uint32_t g = lo + blockIdx.x * blockDim.x + threadIdx.x;
+  if (g < hi) place_children<kLayoutLevels>(T, g, pos[g], size, pos, total);
 }
 
 __global__ void k_leaf_counts(Table T, uint32_t total, const uint32_t* __restrict__ pos, uint32_t* __restrict__ cnt) {
@@ -1100,20 +1318,6 @@ __global__ void k_box_union(const float* __restrict__ aabb, uint32_t n, int32_t*
     }
 }
 
-__global__ void k_iota(uint32_t* v, uint32_t n) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) v[i] = i;
-}
-
-__global__ void k_root_box(const int32_t* lohi, float* box, float* root) {
-  int q = threadIdx.x;
-  if (q < 6) {
-    float v = ordered_to_float(lohi[q]);
-    box[q] = v;
-    root[q] = v;
-  }
-}
-
 // Grow a buffer keeping its first `used` bytes.
 cudaError_t grow_keep(DevBuf& b, size_t bytes, size_t used, cudaStream_t st) {
   if (bytes <= b.cap && b.p) return cudaSuccess;
@@ -1154,24 +1358,22 @@ LevelNodes carve(char* base, uint32_t cap) {
   LevelNodes L;
   size_t o = 0;
   auto take = [&](size_t bytes) { char* p = base + o; o += (bytes + 255) & ~size_t(255); return p; };
-  L.box = (float*)take((size_t)cap * 24);
-  L.depth = (int32_t*)take((size_t)cap * 4);
-  L.bad = (int32_t*)take((size_t)cap * 4);
+  L.lo = (float4*)take((size_t)cap * 16);
+  L.hi = (float4*)take((size_t)cap * 16);
+  L.plan = (uint4*)take((size_t)cap * 16);
+  L.best = (unsigned long long*)take((size_t)cap * 24);
+  L.split = (uint2*)take((size_t)cap * 8);
+  L.open = (uint32_t*)take((size_t)cap * 4);
   L.rs = (uint32_t*)take((size_t)cap * 4);
   L.rc = (uint32_t*)take((size_t)cap * 4);
-  L.axis0 = (int32_t*)take((size_t)cap * 4);
-  L.best = (unsigned long long*)take((size_t)cap * 24);
-  L.state = (int32_t*)take((size_t)cap * 4);
-  L.best_axis = (int32_t*)take((size_t)cap * 4);
-  L.best_off = (uint32_t*)take((size_t)cap * 4);
-  L.tsplit = (float*)take((size_t)cap * 4);
-  L.split_key = (uint32_t*)take((size_t)cap * 4);
-  L.split_v = (uint32_t*)take((size_t)cap * 4);
-  L.sa = (float4*)take((size_t)cap * 16);
-  L.plan = (uint4*)take((size_t)cap * 16);
+  L.depth = (int32_t*)take((size_t)cap * 4);
+  L.bad = (int32_t*)take((size_t)cap * 4);
+  L.axis = (int32_t*)take((size_t)cap * 4);
+  L.irank = (uint32_t*)take((size_t)cap * 4);
+  L.lofs = (uint32_t*)take((size_t)cap * 4);
   return L;
 }
-size_t level_bytes(uint32_t cap) { return (size_t)cap * 124 + 16 * 256; }
+size_t level_bytes(uint32_t cap) { return (size_t)cap * 112 + 13 * 256; }
 
 Table table_at(char* base, uint32_t cap) {
   Table T;
@@ -1187,11 +1389,8 @@ Table table_at(char* base, uint32_t cap) {
   return T;
 }
 size_t table_bytes(uint32_t cap) { return (size_t)cap * 28 + 8 * 256; }
-
-int bitlen(uint32_t v) {
-  int b = 0;
-  while (v) { ++b; v >>= 1; }
-  return b;
+uint32_t table_fits(size_t bytes) {  // largest capacity whose table fits
+  return bytes < 8 * 256 ? 0u : (uint32_t)std::min<size_t>((bytes - 8 * 256) / 28, 0xFFFFFFF0u);
 }
 
 }  // namespace
@@ -1238,53 +1437,41 @@ BuildResult build_kd_tree(const SceneView& s, int max_depth_cfg, AccelBuffers& a
   KD_TRY(sc.m1.ensure((size_t)n * 8 * 2), "KD scratch");
   uint32_t* ref_prim = sc.m1.as<uint32_t>();
   uint32_t* ref_node = ref_prim + (size_t)n;
-  count_launch();
-  k_iota<<<grid(n), kThreads, 0, st>>>(ref_prim, n);
-  KD_TRY(cudaMemsetAsync(ref_node, 0, (size_t)n * 4, st), "KD init");
   // root edge lists, one per axis, each sorted once by t (stable: equal t
-  // start-first, then by primitive id)
+  // start-first, then by primitive id), in one set of launches
   const uint32_t E0 = 2 * n;
-  KD_TRY(sc.keys.ensure((size_t)E0 * kEdgeWords * 4 + 64), "KD edges");
-  KD_TRY(sc.vals.ensure((size_t)E0 * 6 * 4 + 64), "KD edges");
-  EdgeLists el{sc.keys.as<uint32_t>(), (size_t)E0};
+  KD_TRY(sc.keys.ensure((size_t)E0 * 3 * 16 + 64), "KD edges");
+  KD_TRY(sc.vals.ensure((size_t)E0 * 12 * 4 + 64), "KD edges");
+  EdgeLists el{sc.keys.as<uint4>(), (size_t)E0};
   {
-    // the three lists in one set of launches
-    const size_t head = 3 * (kSortHistWords + kSortCounterWords), zwords = head + 3 * sort_status_words(E0, 4);
-    KD_TRY(sc.m4.ensure(zwords * 4 + 64), "KD sort");
+    const size_t head = 3 * (kSortHistWords + kSortCounterWords), zwords = (head + 3 * sort_status_words(E0, 4) + 1) & ~(size_t)1;
+    const uint32_t rtiles = (E0 + kThreads * kRootItems - 1) / (kThreads * kRootItems);
+    KD_TRY(sc.m4.ensure(zwords * 4 + (3 * (size_t)rtiles + 2) * 8 + 64), "KD sort");
     uint32_t* zero = sc.m4.as<uint32_t>();
-    uint32_t* alt = sc.vals.as<uint32_t>();
+    unsigned long long* rstatus = reinterpret_cast<unsigned long long*>(zero + zwords);
+    uint32_t* tk = sc.vals.as<uint32_t>();  // t, v of the three lists, and the sort's other buffers
+    uint32_t* tv = tk + 3 * (size_t)E0;
+    uint32_t* alt = tv + 3 * (size_t)E0;
     SortScratch ss{alt, alt + 3 * (size_t)E0, zero, zero + head, zero + 3 * kSortHistWords};
-    KD_TRY(cudaMemsetAsync(zero, 0, zwords * 4, st), "KD sort");
-    for (int ax = 0; ax < 3; ++ax) {
-      count_launch();
-      k_root_edges<<<grid(n), kThreads, 0, st>>>(aabb, n, ax, el.t(ax), el.v(ax));
-    }
-    launch_histogram(el.t(0), E0, 4, zero, st, 3, el.cap);
-    launch_onesweep(el.t(0), el.v(0), E0, 4, ss, err, st, 3, el.cap);
-    for (int ax = 0; ax < 3; ++ax) {
-      KD_TRY(cudaMemsetAsync(el.n(ax), 0, (size_t)E0 * 4, st), "KD root edges");
-      count_launch();
-      k_start_flags<<<grid(E0), kThreads, 0, st>>>(el.v(ax), E0, el.s(ax));
-      launch_scan_excl(el.s(ax), el.s(ax), E0, sc.vals.as<uint32_t>(), nullptr, st);  // in place
-    }
+    KD_TRY(cudaMemsetAsync(zero, 0, zwords * 4 + (3 * (size_t)rtiles + 2) * 8, st), "KD sort");
+    count_launch(2);
+    k_root_edges<<<grid(n), kThreads, 0, st>>>(aabb, n, tk, tv, ref_prim, ref_node);
+    launch_histogram(tk, E0, 4, zero, st, 3, E0);
+    launch_onesweep(tk, tv, E0, 4, ss, err, st, 3, E0);
+    k_root_lists<<<dim3(rtiles, 3), kThreads, 0, st>>>(tk, tv, E0, el, rstatus,
+                                                       reinterpret_cast<uint32_t*>(rstatus + 3 * (size_t)rtiles), rtiles, err);
     KD_TRY(cudaGetLastError(), "KD root edges");
   }
   // level 0 node
   KD_TRY(sc.m3.ensure(level_bytes(1)), "KD scratch");
   LevelNodes L = carve(sc.m3.as<char>(), 1);
-  {
-    const int32_t h_depth = depth0, h_bad = 0;
-    const uint32_t h_rs = 0, h_rc = n;
-    KD_TRY(cudaMemcpyAsync(L.depth, &h_depth, 4, cudaMemcpyHostToDevice, st), "KD init");
-    KD_TRY(cudaMemcpyAsync(L.bad, &h_bad, 4, cudaMemcpyHostToDevice, st), "KD init");
-    KD_TRY(cudaMemcpyAsync(L.rs, &h_rs, 4, cudaMemcpyHostToDevice, st), "KD init");
-    KD_TRY(cudaMemcpyAsync(L.rc, &h_rc, 4, cudaMemcpyHostToDevice, st), "KD init");
-    count_launch();
-    k_root_box<<<1, 32, 0, st>>>(lohi, L.box, a.root.as<float>());
-  }
+  count_launch();
+  k_root_node<<<1, 32, 0, st>>>(L, lohi, a.root.as<float>(), n, depth0);
+  KD_TRY(sc.host_words(), "KD scratch");
+  uint32_t* h_tot = sc.pinned;
   DevBuf& tabbuf = sc.m5;
   DevBuf& poolbuf = sc.m6;
-  uint32_t table_cap = 0, total = 0, pool_used = 0;
+  uint32_t table_cap = tabbuf.p ? table_fits(tabbuf.cap) : 0, total = 0, pool_used = 0;
   std::vector<uint32_t> level_lo;
   for (int level = 0; M > 0; ++level) {
     if (level > 200) return BuildResult::error(RQ_ERROR_INVALID_ARGUMENT, "KD tree deeper than 200 levels");
@@ -1294,112 +1481,98 @@ BuildResult build_kd_tree(const SceneView& s, int max_depth_cfg, AccelBuffers& a
       uint32_t ncap = (total + M) * 2 + 1024;
       DevBuf nb;
       KD_TRY(nb.ensure(table_bytes(ncap)), "KD table");
-      if (table_cap) {
+      if (total) {
         Table Told = table_at(tabbuf.as<char>(), table_cap), Tnew = table_at(nb.as<char>(), ncap);
         const size_t bytes = (size_t)total * 4;
-        KD_TRY(cudaMemcpyAsync(Tnew.leaf, Told.leaf, bytes, cudaMemcpyDeviceToDevice, st), "KD table");
-        KD_TRY(cudaMemcpyAsync(Tnew.axis, Told.axis, bytes, cudaMemcpyDeviceToDevice, st), "KD table");
-        KD_TRY(cudaMemcpyAsync(Tnew.split, Told.split, bytes, cudaMemcpyDeviceToDevice, st), "KD table");
-        KD_TRY(cudaMemcpyAsync(Tnew.child0, Told.child0, bytes, cudaMemcpyDeviceToDevice, st), "KD table");
-        KD_TRY(cudaMemcpyAsync(Tnew.child1, Told.child1, bytes, cudaMemcpyDeviceToDevice, st), "KD table");
-        KD_TRY(cudaMemcpyAsync(Tnew.count, Told.count, bytes, cudaMemcpyDeviceToDevice, st), "KD table");
-        KD_TRY(cudaMemcpyAsync(Tnew.pool_off, Told.pool_off, bytes, cudaMemcpyDeviceToDevice, st), "KD table");
-        KD_TRY(cudaStreamSynchronize(st), "KD table");
+        const void* from[] = {Told.leaf, Told.axis, Told.split, Told.child0, Told.child1, Told.count, Told.pool_off};
+        void* to[] = {Tnew.leaf, Tnew.axis, Tnew.split, Tnew.child0, Tnew.child1, Tnew.count, Tnew.pool_off};
+        for (int q = 0; q < 7; ++q) {
+          const cudaError_t ce = cudaMemcpyAsync(to[q], from[q], bytes, cudaMemcpyDeviceToDevice, st);
+          if (ce != cudaSuccess) {
+            nb.release();
+            return BuildResult::cuda_error(ce, "KD table");
+          }
+        }
+      }
+      const cudaError_t ce = cudaStreamSynchronize(st);
+      if (ce != cudaSuccess) {
+        nb.release();
+        return BuildResult::cuda_error(ce, "KD table");
       }
       tabbuf.release();
       tabbuf = nb;
-      nb.p = nullptr;
-      nb.cap = 0;
       table_cap = ncap;
     }
     Table T = table_at(tabbuf.as<char>(), table_cap);
-    // per-ref scratch: below / above flags and their scans (R + 1 each)
-    KD_TRY(ensure_after(sc.m2, ((size_t)R + 1) * 4 * 4 + scan_tmp_words((uint64_t)R + 1) * 8 + 64, st), "KD scratch");
-    uint32_t* below = sc.m2.as<uint32_t>();
-    uint32_t* above = below + (R + 1);
-    uint32_t* sB = above + (R + 1);
-    uint32_t* sA = sB + (R + 1);
-    uint32_t* tmp = sA + (R + 1);
+    // per-ref sides (R + 1)
+    KD_TRY(ensure_after(sc.m2, ((size_t)R + 1) * 8 + 64, st), "KD scratch");
+    uint2* sides = sc.m2.as<uint2>();
     // partition scratch: tile counts and the side flags as ballot words
     const uint32_t E2 = 2 * R;
-    const uint32_t runs = (E2 + kEdgeRun - 1) / kEdgeRun, tiles = (E2 + kEdgeTile - 1) / kEdgeTile;
+    const uint32_t runs = (E2 + kCostRun - 1) / kCostRun, tiles = (E2 + kEdgeTile - 1) / kEdgeTile;
     const size_t words = ((size_t)E2 + 31) / 32;
     KD_TRY(ensure_after(sc.m4, (size_t)tiles * 3 * 16 + words * 3 * 8 + 64, st), "KD edges");
     unsigned long long* tile_cnt = sc.m4.as<unsigned long long>();
     uint32_t* sideB = reinterpret_cast<uint32_t*>(tile_cnt + (size_t)tiles * 3 * 2);
     uint32_t* sideA = sideB + words * 3;
-    // interior ranks, leaf pool offsets, children's ref counts
-    KD_TRY(ensure_after(sc.m7, ((size_t)M + 1) * 4 * 4 + scan_tmp_words((uint64_t)M + 1) * 8 + 64, st), "KD scratch");
-    uint32_t* iflag = sc.m7.as<uint32_t>();
-    uint32_t* irank = iflag + (M + 1);
-    uint32_t* lcnt = irank + (M + 1);
-    uint32_t* lofs = lcnt + (M + 1);
-    uint32_t* mtmp = lofs + (M + 1);
-    uint32_t* mtot = mtmp + 2 * scan_tmp_words((uint64_t)M + 1) + 4;  // 4 totals
-    count_launch();
-    k_node_init<<<grid(std::max<uint64_t>(M, (uint64_t)R + 1)), kThreads, 0, st>>>(L, M, below, above, R);
-    if (E2) {
-      count_launch();
-      k_cost<<<grid(3ull * runs * 32), kThreads, 0, st>>>(el, E2, runs, M, L, err);
-    }
-    count_launch(2);
-    k_decide<<<grid((uint64_t)M + 1), kThreads, 0, st>>>(el, L, M, E2, iflag, lcnt, err);
-    k_classify<<<grid(R), kThreads, 0, st>>>(ref_prim, ref_node, R, M, aabb, L, below, above, err);
+    // look-back words of the level's two prefix sums and their tickets (cleared by k_cost), totals
+    const uint32_t dtiles = (M + kThreads - 1) / kThreads;
+    const uint32_t stiles = (R + 1 + kThreads * kSideItems - 1) / (kThreads * kSideItems);
+    const uint32_t clear_words = dtiles + stiles + 1;
+    KD_TRY(ensure_after(sc.m7, ((size_t)clear_words + 2) * 8 + 64, st), "KD scratch");
+    unsigned long long* status = sc.m7.as<unsigned long long>();
+    uint32_t* ticket = reinterpret_cast<uint32_t*>(status + dtiles + stiles);
+    uint32_t* totals = ticket + 2;
+    count_launch(3);
+    k_cost<<<grid(std::max<uint64_t>(3ull * runs * 32, 1)), kThreads, 0, st>>>(el, E2, runs, M, L, status, clear_words, err);
+    k_decide<<<dtiles, kThreads, 0, st>>>(el, L, M, E2, status, ticket, totals, err);
+    k_sides<<<stiles, kThreads, 0, st>>>(ref_prim, ref_node, R, M, aabb, L, sides, status + dtiles, ticket + 1, totals, err);
     KD_TRY(cudaGetLastError(), "KD split");
-    launch_scan2_excl(iflag, irank, lcnt, lofs, (uint64_t)M + 1, mtmp, mtot, mtot + 1, st);
-    launch_scan2_excl(below, sB, above, sA, (uint64_t)R + 1, tmp, mtot + 2, mtot + 3, st);
-    uint32_t h_tot[4] = {0, 0, 0, 0};
-    KD_TRY(cudaMemcpyAsync(h_tot, mtot, 16, cudaMemcpyDeviceToHost, st), "KD level");
-    KD_TRY(cudaStreamSynchronize(st), "KD level");
+    KD_TRY(cudaMemcpyAsync(h_tot, totals, 16, cudaMemcpyDeviceToHost, st), "KD level");
+    KD_TRY(cudaEventRecord(sc.host_ready, st), "KD level");
+    if (E2) {  // needs no totals: runs while the host reads them
+      count_launch();
+      k_part_count<<<3 * tiles, kThreads, 0, st>>>(el, E2, tiles, R, sides, sideB, sideA, tile_cnt, err);
+      if (tiles > kPartSelf) {
+        count_launch();
+        k_part_scan<<<3, 1024, 0, st>>>(tile_cnt, tiles);
+      }
+    }
+    KD_TRY(cudaEventSynchronize(sc.host_ready), "KD level");
     const uint32_t interiors = h_tot[0], leaf_refs = h_tot[1];
     const uint64_t R2l = (uint64_t)h_tot[2] + h_tot[3];
     if (2 * R2l >= (1ull << 31)) return BuildResult::error(RQ_ERROR_INVALID_ARGUMENT, "KD tree over 2^30 references");
     const uint32_t R2 = (uint32_t)R2l;
-    // next level nodes and child ref counts
+    // next level nodes
     const uint32_t M2 = 2 * interiors;
     DevBuf& nextbuf = (level & 1) ? sc.m3 : sc.keys_alt;  // alternate level buffers
-    KD_TRY(ensure_after(nextbuf, level_bytes(M2 ? M2 : 1) + ((size_t)M2 + 1) * 8 + scan_tmp_words((uint64_t)M2 + 1) * 4 + 64, st),
-           "KD scratch");
+    KD_TRY(ensure_after(nextbuf, level_bytes(M2 ? M2 : 1), st), "KD scratch");
     LevelNodes N = carve(nextbuf.as<char>(), M2 ? M2 : 1);
-    uint32_t* ccnt = reinterpret_cast<uint32_t*>(nextbuf.as<char>() + level_bytes(M2 ? M2 : 1));
-    uint32_t* coff = ccnt + (M2 + 1);
-    uint32_t* ctmp = coff + (M2 + 1);
     // leaf pool growth
     KD_TRY(grow_keep(poolbuf, ((size_t)pool_used + leaf_refs + 1) * 4, (size_t)pool_used * 4, st), "KD pool");
-    // lofs holds offsets relative to this level; shift by pool_used in the kernels
-    count_launch();
-    k_spawn<<<grid(M), kThreads, 0, st>>>(L, M, irank, sB, sA, lofs, pool_used, total, total + M, T, N, ccnt, M2,
-                                          err);
-    KD_TRY(cudaGetLastError(), "KD spawn");
-    if (M2) {
-      launch_scan_excl(ccnt, coff, (uint64_t)M2 + 1, ctmp, nullptr, st);
-      count_launch();
-      k_set_ref_starts<<<grid(M2), kThreads, 0, st>>>(N, M2, ccnt, coff);
-    }
-    // refs of the next level (separate buffer), leaf refs to the pool
+    // the next level's nodes and refs (separate buffer), leaf refs to the pool
     KD_TRY(ensure_after(sc.kd_refs, ((size_t)R2 + 1) * 8, st), "KD refs");
     uint32_t* out_prim = sc.kd_refs.as<uint32_t>();
     uint32_t* out_node = out_prim + (R2 + 1);
     count_launch();
-    k_emit_refs<<<grid(R), kThreads, 0, st>>>(ref_prim, ref_node, R, L, irank, below, above, sB, sA, N, out_prim,
-                                              out_node, lofs, pool_used, poolbuf.as<uint32_t>(), R2,
-                                              (uint32_t)(poolbuf.cap / 4), err);
-    KD_TRY(cudaGetLastError(), "KD emit");
+    k_spawn_emit<<<grid(std::max(R, M)), kThreads, 0, st>>>(L, M, sides, pool_used, total, total + M, T, N, M2, ref_prim,
+                                                            ref_node, R, out_prim, out_node, poolbuf.as<uint32_t>(), R2,
+                                                            (uint32_t)(poolbuf.cap / 4), err);
+    KD_TRY(cudaGetLastError(), "KD spawn");
     // the children's edge lists
-    KD_TRY(ensure_after(sc.vals, (size_t)R2 * 2 * kEdgeWords * 4 + 64, st), "KD edges");
-    EdgeLists eln{sc.vals.as<uint32_t>(), (size_t)R2 * 2};
+    KD_TRY(ensure_after(sc.vals, (size_t)R2 * 2 * 3 * 16 + 64, st), "KD edges");
+    EdgeLists eln{sc.vals.as<uint4>(), (size_t)R2 * 2};
     if (E2 && R2) {
-      count_launch(3);
-      k_part_count<<<3 * tiles, kThreads, 0, st>>>(el, E2, tiles, R, M, below, above, sideB, sideA, tile_cnt, err);
-      k_part_scan<<<3, 1024, 0, st>>>(tile_cnt, tiles);
-      k_partition<<<3 * tiles, kThreads, 0, st>>>(el, E2, tiles, L, sideB, sideA, tile_cnt, sB, sA, eln, 2 * R2, err);
+      count_launch();
+      const auto part = tiles > kPartSelf ? k_partition<true> : k_partition<false>;
+      part<<<3 * tiles, kThreads, 0, st>>>(el, E2, tiles, L, sideB, sideA, tile_cnt, sides, eln, 2 * R2, err);
       KD_TRY(cudaGetLastError(), "KD partition");
     }
     pool_used += leaf_refs;
     total += M;
     std::swap(sc.m1, sc.kd_refs);  // the children's refs become the current refs
     std::swap(sc.keys, sc.vals);   // and their edge lists
-    el = EdgeLists{sc.keys.as<uint32_t>(), (size_t)R2 * 2};
+    el = EdgeLists{sc.keys.as<uint4>(), (size_t)R2 * 2};
     ref_prim = sc.m1.as<uint32_t>();
     ref_node = ref_prim + (R2 + 1);
     R = R2;
@@ -1417,16 +1590,19 @@ BuildResult build_kd_tree(const SceneView& s, int max_depth_cfg, AccelBuffers& a
   uint32_t* off = cnt + (total + 1);
   uint32_t* ltmp = off + (total + 2);
   uint32_t* ltot = ltmp + scan_tmp_words((uint64_t)total + 2) + 4;
-  for (int lv = (int)level_lo.size() - 2; lv >= 0; --lv) {
+  const int levels = (int)level_lo.size() - 1;
+  for (int hi = levels; hi > 0;) {  // the deepest kLayoutLevels first
+    const int d = std::min(hi, kLayoutLevels), lv = hi - d;
     count_launch();
-    k_sizes<<<grid(level_lo[lv + 1] - level_lo[lv]), kThreads, 0, st>>>(T, level_lo[lv], level_lo[lv + 1], size,
-                                                                         total, err);
+    const auto k = d == 3 ? k_sizes<3> : d == 2 ? k_sizes<2> : k_sizes<1>;
+    k<<<grid(level_lo[lv + 1] - level_lo[lv]), kThreads, 0, st>>>(T, level_lo[lv], level_lo[lv + 1], size, total, err);
+    hi = lv;
   }
   KD_TRY(cudaMemsetAsync(pos, 0, 4, st), "KD layout");
-  for (size_t lv = 0; lv + 1 < level_lo.size(); ++lv) {
+  for (int lv = 0; lv < levels; lv += kLayoutLevels) {
     count_launch();
     k_positions<<<grid(level_lo[lv + 1] - level_lo[lv]), kThreads, 0, st>>>(T, level_lo[lv], level_lo[lv + 1], size,
-                                                                             pos, total);
+                                                                            pos, total);
   }
   count_launch();
   k_leaf_counts<<<grid((uint64_t)total + 1), kThreads, 0, st>>>(T, total, pos, cnt);

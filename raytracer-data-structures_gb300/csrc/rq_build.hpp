@@ -61,6 +61,14 @@ struct BuildScratch {
   DevBuf exact;               // rays that need the exact box test, set aside by FAST queries
   DevBuf heights;             // LBVH treelet restructuring: internal node heights (bytes)
   const uint32_t* stall = nullptr;  // sort test hook (SortScratch::stall); null in normal use
+  uint32_t* pinned = nullptr;       // host words that device totals are copied to
+  cudaEvent_t host_ready = nullptr; // recorded after such a copy
+  cudaError_t host_words() {
+    cudaError_t e = cudaSuccess;
+    if (!pinned) e = cudaMallocHost(&pinned, 64);
+    if (e == cudaSuccess && !host_ready) e = cudaEventCreateWithFlags(&host_ready, cudaEventDisableTiming);
+    return e;
+  }
   void release() {
     work.release();
     top.release();
@@ -70,6 +78,10 @@ struct BuildScratch {
     keys.release(); vals.release();
     m0.release(); m1.release(); m2.release(); m3.release(); m4.release(); m5.release(); m6.release(); m7.release();
     kd_refs.release();
+    if (pinned) cudaFreeHost(pinned);
+    if (host_ready) cudaEventDestroy(host_ready);
+    pinned = nullptr;
+    host_ready = nullptr;
   }
 };
 
