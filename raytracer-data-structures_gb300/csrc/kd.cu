@@ -34,6 +34,7 @@
 // four more: 36k spheres 4552 -> 1656 us, 82k triangles 5522 -> 2316, 330k
 // 9164 -> 5401, 998k 13824 -> 9880.
 #include <algorithm>
+#include <atomic>
 #include <vector>
 
 #include "rq_build.hpp"
@@ -1049,10 +1050,13 @@ __global__ void __launch_bounds__(128, ANY ? 9 : 8) k_trace_kd_shared(KdView kd,
   const uint32_t limit = 2u * n_nodes + 8u;  // meetings: a piece has a node of its ray behind it for every one
   int2 todo[kStackSize];                     // (node, bits of tMin)
   for (;;) {
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(work, grab);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= n) break;
+    // without a counter every warp has its rays by its place
+    uint32_t base = (blockIdx.x * 4 + (threadIdx.x >> 5)) * grab;
+    if (work) {
+      if (lane == 0) base = atomicAdd(work, grab);
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (base >= n) break;
+    }
     const uint32_t r = base + lane;
     const bool own = lane < grab && r < n;
     float first = 0.f, last = 0.f;  // the ray's interval in the root box
@@ -1253,25 +1257,39 @@ __global__ void __launch_bounds__(128, ANY ? 9 : 8) k_trace_kd_shared(KdView kd,
       if (ANY || !__any_sync(0xffffffffu, open)) break;
     }
     if constexpr (ANY) {
-      const bool occluded = (found >> lane) & 1u;
-      if (grab < 32u) {
-        if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
-      } else {
-        const uint32_t bits = __ballot_sync(0xffffffffu, occluded);
-        if (lane == 0) occ[base >> 5] = bits;
+      if (work) {
+        if (lane == 0) occ[base >> 5] = found;
+      } else {  // the block's warps put their bits together (grab is 8 or more)
+        __shared__ uint32_t bits[4];
+        if (lane == 0) bits[threadIdx.x >> 5] = found;
+        __syncthreads();
+        const uint32_t per = 32u / grab, word = blockIdx.x * grab / 8u + threadIdx.x;  // warps a word
+        if (threadIdx.x < grab / 8u && word < (n + 31) / 32) {
+          uint32_t w = 0;
+          for (uint32_t q = 0; q < per; ++q) w |= bits[threadIdx.x * per + q] << (q * grab);
+          occ[word] = w;
+        }
       }
     }
+    if (!work) break;
   }
 }
 
-template <typename K>
-uint32_t kd_resident_blocks(K k) {
-  int per_sm = 0, dev = 0, sms = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 128, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      sms < 1)
-    sms = 1;
-  return (uint32_t)(per_sm * sms);
+// Blocks of K (128 threads) resident on the current device at once (asked for
+// once per device).
+template <auto K>
+uint32_t kd_resident_blocks() {
+  static std::atomic<uint32_t> cache[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  uint32_t v = cache[dev & 63].load();
+  if (v == 0) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K, 128, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
+    v = (uint32_t)(per_sm * device_sm_count());
+    cache[dev & 63].store(v);
+  }
+  return v;
 }
 
 template <int KIND, bool ANY>
@@ -1279,19 +1297,29 @@ void dispatch_kd(int traversal, const KdView& v, uint32_t n_nodes, const float4*
                  uint32_t* occ, uint32_t* err, uint32_t* work, cudaStream_t s) {
   const unsigned g = (n + 127) / 128;
   if (work) {
-    cudaMemsetAsync(work, 0, 4, s);
     if (traversal == RQ_TRAVERSAL_REFERENCE || (ANY && n > kKdSharedAnyMax)) {
-      const auto k = traversal == RQ_TRAVERSAL_REFERENCE ? k_trace_kd_warps<KIND, ANY, true> : k_trace_kd_warps<KIND, ANY, false>;
-      k<<<std::min(g, kd_resident_blocks(k)), 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work);
+      cudaMemsetAsync(work, 0, 4, s);
+      if (traversal == RQ_TRAVERSAL_REFERENCE) {
+        const uint32_t blocks = kd_resident_blocks<k_trace_kd_warps<KIND, ANY, true>>();
+        k_trace_kd_warps<KIND, ANY, true><<<std::min(g, blocks), 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work);
+      } else {
+        const uint32_t blocks = kd_resident_blocks<k_trace_kd_warps<KIND, ANY, false>>();
+        k_trace_kd_warps<KIND, ANY, false><<<std::min(g, blocks), 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work);
+      }
       return;
     }
-    // fewer rays a warp when there are fewer rays than resident lanes, as for the BVH (trace.cu)
-    const auto k = k_trace_kd_shared<KIND, ANY>;
-    const uint32_t blocks = kd_resident_blocks(k);
+    // fewer rays a warp when there are fewer rays than resident lanes, and no
+    // counter when every warp's rays follow from its place, as for the BVH (trace.cu)
+    const uint32_t blocks = kd_resident_blocks<k_trace_kd_shared<KIND, ANY>>();
     uint32_t grab = 32u;
-    while (grab > 1u && (uint64_t)blocks * 4 * (grab / 2) >= n) grab /= 2;
-    if (ANY && grab < 32u) cudaMemsetAsync(occ, 0, (size_t)((n + 31) / 32) * 4, s);
-    k<<<std::min((n + 4 * grab - 1) / (4 * grab), blocks), 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work, grab);
+    while (grab > (ANY ? 8u : 1u) && (uint64_t)blocks * 4 * (grab / 2) >= n) grab /= 2;
+    const uint32_t need = (n + 4 * grab - 1) / (4 * grab);
+    if (need <= blocks) {
+      k_trace_kd_shared<KIND, ANY><<<need, 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, nullptr, grab);
+    } else {
+      cudaMemsetAsync(work, 0, 4, s);
+      k_trace_kd_shared<KIND, ANY><<<blocks, 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work, grab);
+    }
   } else if (traversal == RQ_TRAVERSAL_REFERENCE) {
     k_trace_kd<KIND, ANY, true><<<g, 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err);
   } else {

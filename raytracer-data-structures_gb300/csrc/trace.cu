@@ -16,6 +16,7 @@
 // Any-hit queries stop at the first accepted primitive and write one bit per
 // ray (warp ballot).
 #include <algorithm>
+#include <atomic>
 
 #include "trace_device.cuh"
 
@@ -61,30 +62,29 @@ __global__ void __launch_bounds__(kThreads, 10) k_trace_fast(Bvh2View bvh, const
 }
 
 // The FAST walk as persistent warps: a grid that fits on the GPU at once,
-// each warp taking the next rays from a counter (list[1]) until none are
+// each warp taking the next 32 rays from a counter (list[1]) until none are
 // left, so no warp idles while the slowest warp of its block finishes.  The
 // rays of a warp share its lanes (walk_warp, trace_device.cuh).  Rays that
 // need the exact box test (a direction component zero or too small for the
 // fused form) are not walked here but appended to list[2..] (count in
 // list[0]) for k_trace_exact, so this kernel carries only the fused walk.
 // UNIT: the LBVH's one-primitive leaves (4-byte stack entries).
-// grab: rays a warp takes at a time (at most 32).
 template <int KIND, bool ANY, bool UNIT>
 __global__ void __launch_bounds__(kThreads, kWalkBlocks) k_trace_warps(Bvh2View bvh, const float4* __restrict__ rays,
                                                           uint32_t n, float4* __restrict__ hits,
                                                           uint32_t* __restrict__ occ, uint32_t* err,
                                                           const uint32_t* __restrict__ perm,
-                                                          uint32_t* __restrict__ list, uint32_t grab) {
+                                                          uint32_t* __restrict__ list) {
   __shared__ WarpShare<ANY, false> share[kThreads / 32];
   WarpShare<ANY, false>& sh = share[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31;
   for (;;) {
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(list + 1, grab);
+    if (lane == 0) base = atomicAdd(list + 1, 32u);
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= n) break;
     const uint32_t i = base + lane;
-    const bool live = lane < grab && i < n;
+    const bool live = i < n;
     Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
     SlabRay sr = {};
     bool walk = live;
@@ -99,15 +99,68 @@ __global__ void __launch_bounds__(kThreads, kWalkBlocks) k_trace_warps(Bvh2View 
     }
     const bool own = walk;  // this lane's ray is walked here
     Closest c = {ray.tmax, kMiss, 0.f, 0.f};
-    const bool occluded = walk_warp<KIND, ANY, UNIT, kStackSize, false>(bvh, ray, sr, walk, grab < 32u, c, sh, err);
+    const bool occluded = walk_warp<KIND, ANY, UNIT, kStackSize, false>(bvh, ray, sr, walk, false, c, sh, err);
     const uint32_t r = (perm && live) ? __ldg(perm + i) : i;
     if (!ANY) {
       if (own) store_hit(hits, r, c);
-    } else if (perm || grab < 32u) {
+    } else if (perm) {
       if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
     } else {
       const uint32_t bits = __ballot_sync(0xffffffffu, occluded);
       if (lane == 0) occ[base >> 5] = bits;
+    }
+  }
+}
+
+// The same for launches whose warps the GPU holds at once: every warp has
+// its rays by its place (grab: rays a warp, 32 or fewer), and walks those
+// that need the exact box test itself first, so a query is this one launch:
+// no counter, list or second kernel to clear and start (1023 rays 26.7 ->
+// 21.8 us), and registers are not what bounds it.  Any hit without a perm:
+// the block's warps put their bits together (grab is 8 or more).
+template <int KIND, bool ANY, bool UNIT>
+__global__ void __launch_bounds__(kThreads) k_trace_once(Bvh2View bvh, const float4* __restrict__ rays, uint32_t n,
+                                                         float4* __restrict__ hits, uint32_t* __restrict__ occ,
+                                                         uint32_t* err, const uint32_t* __restrict__ perm,
+                                                         uint32_t grab) {
+  __shared__ WarpShare<ANY, false> share[kThreads / 32];
+  __shared__ uint32_t bits[kThreads / 32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t i = (blockIdx.x * (kThreads / 32) + warp) * grab + lane;
+  const bool live = lane < grab && i < n;
+  Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
+  SlabRay sr = {};
+  bool walk = live, exact_hit = false;
+  uint32_t r = i;
+  if (live) {
+    if (perm) r = __ldg(perm + i);
+    ray = load_ray(rays, r);
+    sr = slab_ray(ray.o, ray.d);
+  }
+  Closest c = {ray.tmax, kMiss, 0.f, 0.f};
+  if (live && zero_dir(sr)) {
+    uint32_t visits = 0, tests = 0;
+    exact_hit = walk_bvh2_form<KIND, ANY, false, kStackSize, true, UNIT>(bvh, ray, sr, c, visits, tests, err);
+    if (!ANY) store_hit(hits, r, c);
+    walk = false;
+  }
+  __syncwarp();
+  const bool own = walk;
+  const bool occluded =
+      walk_warp<KIND, ANY, UNIT, kStackSize, false>(bvh, ray, sr, walk, grab < 32u, c, share[warp], err) || exact_hit;
+  if (!ANY) {
+    if (own) store_hit(hits, r, c);
+  } else if (perm) {
+    if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
+  } else {
+    const uint32_t mine = __ballot_sync(0xffffffffu, occluded);
+    if (lane == 0) bits[warp] = mine;
+    __syncthreads();
+    const uint32_t per = 32u / grab, word = blockIdx.x * grab / 8u + threadIdx.x;  // warps a word
+    if (threadIdx.x < grab / 8u && word < (n + 31) / 32) {
+      uint32_t w = 0;
+      for (uint32_t q = 0; q < per; ++q) w |= bits[threadIdx.x * per + q] << (q * grab);
+      occ[word] = w;
     }
   }
 }
@@ -134,15 +187,43 @@ __global__ void __launch_bounds__(kThreads) k_trace_exact(Bvh2View bvh, const fl
   }
 }
 
-// Blocks of `k` (kThreads each) resident on the current device at once.
-template <typename K>
-uint32_t resident_blocks(K k) {
-  int per_sm = 0, dev = 0, sms = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      sms < 1)
-    sms = 1;
-  return (uint32_t)(per_sm * sms);
+// Blocks of K (kThreads each) resident on the current device at once (asked
+// for once per device).
+template <auto K>
+uint32_t resident_blocks() {
+  static std::atomic<uint32_t> cache[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  uint32_t v = cache[dev & 63].load();
+  if (v == 0) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K, kThreads, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
+    v = (uint32_t)(per_sm * device_sm_count());
+    cache[dev & 63].store(v);
+  }
+  return v;
+}
+
+template <int KIND, bool ANY, bool UNIT>
+void dispatch_fast(const Bvh2View& v, const float4* rays, uint32_t n, float4* hits, uint32_t* occ, uint32_t* err,
+                   const uint32_t* perm, uint32_t* exact, cudaStream_t s) {
+  constexpr uint32_t kWarps = kThreads / 32;
+  const uint32_t once = resident_blocks<k_trace_once<KIND, ANY, UNIT>>() * kWarps;  // warps
+  if (n <= once * 32u) {
+    // fewer rays a warp while every ray still has a warp to go to, so idle
+    // lanes share the work of few rays at once (1k random rays: 32 a warp 75
+    // us, one a warp 37)
+    uint32_t grab = 32u;
+    while (grab > (ANY && !perm ? 8u : 1u) && (uint64_t)once * (grab / 2) >= n) grab /= 2;
+    k_trace_once<KIND, ANY, UNIT><<<(n + grab * kWarps - 1) / (grab * kWarps), kThreads, 0, s>>>(v, rays, n, hits, occ, err,
+                                                                                            perm, grab);
+    return;
+  }
+  cudaMemsetAsync(exact, 0, 8, s);  // exact-ray count and work counter
+  k_trace_warps<KIND, ANY, UNIT><<<resident_blocks<k_trace_warps<KIND, ANY, UNIT>>(), kThreads, 0, s>>>(
+      v, rays, n, hits, occ, err, perm, exact);
+  count_launch();
+  k_trace_exact<KIND, ANY><<<kExactBlocks, kThreads, 0, s>>>(v, rays, exact, hits, occ, err);
 }
 
 // ------------------------------------------------ top levels in shared memory
@@ -883,19 +964,8 @@ void dispatch_bvh2(int traversal, const Bvh2View& v, const float4* rays, uint32_
   } else if (small_stack) {
     k_trace_fast<KIND, ANY, false, kDebugStack><<<g, kThreads, 0, s>>>(v, rays, n, hits, occ, err, nullptr, perm);
   } else if (exact) {
-    cudaMemsetAsync(exact, 0, 8, s);  // exact-ray count and work counter
-    const auto k = v.unit_leaves ? k_trace_warps<KIND, ANY, true> : k_trace_warps<KIND, ANY, false>;
-    // Fewer rays than the resident warps' lanes: fewer rays a warp, halved
-    // while every ray still has a warp to go to, so idle lanes share the work
-    // of few rays at once (1k random rays: 32 a warp 75 us, one a warp 37).
-    const uint32_t blocks = resident_blocks(k);
-    uint32_t grab = 32u;
-    while (grab > 1u && (uint64_t)blocks * (kThreads / 32) * (grab / 2) >= n) grab /= 2;
-    g = (n + grab * (kThreads / 32) - 1) / (grab * (kThreads / 32));
-    if (ANY && !perm && grab < 32u) cudaMemsetAsync(occ, 0, (size_t)((n + 31) / 32) * 4, s);
-    k<<<std::min(g, blocks), kThreads, 0, s>>>(v, rays, n, hits, occ, err, perm, exact, grab);
-    count_launch();
-    k_trace_exact<KIND, ANY><<<kExactBlocks, kThreads, 0, s>>>(v, rays, exact, hits, occ, err);
+    if (v.unit_leaves) dispatch_fast<KIND, ANY, true>(v, rays, n, hits, occ, err, perm, exact, s);
+    else dispatch_fast<KIND, ANY, false>(v, rays, n, hits, occ, err, perm, exact, s);
   } else {
     k_trace_fast<KIND, ANY, false><<<g, kThreads, 0, s>>>(v, rays, n, hits, occ, err, nullptr, perm);
   }
