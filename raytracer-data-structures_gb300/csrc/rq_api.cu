@@ -306,18 +306,14 @@ rq_status_t rq_scene_update(rq_ctx_t ctx, rq_scene_t s, const float* data, const
   const bool tri = s->kind == kTriangles;
   const size_t bytes = tri ? (size_t)s->nv * 12 : (size_t)s->n * 16;
   const size_t idx_bytes = (idx && tri) ? (size_t)s->n * 12 : 0;
-  void* dst = tri ? s->verts.p : s->sph.p;
-  if (dev) {
-    RQ_TRY_CUDA(ctx, cudaMemcpyAsync(dst, data, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-    if (idx_bytes) RQ_TRY_CUDA(ctx, cudaMemcpyAsync(s->idx.p, idx, idx_bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-    launch_validate(tri ? s->verts.as<float>() : nullptr, tri ? s->nv : 0, idx_bytes ? s->idx.as<uint32_t>() : nullptr,
-                    idx_bytes ? s->n : 0, tri ? nullptr : s->sph.as<float4>(), tri ? 0 : s->n, ctx->d_err, ctx->stream);
-    if (tri)
-      launch_pack_tris(s->verts.as<float>(), s->nv, s->idx.as<uint32_t>(), s->n, s->verts4.as<float4>(),
-                       idx_bytes ? s->idx4.as<uint4>() : nullptr, ctx->stream);
-    RQ_TRY(check_launch(ctx, "validate launch"));
-    return RQ_SUCCESS;  // device-side validation result arrives with rq_synchronize
-  }
+  // Enqueues the new geometry (device memory) into the scene.
+  auto take = [&](const float* from, const uint32_t* from_idx) -> rq_status_t {
+    launch_update(tri ? from : nullptr, tri ? s->nv : 0, s->verts.as<float>(), s->verts4.as<float4>(),
+                  idx_bytes ? from_idx : nullptr, idx_bytes ? s->n : 0, s->idx.as<uint32_t>(), s->idx4.as<uint4>(),
+                  tri ? nullptr : from, tri ? 0 : s->n, s->sph.as<float4>(), ctx->d_err, ctx->stream);
+    return check_launch(ctx, "update launch");
+  };
+  if (dev) return take(data, idx);  // the device-side check's result arrives with rq_synchronize
   // Host data: upload to a staging buffer, validate there on the device, and
   // only then replace the scene's geometry, so a rejected update leaves the
   // scene as it was.
@@ -331,14 +327,7 @@ rq_status_t rq_scene_update(rq_ctx_t ctx, rq_scene_t s, const float* data, const
                   tri ? nullptr : reinterpret_cast<const float4*>(st), tri ? 0 : s->n, ctx->d_err, ctx->stream);
   RQ_TRY(check_launch(ctx, "validate launch"));
   RQ_TRY(collect_device_errors(ctx));
-  RQ_TRY_CUDA(ctx, cudaMemcpyAsync(dst, st, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-  if (idx_bytes) RQ_TRY_CUDA(ctx, cudaMemcpyAsync(s->idx.p, st + off, idx_bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-  if (tri) {
-    launch_pack_tris(s->verts.as<float>(), s->nv, s->idx.as<uint32_t>(), s->n, s->verts4.as<float4>(),
-                     idx_bytes ? s->idx4.as<uint4>() : nullptr, ctx->stream);
-    RQ_TRY(check_launch(ctx, "pack launch"));
-  }
-  return RQ_SUCCESS;
+  return take(reinterpret_cast<const float*>(st), reinterpret_cast<const uint32_t*>(st + off));
 }
 
 rq_status_t rq_scene_destroy(rq_scene_t s) {

@@ -180,6 +180,11 @@ uint64_t launch_total();
 BuildResult trace_counted(int type, const SceneView& s, const AccelBuffers& a, bool any, const QueryTarget& q,
                           unsigned long long* counters, uint32_t* err, cudaStream_t st);
 
+// Checks, copies and packs new geometry (device memory) into a scene's arrays:
+// nv vertices, nt triangles (0: the scene keeps its own), n spheres.
+void launch_update(const float* verts, uint32_t nv, float* to_verts, float4* verts4, const uint32_t* idx, uint32_t nt,
+                   uint32_t* to_idx, uint4* idx4, const float* sph, uint32_t n, float4* to_sph, uint32_t* err,
+                   cudaStream_t st);
 void launch_validate(const float* verts, uint32_t nv, const uint32_t* idx, uint32_t nt,
                      const float4* sph, uint32_t n, uint32_t* err, cudaStream_t st);
 
