@@ -168,6 +168,11 @@ constexpr int kDebugStack = 8;
 void launch_trace_bvh2(int kind, int traversal, bool any, const Bvh2View& v, const float4* rays,
                        uint32_t n, float4* hits, uint32_t* occ, uint32_t* err, cudaStream_t s,
                        const uint32_t* perm = nullptr, bool small_stack = false, uint32_t* exact = nullptr);
+// FAST queries over the rays of a list whose length is on the device (results
+// at the rays' own indices; occ zeroed by the caller): no host wait between
+// the kernel that fills the list and the query.
+void launch_trace_bvh2_list(int kind, bool any, const Bvh2View& v, const float4* rays, float4* hits, uint32_t* occ,
+                            uint32_t* err, const uint32_t* list, const uint32_t* count, cudaStream_t s);
 // boxIntersect's candidate lists: ids == null counts per ray into counts;
 // otherwise writes each ray's ids at offs[r] (and checks the counts).
 // Count pass (ids null): counts[r] and *total (64-bit sum, zeroed by the

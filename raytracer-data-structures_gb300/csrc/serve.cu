@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kThreads) k_serve_rays(const ServeReq* __restr
   if (r >= nray) return;
   const uint32_t q = segment_of(roff, n_req, r);
   V3 o, d;
-  view_ray(reqs[q].v, r - __ldg(roff + q), o, d);
+  view_ray(reqs[q].v, view_basis(reqs[q].v), r - __ldg(roff + q), o, d);
   store_ray(rays, r, o, 0.f, d, __int_as_float(0x7F800000));
   cw[r] = make_float4(0.f, 0.f, 0.f, 1.f);
 }

@@ -118,50 +118,68 @@ __global__ void __launch_bounds__(kThreads, kWalkBlocks) k_trace_warps(Bvh2View 
 // no counter, list or second kernel to clear and start (1023 rays 26.7 ->
 // 21.8 us), and registers are not what bounds it.  Any hit without a perm:
 // the block's warps put their bits together (grab is 8 or more).
+// n_dev (optional): the ray count is read on the device (a list that an
+// earlier kernel filled); the grid is then the resident one, grab follows
+// from the count by the host's rule and warps stride over what is left.
+__host__ __device__ inline uint32_t rays_a_warp(uint32_t warps, uint32_t n, uint32_t least) {
+  uint32_t grab = 32u;
+  while (grab > least && (uint64_t)warps * (grab / 2) >= n) grab /= 2;
+  return grab;
+}
+
 template <int KIND, bool ANY, bool UNIT>
 __global__ void __launch_bounds__(kThreads) k_trace_once(Bvh2View bvh, const float4* __restrict__ rays, uint32_t n,
                                                          float4* __restrict__ hits, uint32_t* __restrict__ occ,
                                                          uint32_t* err, const uint32_t* __restrict__ perm,
-                                                         uint32_t grab) {
+                                                         uint32_t grab, const uint32_t* __restrict__ n_dev) {
   __shared__ WarpShare<ANY, false> share[kThreads / 32];
   __shared__ uint32_t bits[kThreads / 32];
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t i = (blockIdx.x * (kThreads / 32) + warp) * grab + lane;
-  const bool live = lane < grab && i < n;
-  Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
-  SlabRay sr = {};
-  bool walk = live, exact_hit = false;
-  uint32_t r = i;
-  if (live) {
-    if (perm) r = __ldg(perm + i);
-    ray = load_ray(rays, r);
-    sr = slab_ray(ray.o, ray.d);
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = gridDim.x * (kThreads / 32);
+  if (n_dev) {
+    n = __ldg(n_dev);
+    grab = rays_a_warp(warps, n, 1u);
   }
-  Closest c = {ray.tmax, kMiss, 0.f, 0.f};
-  if (live && zero_dir(sr)) {
-    uint32_t visits = 0, tests = 0;
-    exact_hit = walk_bvh2_form<KIND, ANY, false, kStackSize, true, UNIT>(bvh, ray, sr, c, visits, tests, err);
-    if (!ANY) store_hit(hits, r, c);
-    walk = false;
-  }
-  __syncwarp();
-  const bool own = walk;
-  const bool occluded =
-      walk_warp<KIND, ANY, UNIT, kStackSize, false>(bvh, ray, sr, walk, grab < 32u, c, share[warp], err) || exact_hit;
-  if (!ANY) {
-    if (own) store_hit(hits, r, c);
-  } else if (perm) {
-    if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
-  } else {
-    const uint32_t mine = __ballot_sync(0xffffffffu, occluded);
-    if (lane == 0) bits[warp] = mine;
-    __syncthreads();
-    const uint32_t per = 32u / grab, word = blockIdx.x * grab / 8u + threadIdx.x;  // warps a word
-    if (threadIdx.x < grab / 8u && word < (n + 31) / 32) {
-      uint32_t w = 0;
-      for (uint32_t q = 0; q < per; ++q) w |= bits[threadIdx.x * per + q] << (q * grab);
-      occ[word] = w;
+  for (uint32_t base = (blockIdx.x * (kThreads / 32) + warp) * grab;;) {
+    const uint32_t i = base + lane;
+    const bool live = lane < grab && i < n;
+    Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
+    SlabRay sr = {};
+    bool walk = live, exact_hit = false;
+    uint32_t r = i;
+    if (live) {
+      if (perm) r = __ldg(perm + i);
+      ray = load_ray(rays, r);
+      sr = slab_ray(ray.o, ray.d);
     }
+    Closest c = {ray.tmax, kMiss, 0.f, 0.f};
+    if (live && zero_dir(sr)) {
+      uint32_t visits = 0, tests = 0;
+      exact_hit = walk_bvh2_form<KIND, ANY, false, kStackSize, true, UNIT>(bvh, ray, sr, c, visits, tests, err);
+      if (!ANY) store_hit(hits, r, c);
+      walk = false;
+    }
+    __syncwarp();
+    const bool own = walk;
+    const bool occluded =
+        walk_warp<KIND, ANY, UNIT, kStackSize, false>(bvh, ray, sr, walk, grab < 32u, c, share[warp], err) || exact_hit;
+    if (!ANY) {
+      if (own) store_hit(hits, r, c);
+    } else if (perm) {
+      if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
+    } else {  // one round: every warp of the block is here
+      const uint32_t mine = __ballot_sync(0xffffffffu, occluded);
+      if (lane == 0) bits[warp] = mine;
+      __syncthreads();
+      const uint32_t per = 32u / grab, word = blockIdx.x * grab / 8u + threadIdx.x;  // warps a word
+      if (threadIdx.x < grab / 8u && word < (n + 31) / 32) {
+        uint32_t w = 0;
+        for (uint32_t q = 0; q < per; ++q) w |= bits[threadIdx.x * per + q] << (q * grab);
+        occ[word] = w;
+      }
+    }
+    if (!n_dev) break;
+    base += warps * grab;
+    if (base >= n) break;
   }
 }
 
@@ -213,10 +231,9 @@ void dispatch_fast(const Bvh2View& v, const float4* rays, uint32_t n, float4* hi
     // fewer rays a warp while every ray still has a warp to go to, so idle
     // lanes share the work of few rays at once (1k random rays: 32 a warp 75
     // us, one a warp 37)
-    uint32_t grab = 32u;
-    while (grab > (ANY && !perm ? 8u : 1u) && (uint64_t)once * (grab / 2) >= n) grab /= 2;
+    const uint32_t grab = rays_a_warp(once, n, ANY && !perm ? 8u : 1u);
     k_trace_once<KIND, ANY, UNIT><<<(n + grab * kWarps - 1) / (grab * kWarps), kThreads, 0, s>>>(v, rays, n, hits, occ, err,
-                                                                                            perm, grab);
+                                                                                            perm, grab, nullptr);
     return;
   }
   cudaMemsetAsync(exact, 0, 8, s);  // exact-ray count and work counter
@@ -971,6 +988,13 @@ void dispatch_bvh2(int traversal, const Bvh2View& v, const float4* rays, uint32_
   }
 }
 
+template <int KIND, bool ANY, bool UNIT>
+void dispatch_list(const Bvh2View& v, const float4* rays, float4* hits, uint32_t* occ, uint32_t* err,
+                   const uint32_t* list, const uint32_t* count, cudaStream_t s) {
+  k_trace_once<KIND, ANY, UNIT><<<resident_blocks<k_trace_once<KIND, ANY, UNIT>>(), kThreads, 0, s>>>(
+      v, rays, 0, hits, occ, err, list, 0, count);
+}
+
 template <int KIND, bool ANY>
 void dispatch_brute(int traversal, const float4* prims, uint32_t np, const float4* rays, uint32_t n,
                     float4* hits, uint32_t* occ, cudaStream_t s) {
@@ -1018,6 +1042,17 @@ void launch_trace_bvh2(int kind, int traversal, bool any, const Bvh2View& v, con
     if (any) dispatch_bvh2<kSpheres, true>(traversal, v, rays, n, hits, occ, err, perm, small_stack, exact, s);
     else dispatch_bvh2<kSpheres, false>(traversal, v, rays, n, hits, occ, err, perm, small_stack, exact, s);
   }
+}
+
+void launch_trace_bvh2_list(int kind, bool any, const Bvh2View& v, const float4* rays, float4* hits, uint32_t* occ,
+                            uint32_t* err, const uint32_t* list, const uint32_t* count, cudaStream_t s) {
+  count_launch();
+  const bool tri = kind == kTriangles, unit = v.unit_leaves != 0;
+  const auto run = any ? (tri ? (unit ? dispatch_list<kTriangles, true, true> : dispatch_list<kTriangles, true, false>)
+                              : (unit ? dispatch_list<kSpheres, true, true> : dispatch_list<kSpheres, true, false>))
+                       : (tri ? (unit ? dispatch_list<kTriangles, false, true> : dispatch_list<kTriangles, false, false>)
+                              : (unit ? dispatch_list<kSpheres, false, true> : dispatch_list<kSpheres, false, false>));
+  run(v, rays, hits, occ, err, list, count, s);
 }
 
 void launch_trace_bvh4(int kind, bool any, const Bvh4View& v, const float4* rays, uint32_t n, float4* hits,

@@ -33,27 +33,35 @@ namespace rq {
 namespace {
 
 constexpr int kThreads = 128;
+constexpr uint64_t kDeviceCountsMax = 1u << 20;  // samples of a frame queued without reading list lengths back
 
-__global__ void __launch_bounds__(kThreads) k_view_rays(ViewDev v, uint64_t nray, float4* __restrict__ rays,
-                                                        float4* __restrict__ cw) {
-  uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nray) return;
-  V3 o, d;
-  view_ray(v, r, o, d);
-  store_ray(rays, r, o, 0.f, d, __int_as_float(0x7F800000));
-  cw[r] = make_float4(0.f, 0.f, 0.f, 1.f);
+// kRaysPer rays a thread: the camera's axes (two normalisations) are worked
+// out once for them, and rays are stored 16 bytes a lane.
+constexpr int kRaysPer = 4;
+__global__ void __launch_bounds__(kThreads) k_view_rays(ViewDev v, uint32_t nray, float4* __restrict__ rays) {
+  const ViewBasis b = view_basis(v);
+  const uint32_t r0 = blockIdx.x * (kThreads * kRaysPer) + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < kRaysPer; ++k) {
+    const uint32_t r = r0 + (uint32_t)k * kThreads;
+    if (r >= nray) return;
+    V3 o, d;
+    view_ray(v, b, r, o, d);
+    store_ray(rays, r, o, 0.f, d, __int_as_float(0x7F800000));
+  }
 }
 
 // counters[0] += shadow rays emitted, counters[1] += mirror rays emitted.
 template <int KIND>
-__global__ void __launch_bounds__(kThreads) k_shade_hits(ViewDev v, SceneView sc, uint64_t nray, bool last,
+__global__ void __launch_bounds__(kThreads) k_shade_hits(ViewDev v, SceneView sc, uint64_t nray, bool first,
+                                                         bool last,
                                                          float4* __restrict__ rays, const float4* __restrict__ hits,
                                                          float4* __restrict__ shadow, float4* __restrict__ cw,
                                                          float4* __restrict__ pend,
                                                          unsigned long long* __restrict__ counters) {
   uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   bool emit_shadow = false, emit_mirror = false;
-  if (r < nray) shade_sample<KIND>(v, sc, r, last, rays, hits, shadow, cw, pend, emit_shadow, emit_mirror);
+  if (r < nray) shade_sample<KIND>(v, sc, r, last, rays, hits, shadow, cw, pend, emit_shadow, emit_mirror, first);
   const uint32_t bs = __ballot_sync(0xffffffffu, emit_shadow), bm = __ballot_sync(0xffffffffu, emit_mirror);
   if ((threadIdx.x & 31) == 0 && (bs | bm)) {
     if (bs) atomicAdd(counters, (unsigned long long)__popc(bs));
@@ -73,51 +81,70 @@ __global__ void __launch_bounds__(kThreads) k_pixels(uint64_t npix, uint32_t spp
   if (p < npix) resolve_pixel(p, spp, cw, pixels, rgb);
 }
 
-// Warp-aggregated append of r to list when `take` (one atomic per warp).
-__device__ __forceinline__ void warp_append(bool take, uint32_t r, uint32_t* __restrict__ list,
-                                            uint32_t* __restrict__ count) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t bits = __ballot_sync(0xffffffffu, take);
-  if (!bits) return;
-  const uint32_t leader = __ffs(bits) - 1;
-  uint32_t base = 0;
-  if (lane == leader) base = atomicAdd(count, (uint32_t)__popc(bits));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  if (take) list[base + __popc(bits & ((1u << lane) - 1u))] = r;
-}
-
-// Shading over a list of live samples (all samples when list is null) that
-// also compacts the samples that emitted a shadow ray and a mirror ray into
-// s_list / m_list (counts[0], counts[1]).
+// Shading over a list of live samples (all samples, at the first depth, when
+// list is null) that also compacts the samples that emitted a shadow ray and
+// a mirror ray into s_list / m_list (counts[0], counts[1]): the block's
+// samples take their places with one 64-bit add on both counts (one add a
+// warp and list, and two on the ray counters, were 400k adds on two lines at
+// 33M samples).  n_dev (optional): the list's length, on the device.
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) k_shade_list(ViewDev v, SceneView sc, const uint32_t* __restrict__ list,
-                                                         uint32_t n, bool last, float4* __restrict__ rays,
+                                                         uint32_t n, const uint32_t* __restrict__ n_dev, bool last,
+                                                         float4* __restrict__ rays,
                                                          const float4* __restrict__ hits, float4* __restrict__ shadow,
                                                          float4* __restrict__ cw, float4* __restrict__ pend,
                                                          uint32_t* __restrict__ s_list, uint32_t* __restrict__ m_list,
-                                                         uint32_t* __restrict__ counts,
+                                                         unsigned long long* __restrict__ counts,
                                                          unsigned long long* __restrict__ counters) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ uint32_t ws[kThreads / 32], wm[kThreads / 32], base_s, base_m;
+  if (n_dev) {
+    n = __ldg(n_dev);
+    if (blockIdx.x * blockDim.x >= n) return;  // whole blocks
+  }
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   bool es = false, em = false;
   uint32_t r = 0;
   if (i < n) {
     r = list ? __ldg(list + i) : i;
-    shade_sample<KIND, true>(v, sc, r, last, rays, hits, shadow, cw, pend, es, em);
+    shade_sample<KIND, true>(v, sc, r, last, rays, hits, shadow, cw, pend, es, em, list == nullptr);
   }
-  warp_append(es, r, s_list, counts);
-  warp_append(em, r, m_list, counts + 1);
   const uint32_t bs = __ballot_sync(0xffffffffu, es), bm = __ballot_sync(0xffffffffu, em);
-  if ((threadIdx.x & 31) == 0 && (bs | bm)) {
-    if (bs) atomicAdd(counters, (unsigned long long)__popc(bs));
-    if (bm) atomicAdd(counters + 1, (unsigned long long)__popc(bm));
+  if (lane == 0) {
+    ws[warp] = __popc(bs);
+    wm[warp] = __popc(bm);
   }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t ns = 0, nm = 0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      ns += ws[w];
+      nm += wm[w];
+    }
+    if (ns | nm) {
+      const unsigned long long at = atomicAdd(counts, ((unsigned long long)nm << 32) | ns);
+      base_s = (uint32_t)at;
+      base_m = (uint32_t)(at >> 32);
+      if (ns) atomicAdd(counters, (unsigned long long)ns);
+      if (nm) atomicAdd(counters + 1, (unsigned long long)nm);
+    }
+  }
+  __syncthreads();
+  uint32_t ps = base_s, pm = base_m;
+  for (uint32_t w = 0; w < warp; ++w) {
+    ps += ws[w];
+    pm += wm[w];
+  }
+  const uint32_t lt = (1u << lane) - 1u;
+  if (es) s_list[ps + __popc(bs & lt)] = r;
+  if (em) m_list[pm + __popc(bm & lt)] = r;
 }
 
 __global__ void __launch_bounds__(kThreads) k_accum_list(const uint32_t* __restrict__ list, uint32_t n,
+                                                         const uint32_t* __restrict__ n_dev,
                                                          const uint32_t* __restrict__ bits,
                                                          const float4* __restrict__ pend, float4* __restrict__ cw) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) shadow_accum(__ldg(list + i), bits, pend, cw);
+  if (i < (n_dev ? __ldg(n_dev) : n)) shadow_accum(__ldg(list + i), bits, pend, cw);
 }
 
 }  // namespace
@@ -145,7 +172,7 @@ cudaError_t render_view(int type, const SceneView& s, const AccelBuffers& a, con
   uint32_t* bits = rs.bits.as<uint32_t>();
   const unsigned gr = (unsigned)((nray + kThreads - 1) / kThreads);
   count_launch();
-  k_view_rays<<<gr, kThreads, 0, st>>>(v, nray, rays, cw);
+  k_view_rays<<<(unsigned)((nray + kThreads * kRaysPer - 1) / (kThreads * kRaysPer)), kThreads, 0, st>>>(v, (uint32_t)nray, rays);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const bool compact = (type == RQ_LBVH || type == RQ_BVH) && cfg.traversal == RQ_TRAVERSAL_FAST;
   if (compact) {
@@ -162,7 +189,7 @@ cudaError_t render_view(int type, const SceneView& s, const AccelBuffers& a, con
     uint32_t* next = rs.list_a.as<uint32_t>();
     uint32_t* spare = rs.list_b.as<uint32_t>();
     uint32_t* slist = rs.list_s.as<uint32_t>();
-    uint32_t* counts = rs.list_n.as<uint32_t>();
+    uint32_t* counts = rs.list_n.as<uint32_t>();  // [0] shadow rays, [1] mirror rays of this depth, [2], [3] of the last
     uint32_t n_live = (uint32_t)nray;
     const Bvh2View bv{a.nodes.as<const float4>(), a.prims.as<const float4>(), a.order.as<const uint32_t>(),
                       a.root.as<const float>(), a.n_nodes, a.n_slots, a.unit_leaves ? 1u : 0u};
@@ -170,8 +197,16 @@ cudaError_t render_view(int type, const SceneView& s, const AccelBuffers& a, con
                       a.root.as<const float>(), a.n_nodes, a.n_slots};
     const Bvh8View b8{a.nodes4.as<const float4>(), a.prims.as<const float4>(), a.order.as<const uint32_t>(),
                       a.root.as<const float>(), a.n_nodes, a.n_slots};
+    // Small frames leave the lists' lengths on the device (queries and kernels
+    // read them there, grids cover every sample), so the frame is queued
+    // without a wait (some 15 us a depth); large ones read them back, which
+    // sizes the launches.
+    const bool on_device = nray <= kDeviceCountsMax && a.node_width == 2;
+    const unsigned g_all = (unsigned)((nray + kThreads - 1) / kThreads);
     for (uint32_t depth = 0; depth <= v.bounces && n_live > 0; ++depth) {
       const bool last = depth == v.bounces;
+      uint32_t* now = counts + 2 * (depth & 1u);
+      const uint32_t* live_n = on_device && depth ? counts + 2 * ((depth + 1) & 1u) + 1 : nullptr;
       if (depth == 0) {
         QueryTarget q;
         q.rays = rays;
@@ -182,6 +217,8 @@ cudaError_t render_view(int type, const SceneView& s, const AccelBuffers& a, con
           *status = br.status;
           return br.cuda;
         }
+      } else if (on_device) {
+        launch_trace_bvh2_list(s.kind, false, bv, rays, hits, nullptr, err, live, live_n, st);
       } else if (a.node_width == 4) {
         launch_trace_bvh4(s.kind, false, b4, rays, n_live, hits, nullptr, err, st, live);
       } else if (a.node_width == 8) {
@@ -190,24 +227,25 @@ cudaError_t render_view(int type, const SceneView& s, const AccelBuffers& a, con
         launch_trace_bvh2(s.kind, RQ_TRAVERSAL_FAST, false, bv, rays, n_live, hits, nullptr, err, st, live, false,
                           exact);
       }
-      if ((e = cudaMemsetAsync(counts, 0, 8, st)) != cudaSuccess) return e;
+      if ((e = cudaMemsetAsync(now, 0, 8, st)) != cudaSuccess) return e;
       count_launch();
-      const unsigned gl = (n_live + kThreads - 1) / kThreads;
-      if (s.kind == kTriangles)
-        k_shade_list<kTriangles><<<gl, kThreads, 0, st>>>(v, s, live, n_live, last, rays, hits, shadow, cw, pend,
-                                                           slist, next, counts, counters);
-      else
-        k_shade_list<kSpheres><<<gl, kThreads, 0, st>>>(v, s, live, n_live, last, rays, hits, shadow, cw, pend,
-                                                         slist, next, counts, counters);
+      const unsigned gl = on_device ? g_all : (n_live + kThreads - 1) / kThreads;
+      const auto shade = s.kind == kTriangles ? k_shade_list<kTriangles> : k_shade_list<kSpheres>;
+      shade<<<gl, kThreads, 0, st>>>(v, s, live, n_live, live_n, last, rays, hits, shadow, cw, pend, slist, next,
+                                     reinterpret_cast<unsigned long long*>(now), counters);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
-      uint32_t host_counts[2] = {0, 0};
-      if ((e = cudaMemcpyAsync(host_counts, counts, 8, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
-      if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+      uint32_t host_counts[2] = {(uint32_t)nray, (uint32_t)nray};
+      if (!on_device) {
+        if ((e = cudaMemcpyAsync(host_counts, now, 8, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
+        if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+      }
       const uint32_t n_shadow = host_counts[0];
       if (n_shadow > 0) {
         // occlusion bits are indexed by sample: clear them all, trace the list
         if ((e = cudaMemsetAsync(bits, 0, ((nray + 31) / 32) * 4, st)) != cudaSuccess) return e;
-        if (a.node_width == 4)
+        if (on_device)
+          launch_trace_bvh2_list(s.kind, true, bv, shadow, nullptr, bits, err, slist, now, st);
+        else if (a.node_width == 4)
           launch_trace_bvh4(s.kind, true, b4, shadow, n_shadow, nullptr, bits, err, st, slist);
         else if (a.node_width == 8)
           launch_trace_bvh8(s.kind, true, b8, shadow, n_shadow, nullptr, bits, err, st, slist);
@@ -215,7 +253,8 @@ cudaError_t render_view(int type, const SceneView& s, const AccelBuffers& a, con
           launch_trace_bvh2(s.kind, RQ_TRAVERSAL_FAST, true, bv, shadow, n_shadow, nullptr, bits, err, st, slist,
                             false, exact);
         count_launch();
-        k_accum_list<<<(n_shadow + kThreads - 1) / kThreads, kThreads, 0, st>>>(slist, n_shadow, bits, pend, cw);
+        k_accum_list<<<(n_shadow + kThreads - 1) / kThreads, kThreads, 0, st>>>(slist, n_shadow, on_device ? now : nullptr,
+                                                                                bits, pend, cw);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
       }
       n_live = host_counts[1];
@@ -238,9 +277,9 @@ cudaError_t render_view(int type, const SceneView& s, const AccelBuffers& a, con
       }
       count_launch();
       if (s.kind == kTriangles)
-        k_shade_hits<kTriangles><<<gr, kThreads, 0, st>>>(v, s, nray, last, rays, hits, shadow, cw, pend, counters);
+        k_shade_hits<kTriangles><<<gr, kThreads, 0, st>>>(v, s, nray, depth == 0, last, rays, hits, shadow, cw, pend, counters);
       else
-        k_shade_hits<kSpheres><<<gr, kThreads, 0, st>>>(v, s, nray, last, rays, hits, shadow, cw, pend, counters);
+        k_shade_hits<kSpheres><<<gr, kThreads, 0, st>>>(v, s, nray, depth == 0, last, rays, hits, shadow, cw, pend, counters);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
       QueryTarget qs;
       qs.rays = shadow;
