@@ -831,13 +831,12 @@ def run_serve_leg(args):
 
 def build_bytes_per_tri(treelets=False):
     """Compulsory bytes per triangle of the LBVH build kernels:
-    bounds 6 (12 B per vertex, 0.5 vertex per triangle) + Morton 26 (12 B indices,
-    6 B vertices, 8 B code/index write) + 4 sort passes x 16 + Karras 28 (code
-    read 4, links 16, parents 8) + refit 150 (order 4, indices 12, vertices 6,
-    48 B payload write, 24 B child box write, 48 B sibling reread per internal
-    node, 4 B parent link, 4 B flag); with the treelet pass + 140 per internal
-    node (64 B node read and write, 4 B cost write, 8 B parent links)."""
-    return 6 + 26 + 64 + 28 + 150 + (140 if treelets else 0)
+    bounds 6 (12 B per vertex, 0.5 vertex per triangle) + Morton 22 (12 B indices,
+    6 B vertices, 4 B code write) + 4 sort passes x 16 + tree 138 (code 4, order 4,
+    indices 12, vertices 6, 48 B payload and 64 B node write); with the treelet
+    pass + 140 per internal node (64 B node read and write, 4 B cost write, 8 B
+    parent links)."""
+    return 6 + 22 + 64 + 138 + (140 if treelets else 0)
 
 
 def run_e2e(eng, scene, acc, verts, idx, primary, secondary, shadow, args, sort_choice):

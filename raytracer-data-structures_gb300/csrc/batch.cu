@@ -1,10 +1,10 @@
 // Batched LBVH build: every scene of a batch in one pass of kernels (scene
-// boxes, Morton codes, one segmented radix sort, Karras topology, refit)
-// instead of one pipeline per scene.  Each scene's arrays come out exactly
+// boxes, Morton codes, one segmented radix sort, the trees) instead of one
+// pipeline per scene.  Each scene's arrays come out exactly
 // as a single build would write them (same device helpers, same stable
 // order), laid out back to back in one allocation:
 //   prims, order, codes at slot offset P_s (P = prefix sum of primitive counts)
-//   internal nodes at I_s = P_s - s, parent links at 2 P_s - s
+//   internal nodes at P_s - s
 //   root box (8 floats) at 8 s
 // The reference has no batched build; this is the engine's many-scene path
 // (one launch per stage for all scenes).
@@ -22,7 +22,6 @@ namespace rq {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr uint32_t kCodeMask = (1u << 30) - 1u;
 
 __global__ void k_batch_init_bounds(int32_t* lohi, uint32_t n_scenes) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -118,7 +117,7 @@ __global__ void __launch_bounds__(kThreads) k_batch_morton(const BatchDesc* __re
     float lo[3], ext[3];
     bounds_from(lohi + 6 * s, lo, ext);
     if (mode == RQ_MORTON_SCENE_CUBE) cube_extent(ext);
-    code = code_scene(tri_centroid(desc[s].verts, desc[s].idx, i), lo, ext);
+    code = code_scene(tri_centroid(desc[s].verts4, desc[s].idx4, i), lo, ext);
   } else {
     const float4 c = __ldg(desc[s].sph + i);
     if (mode == RQ_MORTON_REFERENCE) {
@@ -134,73 +133,6 @@ __global__ void __launch_bounds__(kThreads) k_batch_morton(const BatchDesc* __re
   }
   keys[g] = ((uint64_t)s << 30) | code;
   vals[g] = g;
-}
-
-// Sorted (key, global index) -> per-scene codes and local order.
-__global__ void __launch_bounds__(kThreads) k_batch_split(const uint64_t* __restrict__ keys,
-                                                          const uint32_t* __restrict__ vals,
-                                                          const uint32_t* __restrict__ poff, uint32_t n_scenes,
-                                                          uint32_t* __restrict__ codes, uint32_t* __restrict__ order,
-                                                          uint32_t* err) {
-  const uint32_t total = __ldg(poff + n_scenes);
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= total) return;
-  const uint64_t k = keys[g];
-  const uint32_t s = segment_of(poff, n_scenes, g);
-  const uint32_t v = vals[g], p0 = __ldg(poff + s);
-  // the sort keeps scenes contiguous: the source primitive is in the same scene
-  if ((uint32_t)(k >> 30) != s || v < p0 || v >= __ldg(poff + s + 1)) {
-    atomicOr(err, kErrCorrupt);
-    return;
-  }
-  codes[g] = (uint32_t)k & kCodeMask;
-  order[g] = v - p0;
-}
-
-__global__ void __launch_bounds__(kThreads) k_batch_karras(const uint32_t* __restrict__ codes,
-                                                           const uint32_t* __restrict__ poff,
-                                                           const uint32_t* __restrict__ ioff, uint32_t n_scenes,
-                                                           float4* __restrict__ nodes, uint32_t* __restrict__ parent) {
-  const uint32_t total = __ldg(ioff + n_scenes);
-  const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = gi < total;  // every lane stays for the warp searches
-  uint32_t s = 0, p0 = 0, i0 = 0, ki = 0;
-  int N = 2, i = 0, dprev = -1, dnext = -1;
-  if (active) {
-    s = segment_of(ioff, n_scenes, gi);
-    p0 = __ldg(poff + s);
-    i0 = __ldg(ioff + s);
-    N = (int)(__ldg(poff + s + 1) - p0);
-    i = (int)(gi - i0);
-    ki = __ldg(codes + p0 + i);
-    dnext = delta32(codes + p0, N, i, i + 1, ki);
-    dprev = delta32(codes + p0, N, i, i - 1, ki);
-  }
-  const int4 ch = karras_node_warp(codes + p0, N, i, ki, dprev, dnext, active);
-  if (!active) return;
-  float4* nd = nodes + 4 * (size_t)i0;
-  uint32_t* par = parent + (2 * (size_t)p0 - s);
-  reinterpret_cast<int4*>(nd)[4 * (size_t)i + 3] = make_int4(ch.x, ch.y, ch.x < 0 ? 1 : 0, ch.y < 0 ? 1 : 0);
-  par[ch.x >= 0 ? ch.x : (N - 1 + ~ch.x)] = ((uint32_t)i << 1) | 0u;
-  par[ch.y >= 0 ? ch.y : (N - 1 + ~ch.y)] = ((uint32_t)i << 1) | 1u;
-}
-
-__global__ void __launch_bounds__(kThreads) k_batch_refit(const BatchDesc* __restrict__ desc, int kind,
-                                                          const uint32_t* __restrict__ poff,
-                                                          const uint32_t* __restrict__ ioff, uint32_t n_scenes,
-                                                          const uint32_t* __restrict__ order, float4* nodes,
-                                                          const uint32_t* __restrict__ parent, uint32_t* flags,
-                                                          float4* __restrict__ prims, float* __restrict__ roots,
-                                                          uint32_t* err) {
-  const uint32_t total = __ldg(poff + n_scenes);
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= total) return;
-  const uint32_t s = segment_of(poff, n_scenes, g);
-  const uint32_t p0 = __ldg(poff + s), i0 = __ldg(ioff + s);
-  const uint32_t n = __ldg(poff + s + 1) - p0, j = g - p0;
-  const size_t payload = kind == kTriangles ? 3 : 1;
-  Box6 b = emit_prim(kind, desc[s].verts, desc[s].idx, desc[s].sph, __ldg(order + g), prims + payload * p0, j);
-  refit_climb(n, j, b, nodes + 4 * (size_t)i0, parent + (2 * (size_t)p0 - s), flags + i0, roots + 8 * (size_t)s, err);
 }
 
 #define RQ_BB(call, what)                                            \
@@ -225,14 +157,14 @@ cudaError_t BatchStore::allocate() {
   const int passes = batch_sort_passes(n);
   cudaError_t e;
   if ((e = desc.ensure(sizeof(BatchDesc) * n)) != cudaSuccess) return e;
-  if ((e = offs.ensure(4 * (3 * (size_t)n + 3))) != cudaSuccess) return e;
+  if ((e = offs.ensure(4 * (2 * (size_t)n + 2))) != cudaSuccess) return e;
   if ((e = lohi.ensure(24 * (size_t)n)) != cudaSuccess) return e;
   if ((e = nodes.ensure(64 * std::max<size_t>(1, (size_t)total - n))) != cudaSuccess) return e;
   if ((e = prims.ensure(payload * total)) != cudaSuccess) return e;
   if ((e = order.ensure(4 * (size_t)total)) != cudaSuccess) return e;
   if ((e = codes.ensure(4 * (size_t)total)) != cudaSuccess) return e;
   if ((e = roots.ensure(32 * (size_t)n)) != cudaSuccess) return e;
-  if ((e = parent.ensure(4 * (2 * (size_t)total))) != cudaSuccess) return e;
+  if ((e = subtrees.ensure(tree_pool_bytes(total))) != cudaSuccess) return e;
   if ((e = keys.ensure(8 * (size_t)total)) != cudaSuccess) return e;
   if ((e = keys_alt.ensure(8 * (size_t)total)) != cudaSuccess) return e;
   if ((e = vals.ensure(4 * (size_t)total)) != cudaSuccess) return e;
@@ -243,11 +175,10 @@ cudaError_t BatchStore::allocate() {
 }
 
 cudaError_t BatchStore::upload_tables(cudaStream_t st) {
-  // offs = [P (n + 1)] [V (n + 1)] [I (n + 1)]
+  // offs = [P (n + 1)] [V (n + 1)]
   std::vector<uint32_t> t;
   t.insert(t.end(), poff.begin(), poff.end());
   t.insert(t.end(), voff.begin(), voff.end());
-  for (uint32_t s = 0; s <= n_scenes; ++s) t.push_back(poff[s] - s);
   cudaError_t e = cudaMemcpyAsync(offs.p, t.data(), t.size() * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(desc.p, host_desc.data(), sizeof(BatchDesc) * n_scenes, cudaMemcpyHostToDevice, st);
@@ -260,7 +191,6 @@ BuildResult build_batch(BatchStore& b, int morton_mode, uint32_t* err, cudaStrea
   const int passes = batch_sort_passes(n);
   const uint32_t* P = b.offs.as<const uint32_t>();
   const uint32_t* V = P + (n + 1);
-  const uint32_t* I = V + (n + 1);
   const BatchDesc* desc = b.desc.as<const BatchDesc>();
   uint32_t* z = b.zero.as<uint32_t>();
   RQ_BB(cudaMemsetAsync(z, 0, 4 * b.zero_words, st), "memset");
@@ -276,15 +206,23 @@ BuildResult build_batch(BatchStore& b, int morton_mode, uint32_t* err, cudaStrea
   launch_histogram64(b.keys.as<uint64_t>(), total, passes, z, st);
   launch_onesweep64(b.keys.as<uint64_t>(), b.vals.as<uint32_t>(), total, passes, b.keys_alt.as<uint64_t>(),
                     b.vals_alt.as<uint32_t>(), z, z + 2048 + 16, z + 2048, err, st);
-  count_launch(3);
-  k_batch_split<<<grid(total), kThreads, 0, st>>>(b.keys.as<const uint64_t>(), b.vals.as<const uint32_t>(), P, n,
-                                                  b.codes.as<uint32_t>(), b.order.as<uint32_t>(), err);
-  if (total > n)
-    k_batch_karras<<<grid(total - n), kThreads, 0, st>>>(b.codes.as<const uint32_t>(), P, I, n, b.nodes.as<float4>(),
-                                                          b.parent.as<uint32_t>());
-  k_batch_refit<<<grid(total), kThreads, 0, st>>>(desc, b.kind, P, I, n, b.order.as<const uint32_t>(),
-                                                  b.nodes.as<float4>(), b.parent.as<const uint32_t>(), flags,
-                                                  b.prims.as<float4>(), b.roots.as<float>(), err);
+  TreeArgs t;
+  t.kind = b.kind;
+  t.desc = desc;
+  t.poff = P;
+  t.n_scenes = n;
+  t.n = total;
+  t.keys = b.keys.as<const uint64_t>();
+  t.vals = b.vals.as<const uint32_t>();
+  t.codes_out = b.codes.as<uint32_t>();
+  t.order_out = b.order.as<uint32_t>();
+  t.nodes = b.nodes.as<float4>();
+  t.prims = b.prims.as<float4>();
+  t.roots = b.roots.as<float>();
+  t.flags = flags;
+  t.pool = b.subtrees.as<float4>();
+  t.err = err;
+  RQ_BB(launch_tree(t, false, st), "batched tree launch");
   RQ_BB(cudaGetLastError(), "batched build launch");
   return {};
 }

@@ -93,8 +93,7 @@ void launch_validate(const float* verts, uint32_t nv, const uint32_t* idx, uint3
   k_validate<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(verts, nv, idx, nt, sph, n, err);
 }
 
-// Zero region layout: [hist 1024][counters 16][status words][refit flags]
-// [hist 1024][counters 16][look-back status][refit flags n - 1][top count 4]
+// Zero region layout: [hist 1024][counters 16][look-back status][tree arrivals n - 1][top count 4]
 static size_t zero_words(uint32_t n, int passes) {
   return 1024 + 16 + sort_status_words(n, passes) + (n > 1 ? n - 1 : 0) + 4;
 }
@@ -173,8 +172,13 @@ static BuildResult build_lbvh(const SceneView& s, const rq_settings_t& cfg, Acce
   RQ_B(sc.keys_alt.ensure((size_t)n * 4), "sort scratch");
   RQ_B(sc.vals_alt.ensure((size_t)n * 4), "sort scratch");
   RQ_B(sc.zero.ensure(zero_words(n, kSortPasses) * 4), "build scratch");
-  RQ_B(sc.parent.ensure((size_t)(2 * (uint64_t)n) * 4), "parent links");
-  RQ_B(sc.mark.ensure(refit_mark_words(n) * 4), "refit marks");
+  RQ_B(sc.subtrees.ensure(tree_pool_bytes(n)), "subtree records");
+  const bool treelets = cfg.lbvh_quality == RQ_LBVH_TREELETS && n > 2;
+  if (treelets) {
+    RQ_B(sc.parent.ensure((size_t)n * 4), "parent links");
+    RQ_B(sc.mark.ensure(refit_mark_words(n) * 4), "treelet lists");
+    RQ_B(sc.heights.ensure(n), "node heights");
+  }
   uint32_t* z = sc.zero.as<uint32_t>();
   RQ_B(cudaMemsetAsync(z, 0, zero_words(n, kSortPasses) * 4, st), "memset");
   uint32_t* codes = a.codes.as<uint32_t>();
@@ -183,19 +187,30 @@ static BuildResult build_lbvh(const SceneView& s, const rq_settings_t& cfg, Acce
   if (!r.ok()) return r;
   r = sort_pairs(codes, order, n, kSortPasses, false, sc, err, st, 1, 0, true);
   if (!r.ok()) return r;
-  uint32_t* flags = z + 1040 + sort_status_words(n, kSortPasses);
-  uint32_t* mk = sc.mark.as<uint32_t>();
-  const RefitTop top{mk, mk + n, mk + refit_treelet_offset(n), flags + (n > 1 ? n - 1 : 0)};
-  launch_karras(codes, n, a.nodes.as<float4>(), sc.parent.as<uint32_t>(), top, st);
-  const bool treelets = cfg.lbvh_quality == RQ_LBVH_TREELETS && n > 2;
-  if (treelets) RQ_B(sc.heights.ensure(n), "treelet scratch");
-  RQ_B(launch_refit(s.kind, s.verts4, s.idx4, s.sph, order, n, a.nodes.as<float4>(), sc.parent.as<uint32_t>(),
-                    top, flags, a.prims.as<float4>(), a.root.as<float>(), err, st,
-                    treelets ? sc.heights.as<uint8_t>() : nullptr),
-       "LBVH refit launch");
+  uint32_t* flags = z + 1040 + sort_status_words(n, kSortPasses);  // tree arrivals
+  TreeArgs t;
+  t.kind = s.kind;
+  t.verts = s.verts4;
+  t.idx = s.idx4;
+  t.sph = s.sph;
+  t.n = n;
+  t.codes = codes;
+  t.order = order;
+  t.nodes = a.nodes.as<float4>();
+  t.prims = a.prims.as<float4>();
+  t.roots = a.root.as<float>();
+  t.flags = flags;
+  t.pool = sc.subtrees.as<float4>();
+  t.err = err;
+  if (treelets) {
+    uint32_t* mk = sc.mark.as<uint32_t>();
+    t.heights = sc.heights.as<uint8_t>();
+    t.parent = sc.parent.as<uint32_t>();
+    t.top = {mk, mk + n, mk + refit_treelet_offset(n), flags + (n - 1)};
+  }
+  RQ_B(launch_tree(t, treelets, st), "LBVH tree launch");
   if (treelets)
-    RQ_B(launch_treelet_opt(n, a.nodes.as<float4>(), sc.parent.as<uint32_t>(), top, sc.heights.as<uint8_t>(), err, st),
-         "LBVH treelet launch");
+    RQ_B(launch_treelet_opt(n, t.nodes, t.parent, t.top, t.heights, err, st), "LBVH treelet launch");
   RQ_B(cudaGetLastError(), "LBVH launch");
   a.n_nodes = n > 1 ? n - 1 : 0;
   a.n_slots = n;

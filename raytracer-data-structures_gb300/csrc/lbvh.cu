@@ -1,14 +1,16 @@
-// LBVH topology and bottom-up refit.
+// LBVH topology, payload and boxes.
 //
 // The reference cites Karras' construction (accelerators.h:371,568) but its
-// findSplit (accelerators.h:397-449) is discarded and no refit exists; this
-// file implements the cited method: Karras 2012, "Maximizing Parallelism in
-// the Construction of BVHs, Octrees, and k-d Trees", one thread per internal
-// node, then a bottom-up refit in which the second of a node's two children
-// to finish computes the node's box.  The refit runs by treelets (maximal
-// subtrees of at most kTreeletSpan leaves, one block each, in shared memory)
-// and then the top nodes above them (one block), so no level of the climb
-// waits on device-scope memory unless the top nodes exceed that block.
+// findSplit (accelerators.h:397-449) is discarded and no refit exists.  The
+// tree here is Karras' radix tree over the sorted codes (2012, "Maximizing
+// Parallelism in the Construction of BVHs, Octrees, and k-d Trees"; ties
+// broken by the index), in his numbering: a left child's index is its last
+// leaf, a right child's its first, the root's 0.  It is built from the leaves
+// up (Apetrei 2014, "Fast and Simple Agglomerative LBVH Construction"): a
+// subtree over the leaves l .. r joins the neighbour with which it shares the
+// longer prefix, so its parent's split is r | r + 1 or l - 1 | l, and the
+// second of two siblings to arrive at their split makes the node.  Topology
+// and boxes come out of one pass, with no searches and no parent links.
 //
 // BVH2 node (64 B, 4 x float4):
 //   [0] left  child box (lo.x, hi.x, lo.y, hi.y)
@@ -16,74 +18,13 @@
 //   [2] (left lo.z, left hi.z, right lo.z, right hi.z)
 //   [3] int (left, right, left count, right count); child >= 0 internal,
 //       child < 0 leaf holding slots [~child, ~child + count)
-#include <atomic>
-
 #include "lbvh_device.cuh"
+#include "rq_build.hpp"
 
 namespace rq {
 namespace {
 
 constexpr int kThreads = 256;
-static_assert(kRefitTopCap == kRefitTopCapHost, "top list capacity");
-
-
-// Internal node i of the radix tree (one thread per node; Karras 2012).
-// Also lays out the refit: a node of more than kTreeletSpan leaves is a top
-// node (mark[i] = kTopMark | slot, top[slot] = i for slots below
-// kRefitTopCap, count[0] = their number, possibly above the cap) and lists
-// its children of at most kTreeletSpan leaves as treelets ({first slot,
-// leaf count | kTreeletRight for a right child}, count[1] = their number);
-// a root of at most kTreeletSpan leaves is the one treelet.
-__global__ void __launch_bounds__(kThreads) k_karras(const uint32_t* __restrict__ codes, uint32_t n_,
-                                                     float4* __restrict__ nodes,
-                                                     uint32_t* __restrict__ parent, uint32_t* __restrict__ mark,
-                                                     uint32_t* __restrict__ top, uint32_t* __restrict__ treelets,
-                                                     uint32_t* count) {
-  const int n = (int)n_;
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  // Neighbour deltas from warp shuffles where the neighbour is in the warp.
-  const uint32_t ki = i < n ? __ldg(codes + i) : 0u;
-  uint32_t kprev = __shfl_up_sync(0xffffffffu, ki, 1);
-  uint32_t knext = __shfl_down_sync(0xffffffffu, ki, 1);
-  const bool active = i + 1 < n;  // every lane stays for the warp searches
-  const int lane = threadIdx.x & 31;
-  int dprev = -1, dnext = -1;
-  if (active) {
-    if (lane == 0 && i > 0) kprev = __ldg(codes + i - 1);
-    if (lane == 31) knext = __ldg(codes + i + 1);
-    dnext = ki != knext ? __clz(ki ^ knext) : 32 + __clz((uint32_t)i ^ (uint32_t)(i + 1));
-    dprev = i == 0 ? -1 : (ki != kprev ? __clz(ki ^ kprev) : 32 + __clz((uint32_t)i ^ (uint32_t)(i - 1)));
-  }
-  const int4 nd = karras_node_warp(codes, n, i, ki, dprev, dnext, active);
-  if (!active) return;
-  const int32_t lc = nd.x, rc = nd.y;
-  const int lo = nd.z, hi = nd.w;
-  const int gamma = lc >= 0 ? lc : ~lc;  // the left child ends at the split
-  reinterpret_cast<int4*>(nodes)[4 * (size_t)i + 3] = make_int4(lc, rc, lc < 0 ? 1 : 0, rc < 0 ? 1 : 0);
-  parent[lc >= 0 ? lc : (n - 1 + ~lc)] = ((uint32_t)i << 1) | 0u;
-  parent[rc >= 0 ? rc : (n - 1 + ~rc)] = ((uint32_t)i << 1) | 1u;
-  uint32_t m = 0u;
-  const uint32_t span = (uint32_t)(hi - lo) + 1u;
-  uint2* tl = reinterpret_cast<uint2*>(treelets);
-  if (span > kTreeletSpan) {
-    const uint32_t slot = atomicAdd(count, 1u);
-    if (slot < kRefitTopCap) top[slot] = (uint32_t)i;
-    m = kTopMark | (slot & kSlotMask);
-    const uint32_t ls = (uint32_t)(gamma - lo) + 1u, rs = (uint32_t)(hi - gamma);
-    if (ls <= kTreeletSpan) tl[atomicAdd(count + 1, 1u)] = make_uint2((uint32_t)lo, ls);
-    if (rs <= kTreeletSpan) tl[atomicAdd(count + 1, 1u)] = make_uint2((uint32_t)gamma + 1u, rs | kTreeletRight);
-  } else if (i == 0) {
-    tl[atomicAdd(count + 1, 1u)] = make_uint2(0u, span | kTreeletRight);  // the root's index is its first slot
-  }
-  mark[i] = m;
-}
-
-struct RefitShared {
-  float box[kTreeletSpan][2][6];  // child boxes of the treelet's internal nodes, by index - first slot
-  uint32_t up[kTreeletSpan];      // their parent words
-  uint32_t arrived[kTreeletSpan]; // children finished (2: the node is finished), + their heights << 8
-  uint32_t next;                  // the block's next treelet
-};
 
 // Triangle p's payload (3 float4: (v0, id), (v1 - v0, 0), (v2 - v0, 0)) in
 // q and its box, from the packed copies.
@@ -120,224 +61,245 @@ __device__ __forceinline__ void store_payload_warp(float4* __restrict__ out, int
   }
 }
 
-// Above a treelet root: its box goes into the parent (a top node).  With
-// the top block active that is all; otherwise climb with device-scope
-// arrival counts to the root.
-__device__ __forceinline__ void climb_top(uint32_t pw, Box6 b, bool top_mode, float4* nodes,
-                                          const uint32_t* __restrict__ parent, uint32_t* flags,
-                                          float* __restrict__ root_out, uint32_t* err) {
-  for (int level = 0;; ++level) {
-    if (level >= 128) { atomicOr(err, kErrCorrupt); return; }  // Karras trees are at most 64 deep
-    const uint32_t node = pw >> 1, side = pw & 1u;
-    const uint32_t up = node ? __ldg(parent + node) : 0u;
-    write_child(nodes, node, side, b);
-    if (top_mode) return;
-    if (atomic_add_acq_rel(flags + node, 1u) == 0u) return;
-    const float4 a = __ldcg(nodes + 4 * (size_t)node);
-    const float4 c = __ldcg(nodes + 4 * (size_t)node + 1);
-    const float4 z = __ldcg(nodes + 4 * (size_t)node + 2);
-    b.lo[0] = fminf(a.x, c.x); b.hi[0] = fmaxf(a.y, c.y);
-    b.lo[1] = fminf(a.z, c.z); b.hi[1] = fmaxf(a.w, c.w);
-    b.lo[2] = fminf(z.x, z.z); b.hi[2] = fmaxf(z.y, z.w);
-    if (node == 0) {
-      for (int k = 0; k < 3; ++k) { root_out[k] = b.lo[k]; root_out[3 + k] = b.hi[k]; }
-      return;
-    }
-    pw = up;
-  }
-}
+// The tree over a window of kTreeWindow leaves is made in shared memory, one
+// block a window and one thread a leaf; the subtrees left over (those whose
+// parent reaches into another window: at most one on each step of the paths
+// from the root to the two leaves at a boundary, so at most 2 x 64 a window)
+// climb on with device-scope arrivals, one thread each.
+//
+// Bound by latency: the leaf's three dependent gathers, about ten shared
+// steps, then about log2(windows) device-scope exchanges of a microsecond;
+// whole rebuilds of 36k spheres, 125k, 998k and 2.7M triangles took 124, 144,
+// 265 and 518 us with one search a node, parent links and a second kernel for
+// the boxes, and take 79, 91, 191 and 348 us.  Windows of 1024 leaves: 87,
+// 92, 201, 367 us; 512: 83, 93, 198, 358; 128: 79, 90, 190, 342, with twice
+// the records.
+constexpr uint32_t kTreeBlocks = 6;  // an SM; 5 and 8 blocks: within 3%
+static_assert(kTreeWindow >= kTreeMaxLeft, "one thread a subtree left over");
+static_assert(kTreeWindow <= kTreeletSpan, "a top node is made by the slow climb");
+static_assert(kTreeWindow < (1u << 16), "a far end and a height share a word");
 
-// Persistent blocks over the treelets.  In a treelet of c leaves from slot
-// lo, every internal node has its index in [lo, lo + c) and both children in
-// the treelet: one block gathers the leaves' primitives, climbs with
-// shared-memory boxes and arrival bits (block-scope ordering only) and at
-// the end stores the finished nodes' boxes, coalesced.  heights (optional):
-// each internal node's height (longest path to a leaf, leaves 0), from the
-// children's heights added into the arrival words.
-template <bool HEIGHTS>
-__global__ void __launch_bounds__(kTreeletThreads, kTreeletBlocksPerSM) k_refit(int kind, const float4* __restrict__ verts,
-                                                          const uint4* __restrict__ idx,
-                                                          const float4* __restrict__ sph,
-                                                          const uint32_t* __restrict__ order, uint32_t n,
-                                                          float4* nodes, const uint32_t* __restrict__ parent,
-                                                          const uint32_t* __restrict__ treelets,
-                                                          uint32_t* count,  // [0] top nodes, [1] treelets, [2] treelet queue
-                                                          uint32_t* flags, float4* __restrict__ prims,
-                                                          float* __restrict__ root_out, uint32_t* err,
-                                                          uint8_t* __restrict__ heights) {
-  extern __shared__ __align__(16) unsigned char refit_smem[];
-  RefitShared& sh = *reinterpret_cast<RefitShared*>(refit_smem);
-  if (n == 1) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      const Box6 b = emit_prim(kind, verts, idx, sph, __ldg(order), prims, 0);
-      for (int k = 0; k < 3; ++k) { root_out[k] = b.lo[k]; root_out[3 + k] = b.hi[k]; }
-    }
-    return;
-  }
-  const bool top_mode = __ldcg(count) <= kRefitTopCap;
-  const uint32_t ntl = __ldcg(count + 1);
-  const uint2* tl = reinterpret_cast<const uint2*>(treelets);
-  for (;;) {
-    if (threadIdx.x == 0) sh.next = atomicAdd(count + 2, 1u);  // treelets are taken in turn (uneven sizes)
-    __syncthreads();
-    const uint32_t t = sh.next;
-    if (t >= ntl) break;  // uniform per block
-    const uint2 rec = __ldcg(tl + t);
-    const uint32_t lo = rec.x, cnt = rec.y & ~kTreeletRight;
-    if (cnt == 0 || cnt > kTreeletSpan || lo + cnt > n) {  // uniform per block
-      if (threadIdx.x == 0) atomicOr(err, kErrCorrupt);
-      __syncthreads();  // sh.next is rewritten at the top of the loop
-      continue;
-    }
-    const uint32_t root = cnt == 1 ? ~0u : (rec.y & kTreeletRight) ? lo : lo + cnt - 1;
-    for (uint32_t w = threadIdx.x; w < cnt; w += blockDim.x) {
-      sh.up[w] = __ldg(parent + lo + w);
-      sh.arrived[w] = 0u;
-    }
-    __syncthreads();
-    // Every lane of a warp runs each round (the payload store is warp-wide).
-    const uint32_t lane = threadIdx.x & 31u, wbase = threadIdx.x & ~31u;
-    for (uint32_t w0 = 0; w0 < cnt; w0 += blockDim.x) {
-      const uint32_t w = w0 + threadIdx.x;
-      const bool live = w < cnt;
-      const uint32_t j = lo + w;
-      Box6 b;
-      if (kind == kTriangles) {
-        float4 q[3] = {};
-        if (live) b = tri_payload(verts, idx, __ldg(order + j), q);
-        const int nvalid = (int)cnt - (int)(w0 + wbase);  // live lanes of this warp: a prefix
-        if (nvalid > 0) store_payload_warp(prims + 3 * (size_t)(lo + w0 + wbase), nvalid < 32 ? nvalid : 32, lane, q);
-      } else if (live) {
-        b = emit_sphere(sph, __ldg(order + j), prims, j);
-      }
-      if (!live) continue;
-      uint32_t pw = __ldg(parent + (n - 1) + j);
-      bool at_root = cnt == 1;  // b is the treelet root's box
-      uint32_t h = 0;           // height of the subtree whose box is b
-      for (uint32_t step = 0; !at_root; ++step) {
-        const uint32_t node = pw >> 1, side = pw & 1u;
-        const uint32_t x = node - lo;
-        if (x >= cnt || step > kTreeletSpan) { atomicOr(err, kErrCorrupt); break; }
-        float* mine = sh.box[x][side];
-        for (int k = 0; k < 3; ++k) { mine[k] = b.lo[k]; mine[3 + k] = b.hi[k]; }
-        __threadfence_block();
-        const uint32_t old = atomicAdd(&sh.arrived[x], HEIGHTS ? 1u + (h << 8) : 1u);
-        if ((old & 0xFFu) == 1u) {  // second: finish the node
-          __threadfence_block();
-          const float* L = sh.box[x][0];
-          const float* R = sh.box[x][1];
-          for (int k = 0; k < 3; ++k) { b.lo[k] = fminf(L[k], R[k]); b.hi[k] = fmaxf(L[3 + k], R[3 + k]); }
-          pw = sh.up[x];
-          if constexpr (HEIGHTS) {
-            h = 1u + max(h, old >> 8);
-            sh.up[x] = h;  // nothing reads x's parent word after this climb: it keeps x's height
-          }
-          at_root = node == root;
-        } else {
-          break;
-        }
-      }
-      if (at_root) {
-        if (cnt == n) {  // the treelet is the whole tree
-          for (int k = 0; k < 3; ++k) { root_out[k] = b.lo[k]; root_out[3 + k] = b.hi[k]; }
-        } else {
-          climb_top(pw, b, top_mode, nodes, parent, flags, root_out, err);
-        }
-      }
-    }
-    __syncthreads();
-    // The finished nodes' three box float4s (the fourth, the links, stays),
-    // consecutive threads on consecutive float4s.
-    for (uint32_t f = threadIdx.x; f < 3 * cnt; f += blockDim.x) {
-      const uint32_t w = f / 3, c = f - 3 * w;
-      if ((sh.arrived[w] & 0xFFu) != 2u) continue;  // not an internal node of this treelet
-      if (HEIGHTS && c == 0) heights[lo + w] = (uint8_t)min(sh.up[w], 255u);
-      const float* L = sh.box[w][0];
-      const float* R = sh.box[w][1];
-      nodes[4 * (size_t)(lo + w) + c] = c == 0 ? make_float4(L[0], L[3], L[1], L[4])
-                                      : c == 1 ? make_float4(R[0], R[3], R[1], R[4])
-                                               : make_float4(L[2], L[5], R[2], R[5]);
-    }
-    __syncthreads();  // the next treelet reuses the shared arrays
-  }
-}
-
-// The top nodes, one block: every child box below them is in place (the
-// leaf climb wrote it), so the block climbs the top subtree with shared
-// memory boxes and arrival counts, writing each finished box into its
-// parent node (and the root box).  Nothing to do when the top nodes exceed
-// the cap: the leaf climb went to the root.
-struct TopShared {
-  float box[kRefitTopCap][2][6];
-  uint32_t node[kRefitTopCap];
-  uint32_t up[kRefitTopCap];       // parent slot << 1 | side; ~0u for the root
-  uint32_t arrived[kRefitTopCap];  // children finished
-  uint8_t start[kRefitTopCap];     // both children below the top nodes
+struct TreeShared {
+  float box[6][kTreeWindow];        // a finished subtree's box, at its index (its last leaf as a left child, else its first)
+  uint32_t arrived[kTreeWindow];    // split w | w + 1: 0, or the one child here: (far end + 1) | height << 16 | left << 31
+  int8_t delta[kTreeWindow + 1];    // prefix shared by leaves w - 1 and w; -1 at the ends of a scene
+  uint32_t left_lr[kTreeMaxLeft];   // the subtrees left over: first leaf | last leaf << 16
+  uint8_t left_h[kTreeMaxLeft];     // their heights
+  uint32_t n_left;
 };
 
-__device__ __forceinline__ void load_child_box(const float4* nodes, uint32_t node, uint32_t side, float* out) {
-  const float4 xy = __ldcg(nodes + 4 * (size_t)node + side);
-  const float2 z = __ldcg(reinterpret_cast<const float2*>(nodes + 4 * (size_t)node + 2) + side);
-  out[0] = xy.x; out[3] = xy.y; out[1] = xy.z; out[4] = xy.w; out[2] = z.x; out[5] = z.y;
+// The node over leaves l .. r split after g (scene-local slots): links and
+// both child boxes, two 32-byte stores.
+__device__ __forceinline__ void store_node(float4* node, uint32_t l, uint32_t g, uint32_t r, const Box6& L,
+                                           const Box6& R) {
+  const int lc = g == l ? ~(int)g : (int)g, rc = g + 1 == r ? ~(int)(g + 1) : (int)(g + 1);
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(node), "f"(L.lo[0]), "f"(L.hi[0]),
+               "f"(L.lo[1]), "f"(L.hi[1]), "f"(R.lo[0]), "f"(R.hi[0]), "f"(R.lo[1]), "f"(R.hi[1])
+               : "memory");
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(node + 2), "r"(__float_as_int(L.lo[2])),
+               "r"(__float_as_int(L.hi[2])), "r"(__float_as_int(R.lo[2])), "r"(__float_as_int(R.hi[2])), "r"(lc), "r"(rc),
+               "r"(lc < 0 ? 1 : 0), "r"(rc < 0 ? 1 : 0)
+               : "memory");
 }
 
-__global__ void __launch_bounds__(kRefitTopThreads) k_refit_top(float4* nodes, const uint32_t* __restrict__ parent,
-                                                              const uint32_t* __restrict__ mark,
-                                                              const uint32_t* __restrict__ top,
-                                                              const uint32_t* __restrict__ top_count,
-                                                              float* __restrict__ root_out, uint32_t* err) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  TopShared& sh = *reinterpret_cast<TopShared*>(smem_raw);
-  const uint32_t cnt = __ldg(top_count);
-  if (cnt == 0 || cnt > kRefitTopCap) return;
-  for (uint32_t k = threadIdx.x; k < cnt; k += blockDim.x) {
-    const uint32_t i = __ldg(top + k);
-    sh.node[k] = i;
-    const int4 l = __ldcg(reinterpret_cast<const int4*>(nodes) + 4 * (size_t)i + 3);
-    uint32_t ready = 0;
-    const int32_t ch[2] = {l.x, l.y};
-    for (uint32_t side = 0; side < 2; ++side) {
-      if (ch[side] >= 0 && (__ldg(mark + ch[side]) & kTopMark)) continue;  // a top child: finished here
-      load_child_box(nodes, i, side, sh.box[k][side]);
-      ++ready;
-    }
-    sh.arrived[k] = ready;
-    sh.start[k] = ready == 2;
-    uint32_t up = ~0u;
-    if (i != 0) {
-      const uint32_t pw = __ldg(parent + i);
-      const uint32_t pm = __ldg(mark + (pw >> 1));
-      if (!(pm & kTopMark) || (pm & kSlotMask) >= cnt) {
-        atomicOr(err, kErrCorrupt);  // a top node's parent covers more leaves, so it is a top node
-        sh.start[k] = 0;
-      } else {
-        up = ((pm & kSlotMask) << 1) | (pw & 1u);
+__device__ __forceinline__ Box6 join(const Box6& L, const Box6& R) {
+  Box6 b;
+  for (int k = 0; k < 3; ++k) { b.lo[k] = fminf(L.lo[k], R.lo[k]); b.hi[k] = fmaxf(L.hi[k], R.hi[k]); }
+  return b;
+}
+
+__device__ __forceinline__ void store_root(float* root, const Box6& b) {
+  for (int k = 0; k < 3; ++k) { root[k] = b.lo[k]; root[3 + k] = b.hi[k]; }
+}
+
+// What the treelet pass needs of node i over leaves l .. r split after g: a
+// node of more than kTreeletSpan leaves is a top node (mark[i] = kTopMark |
+// slot, top[slot] = i for slots below kRefitTopCap, count[0] = their number,
+// possibly above the cap; its children get their parent words) and lists its
+// children of at most kTreeletSpan leaves as treelets ({first slot, leaf
+// count | kTreeletRight for a right child}, count[1] = their number); a root
+// of at most kTreeletSpan leaves is the one treelet.
+__device__ __forceinline__ void list_node(const TreeArgs& a, uint32_t i, uint32_t l, uint32_t g, uint32_t r, bool root) {
+  uint2* tl = reinterpret_cast<uint2*>(a.top.treelets);
+  if (r - l + 1 <= kTreeletSpan) {
+    if (root) tl[atomicAdd(a.top.count + 1, 1u)] = make_uint2(0u, (r - l + 1) | kTreeletRight);
+    return;
+  }
+  const uint32_t slot = atomicAdd(a.top.count, 1u);
+  if (slot < kRefitTopCap) a.top.top[slot] = i;
+  a.top.mark[i] = kTopMark | (slot & kSlotMask);
+  const uint32_t ls = g - l + 1, rs = r - g;
+  if (ls > 1) a.parent[g] = i << 1;
+  if (rs > 1) a.parent[g + 1] = i << 1 | 1u;
+  if (ls <= kTreeletSpan) {
+    if (ls > 1) a.top.mark[g] = 0u;
+    tl[atomicAdd(a.top.count + 1, 1u)] = make_uint2(l, ls);
+  }
+  if (rs <= kTreeletSpan) {
+    if (rs > 1) a.top.mark[g + 1] = 0u;
+    tl[atomicAdd(a.top.count + 1, 1u)] = make_uint2(g + 1, rs | kTreeletRight);
+  }
+}
+
+// MANY: the slots of several scenes back to back (poff), each with its own
+// codes, nodes, root and indices, sorted by (scene << 30) | code; otherwise
+// one scene.  LIST: also what the treelet pass reads (node heights, top nodes,
+// treelets).
+template <bool MANY, bool LIST>
+__global__ void __launch_bounds__(kTreeWindow, kTreeBlocks) k_tree(TreeArgs a) {
+  __shared__ TreeShared sh;
+  constexpr uint32_t kCodeMask = (1u << 30) - 1u;
+  const uint32_t base = blockIdx.x * kTreeWindow;
+  const uint32_t cnt = min(kTreeWindow, a.n - base);
+  const uint32_t w = threadIdx.x, lane = w & 31u, g0 = base + w;
+  const bool live = w < cnt;
+  // Scene of slot g (its number and first slot) and the prefix length of the
+  // leaves g - 1 and g.
+  auto scene_of = [&](uint32_t g, uint32_t& s, uint32_t& p0) {
+    s = p0 = 0u;
+    if constexpr (MANY) {
+      s = (uint32_t)(__ldg(a.keys + g) >> 30);
+      if (s >= a.n_scenes || g < __ldg(a.poff + s) || g >= __ldg(a.poff + s + 1)) {
+        atomicOr(a.err, kErrCorrupt);  // the sort keeps scenes contiguous
+        s = segment_of(a.poff, a.n_scenes, g);
       }
+      p0 = __ldg(a.poff + s);
     }
-    sh.up[k] = up;
+  };
+  auto code_of = [&](uint32_t g) { return MANY ? (uint32_t)__ldg(a.keys + g) & kCodeMask : __ldg(a.codes + g); };
+  auto delta_at = [&](uint32_t g, uint32_t p0) {
+    if (g == p0 || g >= a.n) return -1;
+    const uint32_t x = code_of(g - 1), y = code_of(g), i = g - 1 - p0;
+    return x != y ? __clz(x ^ y) : 32 + __clz(i ^ (i + 1u));
+  };
+  auto leave = [&](uint32_t l, uint32_t r, uint32_t h) {
+    const uint32_t at = atomicAdd(&sh.n_left, 1u);
+    if (at >= kTreeMaxLeft) { atomicOr(a.err, kErrCorrupt); return; }
+    sh.left_lr[at] = l | r << 16;
+    sh.left_h[at] = (uint8_t)h;
+  };
+  if (w == 0) {
+    sh.n_left = 0u;
+    uint32_t s = 0u, p0 = 0u;
+    if (base + cnt < a.n) scene_of(base + cnt, s, p0);
+    sh.delta[cnt] = (int8_t)delta_at(base + cnt, p0);
+  }
+  uint32_t s = 0u, p0 = 0u;
+  Box6 b = {};
+  float4 q[3] = {};
+  if (live) {
+    scene_of(g0, s, p0);
+    uint32_t p;
+    if constexpr (MANY) {
+      p = __ldg(a.vals + g0) - p0;
+      if (p >= __ldg(a.poff + s + 1) - p0) {
+        atomicOr(a.err, kErrCorrupt);
+        p = 0u;
+      }
+      a.codes_out[g0] = code_of(g0);
+      a.order_out[g0] = p;
+    } else {
+      p = __ldg(a.order + g0);
+    }
+    sh.arrived[w] = 0u;
+    sh.delta[w] = (int8_t)delta_at(g0, p0);
+    if (a.kind == kTriangles)
+      b = tri_payload(MANY ? a.desc[s].verts4 : a.verts, MANY ? a.desc[s].idx4 : a.idx, p, q);
+    else
+      b = emit_sphere(MANY ? a.desc[s].sph : a.sph, p, a.prims, g0);
+  }
+  if (a.kind == kTriangles) {  // warp-wide stores
+    const int nvalid = (int)cnt - (int)(w - lane);
+    if (nvalid > 0) store_payload_warp(a.prims + 3 * (size_t)(g0 - lane), nvalid < 32 ? nvalid : 32, lane, q);
   }
   __syncthreads();
-  for (uint32_t k = threadIdx.x; k < cnt; k += blockDim.x) {
-    if (!sh.start[k]) continue;
-    uint32_t cur = k;
-    for (uint32_t step = 0; step <= cnt; ++step) {
-      const float* l = sh.box[cur][0];
-      const float* r = sh.box[cur][1];
-      Box6 b;
-      for (int q = 0; q < 3; ++q) { b.lo[q] = fminf(l[q], r[q]); b.hi[q] = fmaxf(l[3 + q], r[3 + q]); }
-      const uint32_t up = sh.up[cur];
-      if (up == ~0u) {  // the root
-        for (int q = 0; q < 3; ++q) { root_out[q] = b.lo[q]; root_out[3 + q] = b.hi[q]; }
+  if (live) {
+    float4* const nodes = a.nodes + 4 * (size_t)(p0 - s);  // scene s's nodes start at its first slot - s
+    const uint32_t off = base - p0;                        // window slot -> scene slot (modulo 2^32)
+    uint32_t l = w, r = w, h = 0;
+    for (int step = 0;; ++step) {
+      if (step >= 128) { atomicOr(a.err, kErrCorrupt); break; }  // the tree is at most 64 deep
+      const int dl = sh.delta[l], dr = sh.delta[r + 1];
+      if ((dl & dr) < 0) {  // the whole scene
+        store_root(a.roots + 8 * (size_t)s, b);
         break;
       }
-      const uint32_t ps = up >> 1, side = up & 1u;
-      write_child(nodes, sh.node[ps], side, b);
-      float* dst = sh.box[ps][side];
-      for (int q = 0; q < 3; ++q) { dst[q] = b.lo[q]; dst[3 + q] = b.hi[q]; }
+      const bool left = dr > dl;  // a left child: the parent's split is r | r + 1
+      if (left ? r + 1 == cnt : l == 0) {
+        leave(l, r, h);
+        for (int c = 0; c < 3; ++c) { sh.box[c][left ? r : l] = b.lo[c]; sh.box[3 + c][left ? r : l] = b.hi[c]; }
+        break;
+      }
+      const uint32_t g = left ? r : l - 1, mine = left ? r : l, other = left ? r + 1 : l - 1;
+      for (int c = 0; c < 3; ++c) { sh.box[c][mine] = b.lo[c]; sh.box[3 + c][mine] = b.hi[c]; }
       __threadfence_block();
-      if (atomicAdd(&sh.arrived[ps], 1u) != 1u) break;  // the other child is not finished yet
+      const uint32_t old = atomicExch(&sh.arrived[g], ((left ? l : r) + 1u) | h << 16 | (left ? 1u << 31 : 0u));
+      if (old == 0u) break;  // the sibling's thread makes the node
       __threadfence_block();
-      cur = ps;
+      sh.arrived[g] = 0u;
+      Box6 o;
+      for (int c = 0; c < 3; ++c) { o.lo[c] = sh.box[c][other]; o.hi[c] = sh.box[3 + c][other]; }
+      const uint32_t far = (old & 0xFFFFu) - 1u;
+      if (left) r = far; else l = far;
+      if (l > r || r >= cnt) { atomicOr(a.err, kErrCorrupt); break; }
+      h = 1u + max(h, (old >> 16) & 0x7FFFu);
+      const int nl = sh.delta[l], nr = sh.delta[r + 1];
+      const uint32_t i = (nl & nr) < 0 ? 0u : (nr > nl ? r : l) + off;
+      store_node(nodes + 4 * (size_t)i, l + off, g + off, r + off, left ? b : o, left ? o : b);
+      b = left ? join(b, o) : join(o, b);
+      if constexpr (LIST) {
+        a.heights[i] = (uint8_t)min(h, 255u);
+        if ((nl & nr) < 0) list_node(a, 0u, l, g, r, true);
+      }
+    }
+  }
+  __syncthreads();
+  // A child whose sibling reaches into another window is left over too.
+  if (live) {
+    const uint32_t v = sh.arrived[w], far = (v & 0xFFFFu) - 1u;
+    if (v) leave(v >> 31 ? far : w + 1u, v >> 31 ? w : far, (v >> 16) & 0x7FFFu);
+  }
+  __syncthreads();
+  if (w >= min(sh.n_left, kTreeMaxLeft)) return;
+  // The subtrees left over, over scene slots; their boxes go to the sibling's
+  // thread in records of this window.
+  const uint32_t wl = sh.left_lr[w] & 0xFFFFu, wr = sh.left_lr[w] >> 16;
+  scene_of(base + wl, s, p0);
+  const uint32_t count = (MANY ? __ldg(a.poff + s + 1) : a.n) - p0;
+  float4* const nodes = a.nodes + 4 * (size_t)(p0 - s);
+  uint32_t l = base + wl - p0, r = base + wr - p0, h = sh.left_h[w];
+  int dl = sh.delta[wl], dr = sh.delta[wr + 1];
+  const uint32_t at = dr > dl ? wr : wl;
+  for (int c = 0; c < 3; ++c) { b.lo[c] = sh.box[c][at]; b.hi[c] = sh.box[3 + c][at]; }
+  const uint32_t rec = blockIdx.x * kTreeMaxLeft + w;
+  for (int step = 0;; ++step) {
+    if (step >= 128) { atomicOr(a.err, kErrCorrupt); break; }
+    const bool left = dr > dl;
+    const uint32_t g = left ? r : l - 1;
+    if (left ? r + 1 >= count : l == 0) { atomicOr(a.err, kErrCorrupt); break; }
+    a.pool[2 * (size_t)rec] = make_float4(b.lo[0], b.lo[1], b.lo[2], __uint_as_float(left ? l : r));
+    a.pool[2 * (size_t)rec + 1] =
+        make_float4(b.hi[0], b.hi[1], b.hi[2], __uint_as_float((uint32_t)((left ? dl : dr) + 1) | h << 8));
+    const uint32_t old = atomic_exch_acq_rel(a.flags + p0 + g, rec + 1u);
+    if (old == 0u) break;
+    const float4 x = __ldcg(a.pool + 2 * (size_t)(old - 1u)), y = __ldcg(a.pool + 2 * (size_t)(old - 1u) + 1);
+    const Box6 o = {{x.x, x.y, x.z}, {y.x, y.y, y.z}};
+    const uint32_t far = __float_as_uint(x.w), dh = __float_as_uint(y.w);
+    const int dfar = (int)(dh & 0xFFu) - 1;
+    if (left) { r = far; dr = dfar; } else { l = far; dl = dfar; }
+    if (l > r || r >= count) { atomicOr(a.err, kErrCorrupt); break; }
+    h = 1u + max(h, dh >> 8);
+    const bool root = (dl & dr) < 0;
+    const uint32_t i = root ? 0u : dr > dl ? r : l;
+    store_node(nodes + 4 * (size_t)i, l, g, r, left ? b : o, left ? o : b);
+    b = left ? join(b, o) : join(o, b);
+    if constexpr (LIST) {
+      a.heights[i] = (uint8_t)min(h, 255u);
+      list_node(a, i, l, g, r, root);
+    }
+    if (root) {
+      store_root(a.roots + 8 * (size_t)s, b);
+      break;
     }
   }
 }
@@ -356,42 +318,12 @@ __global__ void __launch_bounds__(kThreads) k_prims_by_id(int kind, const float*
 
 }  // namespace
 
-void launch_karras(const uint32_t* sorted_codes, uint32_t n, float4* nodes, uint32_t* parent,
-                   const RefitTop& t, cudaStream_t s) {
-  if (n < 2) return;
-  uint32_t g = (n - 1 + kThreads - 1) / kThreads;
+cudaError_t launch_tree(const TreeArgs& a, bool list, cudaStream_t s) {
+  if (a.n == 0) return cudaSuccess;
   count_launch();
-  k_karras<<<g, kThreads, 0, s>>>(sorted_codes, n, nodes, parent, t.mark, t.top, t.treelets, t.count);
-}
-
-cudaError_t launch_refit(int kind, const float4* verts, const uint4* idx, const float4* sph,
-                         const uint32_t* order, uint32_t n, float4* nodes, const uint32_t* parent,
-                         const RefitTop& t, uint32_t* flags, float4* prims, float* root_out, uint32_t* err,
-                         cudaStream_t s, uint8_t* heights) {
-  if (n == 0) return cudaSuccess;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  static std::atomic<uint64_t> attr_set{0};  // devices whose kernels allow their shared memory
-  const uint64_t bit = 1ull << (dev & 63);
-  if (!(attr_set.load() & bit)) {
-    e = cudaFuncSetAttribute(k_refit<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RefitShared));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_refit<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RefitShared));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_refit_top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TopShared));
-    if (e != cudaSuccess) return e;
-    attr_set.fetch_or(bit);
-  }
-  // Persistent: kTreeletBlocksPerSM treelet blocks per SM take treelets from a queue.
-  const uint32_t blocks = n == 1 ? 1u : kTreeletBlocksPerSM * (uint32_t)device_sm_count();
-  count_launch();
-  const auto k = heights ? k_refit<true> : k_refit<false>;
-  k<<<blocks, kTreeletThreads, sizeof(RefitShared), s>>>(kind, verts, idx, sph, order, n, nodes, parent, t.treelets,
-                                                         t.count, flags, prims, root_out, err, heights);
-  if (n < 2) return cudaGetLastError();
-  count_launch();
-  k_refit_top<<<1, kRefitTopThreads, sizeof(TopShared), s>>>(nodes, parent, t.mark, t.top, t.count, root_out, err);
+  const uint32_t blocks = tree_windows(a.n);
+  const auto k = a.poff ? k_tree<true, false> : list ? k_tree<false, true> : k_tree<false, false>;
+  k<<<blocks, kTreeWindow, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -519,7 +519,8 @@ rq_status_t rq_build_batched(rq_ctx_t ctx, const rq_scene_t* scenes, uint32_t n,
       return fail(ctx, RQ_ERROR_INVALID_ARGUMENT, "batch of 2^30 or more primitives");
     store->poff.push_back((uint32_t)p);
     store->voff.push_back((uint32_t)v);
-    store->host_desc.push_back({sc->verts.as<const float>(), sc->idx.as<const uint32_t>(), sc->sph.as<const float4>()});
+    store->host_desc.push_back({sc->verts.as<const float>(), sc->idx.as<const uint32_t>(), sc->sph.as<const float4>(),
+                                sc->verts4.as<const float4>(), sc->idx4.as<const uint4>()});
   }
   RQ_TRY_CUDA(ctx, store->allocate());
   RQ_TRY_CUDA(ctx, store->upload_tables(ctx->stream));

@@ -49,9 +49,10 @@ struct AccelBuffers {
 // Scratch reused across builds of one context (grow-only).
 struct BuildScratch {
   DevBuf keys_alt, vals_alt;  // radix sort ping-pong
-  DevBuf zero;                // [hist 1024][counters 16][look-back status][refit flags]: zeroed per build
-  DevBuf parent;              // Karras parent links
-  DevBuf mark;                // refit top nodes: per-node marks, then the top list
+  DevBuf zero;                // [hist 1024][counters 16][look-back status][arrivals]: zeroed per build
+  DevBuf subtrees;            // LBVH: records of the subtrees a window leaves over
+  DevBuf parent;              // LBVH treelets: parent words of the nodes below top nodes
+  DevBuf mark;                // LBVH treelets: per-node marks, the top list, the treelets
   DevBuf lohi;                // ordered-int scene box
   DevBuf keys, vals;          // generic sort input
   DevBuf m0, m1, m2, m3, m4, m5, m6, m7;  // median / KD working arrays
@@ -74,7 +75,7 @@ struct BuildScratch {
     top.release();
     exact.release();
     heights.release();
-    keys_alt.release(); vals_alt.release(); zero.release(); parent.release(); mark.release(); lohi.release();
+    keys_alt.release(); vals_alt.release(); zero.release(); subtrees.release(); parent.release(); mark.release(); lohi.release();
     keys.release(); vals.release();
     m0.release(); m1.release(); m2.release(); m3.release(); m4.release(); m5.release(); m6.release(); m7.release();
     kd_refs.release();
@@ -135,6 +136,8 @@ struct BatchDesc {  // device copy per scene: its geometry
   const float* verts;
   const uint32_t* idx;
   const float4* sph;
+  const float4* verts4;  // 16-byte copies (triangles)
+  const uint4* idx4;
 };
 // All arrays of a batch of LBVH structures, back to back (see batch.cu).
 struct BatchStore {
@@ -142,7 +145,7 @@ struct BatchStore {
   uint32_t n_scenes = 0;
   std::vector<uint32_t> poff, voff;  // n + 1 prefix sums of primitives / points
   std::vector<BatchDesc> host_desc;
-  DevBuf desc, offs, lohi, nodes, prims, order, codes, roots, parent, keys, keys_alt, vals, vals_alt, zero;
+  DevBuf desc, offs, lohi, nodes, prims, order, codes, roots, subtrees, keys, keys_alt, vals, vals_alt, zero;
   size_t zero_words = 0;
   cudaError_t allocate();
   cudaError_t upload_tables(cudaStream_t st);
@@ -151,11 +154,45 @@ struct BatchStore {
   ~BatchStore() { release(); }
   void release() {
     desc.release(); offs.release(); lohi.release(); nodes.release(); prims.release(); order.release();
-    codes.release(); roots.release(); parent.release(); keys.release(); keys_alt.release(); vals.release();
+    codes.release(); roots.release(); subtrees.release(); keys.release(); keys_alt.release(); vals.release();
     vals_alt.release(); zero.release();
   }
 };
 int batch_sort_passes(uint32_t n_scenes);
+
+// The LBVH of sorted codes (lbvh.cu): nodes, payload and root boxes, of one
+// scene (verts, idx, sph) or of several back to back (desc, poff, n_scenes).
+constexpr uint32_t kTreeWindow = 256;   // leaves a block
+constexpr uint32_t kTreeMaxLeft = 128;   // subtrees a block may leave over
+inline uint32_t tree_windows(uint32_t n) { return (n + kTreeWindow - 1) / kTreeWindow; }
+inline size_t tree_pool_bytes(uint32_t n) { return 32 * (size_t)kTreeMaxLeft * tree_windows(n); }
+struct TreeArgs {
+  int kind = kTriangles;
+  const float4* verts = nullptr;  // 16-byte copies
+  const uint4* idx = nullptr;
+  const float4* sph = nullptr;
+  const BatchDesc* desc = nullptr;
+  const uint32_t* poff = nullptr;
+  uint32_t n_scenes = 0;
+  uint32_t n = 0;  // leaves, all scenes
+  const uint32_t* codes = nullptr;  // one scene: sorted codes and primitives
+  const uint32_t* order = nullptr;
+  const uint64_t* keys = nullptr;   // several: sorted (scene << 30) | code and slots, split into these
+  const uint32_t* vals = nullptr;
+  uint32_t* codes_out = nullptr;
+  uint32_t* order_out = nullptr;
+  float4* nodes = nullptr;
+  float4* prims = nullptr;
+  float* roots = nullptr;     // 8 floats a scene
+  uint32_t* flags = nullptr;  // n words, zeroed
+  float4* pool = nullptr;     // tree_pool_bytes(n)
+  uint32_t* err = nullptr;
+  // for the treelet pass (one scene)
+  uint8_t* heights = nullptr;  // node heights (longest path to a leaf)
+  uint32_t* parent = nullptr;  // parent words of the nodes below top nodes: node << 1 | side
+  RefitTop top = {};
+};
+cudaError_t launch_tree(const TreeArgs& a, bool list, cudaStream_t s);
 // One pass of batched kernels over every scene (no allocation, no host sync).
 BuildResult build_batch(BatchStore& b, int morton_mode, uint32_t* err, cudaStream_t st);
 

@@ -100,32 +100,20 @@ void launch_morton_spheres(const float4* sph, uint32_t n, int mode, const int32_
                            uint32_t* keys, uint32_t* vals, uint32_t* hist, cudaStream_t s);
 
 // ---------------------------------------------------------------- LBVH
-// Refit decomposition written by launch_karras: mark[n - 1] (per internal
-// node), top[2048] (top node list), treelets[2n] (uint2 records) and two
-// counters (top nodes, treelets) zeroed before launch_karras.
+// What the treelet pass reads of a built tree: mark (per node: a top node's
+// slot), top[2048] (top node list), treelets[2n] (uint2 records) and the
+// counters, zeroed before the tree is built.
 constexpr uint32_t kRefitTopCapHost = 2048;  // top list capacity (kRefitTopCap on the device)
 struct RefitTop {
   uint32_t* mark;
   uint32_t* top;
   uint32_t* treelets;
-  uint32_t* count;  // [0] top nodes, [1] treelets
+  uint32_t* count;  // [0] top nodes, [1] treelets, [3] treelet queue
 };
 inline size_t refit_treelet_offset(uint32_t n) { return ((size_t)n + kRefitTopCapHost + 1) & ~(size_t)1; }  // 8-byte aligned
 inline size_t refit_mark_words(uint32_t n) { return refit_treelet_offset(n) + 2 * (size_t)n; }
-void launch_karras(const uint32_t* sorted_codes, uint32_t n, float4* nodes, uint32_t* parent,
-                   const RefitTop& top, cudaStream_t s);
-// Gathers each slot's primitive into the slot-ordered payload and computes
-// every node box: treelets in shared memory, one block each, then the top
-// nodes in one block (or by device-scope climbing when they exceed its
-// capacity); root_out gets 6 floats.  heights (optional, n - 1 bytes): the
-// height of every internal node below the top nodes.
-cudaError_t launch_refit(int kind, const float4* verts, const uint4* idx, const float4* sph,
-                         const uint32_t* order, uint32_t n, float4* nodes, const uint32_t* parent,
-                         const RefitTop& top, uint32_t* flags, float4* prims, float* root_out, uint32_t* err,
-                         cudaStream_t s, uint8_t* heights = nullptr);
 // One bottom-up pass of four-leaf treelet restructuring over a refitted LBVH
-// of n one-primitive leaves (the refit decomposition of launch_karras; its
-// treelet queue word top.count[3] must be zero; heights from launch_refit).
+// of n one-primitive leaves (heights and lists from launch_tree).
 cudaError_t launch_treelet_opt(uint32_t n, float4* nodes, const uint32_t* parent, const RefitTop& top,
                                const uint8_t* heights, uint32_t* err, cudaStream_t s);
 // Payload in primitive-id order (KD and brute force) plus per-primitive boxes.

@@ -175,8 +175,8 @@ uint64_t mesh_estimate_bytes(const Mesh& m) {
 }
 
 uint64_t scratch_bytes(const BuildScratch& sc) {
-  return sc.keys_alt.cap + sc.vals_alt.cap + sc.zero.cap + sc.parent.cap + sc.mark.cap + sc.lohi.cap +
-         sc.keys.cap + sc.vals.cap + sc.m0.cap + sc.m1.cap + sc.m2.cap + sc.m3.cap + sc.m4.cap + sc.m5.cap +
+  return sc.keys_alt.cap + sc.vals_alt.cap + sc.zero.cap + sc.subtrees.cap + sc.parent.cap + sc.mark.cap +
+         sc.lohi.cap + sc.keys.cap + sc.vals.cap + sc.m0.cap + sc.m1.cap + sc.m2.cap + sc.m3.cap + sc.m4.cap + sc.m5.cap +
          sc.m6.cap + sc.m7.cap + sc.kd_refs.cap + sc.work.cap;
 }
 

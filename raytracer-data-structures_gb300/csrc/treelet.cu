@@ -1,6 +1,6 @@
 // Treelet restructuring of an LBVH (Karras and Aila 2013, "Fast parallel
 // construction of high-quality bounding volume hierarchies"): one bottom-up
-// pass over the refitted Karras tree.  At every internal node x the treelet
+// pass over the Karras tree.  At every internal node x the treelet
 // grown from x -- its two children, then repeatedly the internal treelet leaf
 // of largest surface area replaced by its two children, up to four treelet
 // leaves -- is rebuilt with the topology of least SAH cost found by dynamic
@@ -19,8 +19,8 @@
 // median split); the walk's hits do not depend on the tree, only the number of
 // nodes a ray visits does.
 //
-// Two kernels, over the refit decomposition k_karras wrote (node heights
-// from the refit): one block per treelet of at most kTreeletSpan leaves,
+// Two kernels, over the lists the tree kernel wrote (node heights, top nodes,
+// treelets): one block per treelet of at most kTreeletSpan leaves,
 // several in flight per SM, then one block over the top nodes, skipped when
 // the top nodes exceed kRefitTopCap (their Karras topology is kept).  Node data
 // stay in global memory (L2): one restructure is a chain of dependent steps,
@@ -275,9 +275,9 @@ __device__ __forceinline__ void list_by_height(uint32_t cnt, uint32_t top_h, con
   __syncthreads();
 }
 
-// Persistent blocks over the refit treelets (queue counter count[3]), several
+// Persistent blocks over the treelets (queue counter count[3]), several
 // per SM so that their level-by-level latencies overlap: a treelet's internal
-// nodes listed by height (heights from the refit), then restructured one
+// nodes listed by height, then restructured one
 // height at a time, node data in global memory.  A treelet covering leaves
 // [lo, lo + cnt) is a subtree of the Karras tree whose root is lo (a right
 // child) or lo + cnt - 1 (a left child); its internal nodes are the other
