@@ -964,9 +964,10 @@ __global__ void __launch_bounds__(128) k_trace_kd(KdView kd, uint32_t n_nodes, c
   }
 }
 
-// The same walk as persistent warps: a grid the GPU holds at once, each warp
-// taking the next 32 rays from a counter (work, zeroed) until none are left.
-template <int KIND, bool ANY, bool REF>
+// The REFERENCE walk as persistent warps: a grid the GPU holds at once, each
+// warp taking the next 32 rays from a counter (work, zeroed) until none are
+// left.
+template <int KIND, bool ANY>
 __global__ void __launch_bounds__(128) k_trace_kd_warps(KdView kd, uint32_t n_nodes, const float4* __restrict__ rays,
                                                         uint32_t n, float4* __restrict__ hits,
                                                         uint32_t* __restrict__ occ, uint32_t* err, uint32_t* work) {
@@ -977,7 +978,7 @@ __global__ void __launch_bounds__(128) k_trace_kd_warps(KdView kd, uint32_t n_no
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= n) break;
     const uint32_t r = base + lane;
-    const bool occluded = r < n && kd_walk_ray<KIND, ANY, REF>(kd, n_nodes, rays, r, hits, err);
+    const bool occluded = r < n && kd_walk_ray<KIND, ANY, true>(kd, n_nodes, rays, r, hits, err);
     if (ANY) {
       const uint32_t bits = __ballot_sync(0xffffffffu, occluded);
       if (lane == 0) occ[base >> 5] = bits;
@@ -1011,17 +1012,19 @@ __global__ void __launch_bounds__(128) k_trace_kd_warps(KdView kd, uint32_t n_no
 // Rays sit in shared memory (a piece moves without its ray; the split axis
 // indexes them), todo entries are 8 bytes (an entry ends where the one below
 // it begins, the last one at t_end).  The node loop converges at every step:
-// left to itself (a loop a lane leaves at its leaf) it took 2080-3200 us
-// where this takes 1950.
-// Measured against the one-lane walk (us): 1023 random rays 194 -> 60, 300k
-// random rays 377 -> 279 (any hit 347 -> 209), 307k camera rays 260 -> 215,
-// their shadow rays 348 -> 257, 2M bounce rays 2020 -> 1950 (lanes per
-// instruction 5.4 -> 10.9, but leaves of unequal length now take most of the
-// issue slots); 2M coherent shadow rays lose, 697 -> 778 (300k: 260 -> 219),
-// so any-hit launches over a million rays walk one ray a lane.
-constexpr int kKdChunk = 8;  // 2 / 3 / 4 / 8 / 16: 2352 / 2126 / 2025 / 1960 / 2031 us
-constexpr int kKdIdle = 8;   // lanes idle before pieces move
-constexpr uint32_t kKdSharedAnyMax = 1u << 20;  // longer any-hit launches walk one ray a lane (dispatch_kd)
+// left to itself (a loop a lane leaves at its leaf) it was up to 1.6 times
+// slower.  Leaves hold from one to some dozens of primitives, so each lane
+// testing its own left the warp waiting for the longest: the lists of the
+// leaves reached are tested as one, a primitive a lane, and a leaf's answer
+// is the smallest (t, place in the list), which is what testing them in turn
+// finds.
+// us, one lane a ray / lanes shared, own leaves / leaves spread: 1023 random
+// rays 194 / 60 / 46, 300k random rays 377 / 279 / 244 (any hit 347 / 209 /
+// 162), 307k camera rays 260 / 215 / 181, their shadow rays 348 / 257 / 212, 2M
+// bounce rays 2020 / 1950 / 1452, 2M coherent shadow rays 697 / 778 / 674.
+constexpr int kKdChunk = 4;  // 2 / 3 / 4 / 5 / 8 / 16, 2M bounce rays: 1681 / 1569 / 1527 / 1518 / 1565 / 1733 us; 300k shadow rays: 176 / 174 / 172 / 175 / 186 / 212
+constexpr uint32_t kKdLeafMax = 1u << 26;  // primitives of a leaf tested at one meeting (32 lanes' fit 32 bits)
+constexpr int kKdIdle = 8;   // lanes idle before pieces move; 5 / 8 / 12: within 1%
 
 __device__ __forceinline__ int2 load_kd(const int4* __restrict__ nodes, int node) {
   return __ldg(reinterpret_cast<const int2*>(nodes + node));
@@ -1031,6 +1034,7 @@ template <bool ANY>
 struct KdShare {
   float o[3][32], inv[3][32], d[3][32], tmin[32], tmax[32];
   uint32_t give[32];
+  unsigned long long leaf[ANY ? 1 : 32]; // a lane's leaf: (t, its place among the leaves' primitives) of the best hit
   unsigned long long key[ANY ? 1 : 32];  // best hit per ray: (order-preserving bits of t + 0, place)
   uint32_t doubt[ANY ? 1 : 32];          // smallest t found before its leaf, order-preserving bits
   uint32_t prim[ANY ? 1 : 32];
@@ -1038,8 +1042,10 @@ struct KdShare {
   float2 uv[ANY ? 1 : 32];
 };
 
+// Blocks an SM: closest hit 6 / 7 / 8: 1641 / 1452 / 1527 us on the bounce
+// rays (8 spill), any hit 8 / 9 / 10: 701 / 674 / 744 on the 2M shadow rays.
 template <int KIND, bool ANY>
-__global__ void __launch_bounds__(128, ANY ? 9 : 8) k_trace_kd_shared(KdView kd, uint32_t n_nodes,
+__global__ void __launch_bounds__(128, ANY ? 9 : 7) k_trace_kd_shared(KdView kd, uint32_t n_nodes,
                                                                    const float4* __restrict__ rays, uint32_t n,
                                                                    float4* __restrict__ hits,
                                                                    uint32_t* __restrict__ occ, uint32_t* err,
@@ -1118,38 +1124,78 @@ __global__ void __launch_bounds__(128, ANY ? 9 : 8) k_trace_kd_shared(KdView kd,
           }
           __syncwarp();
         }
-        bool hit = false, doubt = false;
-        float doubt_t = 0.f;
-        if (walk && (w.y & 3) == 3) {
-          const int leaf_n = w.y >> 2;
-          const F3 o = {sh.o[0][home], sh.o[1][home], sh.o[2][home]}, d = {sh.d[0][home], sh.d[1][home], sh.d[2][home]};
-          const float rtmin = sh.tmin[home];
-          for (int i = 0; i < leaf_n; ++i) {
-            const uint32_t id = (uint32_t)(leaf_n == 1 ? w.x : __ldg(kd.prim_idx + w.x + i));
-            // equal t: only over a hit from later in the order
-            const float bound = !ANY && place > lo ? nextafterf(best, __int_as_float(0x7F800000)) : best;
-            float t, u = 0.f, v = 0.f;
-            bool ok;
+        // The leaves' primitives, spread over the warp: the leaves' lists laid
+        // end to end in lane order, one primitive a lane at a time.
+        bool hit = false;
+        const uint32_t whole = walk && (w.y & 3) == 3 ? (uint32_t)w.y >> 2 : 0u;
+        const uint32_t leaf_n = whole > kKdLeafMax + 1u ? kKdLeafMax : whole;
+        uint32_t end = leaf_n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t x = __shfl_up_sync(0xffffffffu, end, o);
+          if ((int)lane >= o) end += x;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, end, 31), from = end - leaf_n;
+        const uint32_t owners = __ballot_sync(0xffffffffu, leaf_n != 0u);
+        if (leaf_n) sh.give[__popc(owners & below)] = lane;
+        if constexpr (!ANY) sh.leaf[lane] = ~0ull;
+        // equal t: only over a hit from later in the order
+        const float bound = !ANY && place > lo ? nextafterf(best, __int_as_float(0x7F800000)) : best;
+        unsigned long long mine_leaf = ~0ull;
+        uint32_t begun = 0;  // leaves that begin before this batch
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t batch = 0; batch < total; batch += 32) {
+          const uint32_t p = batch + lane, at = from - batch;
+          const uint32_t starts = __reduce_or_sync(0xffffffffu, leaf_n && at < 32u ? 1u << at : 0u);
+          const bool live = p < total;
+          const int src = live ? (int)sh.give[begun + __popc(starts & (below | 1u << lane)) - 1u] : (int)lane;
+          begun += __popc(starts);
+          const int list = __shfl_sync(0xffffffffu, w.x, src);
+          const uint32_t list_n = __shfl_sync(0xffffffffu, leaf_n, src), list_from = __shfl_sync(0xffffffffu, from, src);
+          const uint32_t h = __shfl_sync(0xffffffffu, home, src);
+          const float bnd = __shfl_sync(0xffffffffu, bound, src);
+          float t = 0.f, u = 0.f, v = 0.f;
+          uint32_t id = 0;
+          bool ok = false;
+          if (live) {
+            id = (uint32_t)(list_n == 1u ? list : __ldg(kd.prim_idx + list + (p - list_from)));
+            const F3 o = {sh.o[0][h], sh.o[1][h], sh.o[2][h]}, d = {sh.d[0][h], sh.d[1][h], sh.d[2][h]};
             if (KIND == kTriangles) {
               const float4* q = kd.prims + 3 * (size_t)id;
-              ok = tri_mt(__ldg(q), __ldg(q + 1), __ldg(q + 2), o, d, rtmin, bound, t, u, v);
+              ok = tri_mt(__ldg(q), __ldg(q + 1), __ldg(q + 2), o, d, sh.tmin[h], bnd, t, u, v);
             } else {
-              ok = sphere_closest(__ldg(kd.prims + id), o, d, rtmin, bound, false, t);
+              ok = sphere_closest(__ldg(kd.prims + id), o, d, sh.tmin[h], bnd, false, t);
             }
-            if (!ok) continue;
-            if (ANY) {
-              hit = true;
-              break;
-            }
-            if (shared && t < tMin) {  // an earlier leaf's
-              doubt_t = doubt ? fminf(doubt_t, t) : t;
-              doubt = true;
-              continue;
-            }
-            best = t; bprim = id; bu = u; bv = v;
-            place = shared ? lo : 0u;
-            hit = true;
           }
+          __syncwarp();
+          if (!__any_sync(0xffffffffu, ok)) continue;
+          if constexpr (ANY) {
+            found |= __reduce_or_sync(0xffffffffu, ok ? 1u << h : 0u);
+          } else {
+            const float begin = __shfl_sync(0xffffffffu, tMin, src);
+            const bool early = ok && shared && t < begin;  // an earlier leaf's
+            if (early) atomicMin(&sh.doubt[h], order_key(t));
+            // the first of the smallest: list order is p's order, p's lane p & 31
+            if (ok && !early) atomicMin(&sh.leaf[src], (unsigned long long)order_key(__fadd_rn(t, 0.f)) << 32 | p);
+            __syncwarp();
+            const unsigned long long now = sh.leaf[lane];
+            const int win = (int)((uint32_t)now & 31u);
+            const float nt = __shfl_sync(0xffffffffu, t, win), nu = __shfl_sync(0xffffffffu, u, win);
+            const float nv = __shfl_sync(0xffffffffu, v, win);
+            const uint32_t nid = __shfl_sync(0xffffffffu, id, win);
+            if (now != mine_leaf) {
+              mine_leaf = now;
+              best = nt; bprim = nid; bu = nu; bv = nv;
+              place = shared ? lo : 0u;
+              hit = true;
+            }
+          }
+        }
+        if (leaf_n != whole) {
+          w.x += (int)leaf_n;
+          w.y -= (int)(leaf_n << 2);
+        } else if (walk && (w.y & 3) == 3) {
           if (tp > bot) {
             const int2 e = todo[--tp];
             node = e.x;
@@ -1163,14 +1209,10 @@ __global__ void __launch_bounds__(128, ANY ? 9 : 8) k_trace_kd_shared(KdView kd,
         }
         __syncwarp();
         if constexpr (ANY) {
-          if (__any_sync(0xffffffffu, hit)) {
-            found |= __reduce_or_sync(0xffffffffu, hit ? 1u << home : 0u);
-            if ((found >> home) & 1u) walk = false;
-          }
-        } else if (shared && __any_sync(0xffffffffu, hit || doubt)) {
+          if ((found >> home) & 1u) walk = false;
+        } else if (shared && __any_sync(0xffffffffu, hit)) {
           const unsigned long long mine = ((unsigned long long)order_key(__fadd_rn(best, 0.f)) << 32) | place;
           if (hit) atomicMin(&sh.key[home], mine);
-          if (doubt) atomicMin(&sh.doubt[home], order_key(doubt_t));
           __syncwarp();
           const unsigned long long now = sh.key[home];
           if (hit && now == mine) {  // one piece, one t: one lane
@@ -1297,15 +1339,10 @@ void dispatch_kd(int traversal, const KdView& v, uint32_t n_nodes, const float4*
                  uint32_t* occ, uint32_t* err, uint32_t* work, cudaStream_t s) {
   const unsigned g = (n + 127) / 128;
   if (work) {
-    if (traversal == RQ_TRAVERSAL_REFERENCE || (ANY && n > kKdSharedAnyMax)) {
+    if (traversal == RQ_TRAVERSAL_REFERENCE) {
       cudaMemsetAsync(work, 0, 4, s);
-      if (traversal == RQ_TRAVERSAL_REFERENCE) {
-        const uint32_t blocks = kd_resident_blocks<k_trace_kd_warps<KIND, ANY, true>>();
-        k_trace_kd_warps<KIND, ANY, true><<<std::min(g, blocks), 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work);
-      } else {
-        const uint32_t blocks = kd_resident_blocks<k_trace_kd_warps<KIND, ANY, false>>();
-        k_trace_kd_warps<KIND, ANY, false><<<std::min(g, blocks), 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work);
-      }
+      const uint32_t blocks = kd_resident_blocks<k_trace_kd_warps<KIND, ANY>>();
+      k_trace_kd_warps<KIND, ANY><<<std::min(g, blocks), 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work);
       return;
     }
     // fewer rays a warp when there are fewer rays than resident lanes, and no

@@ -106,8 +106,8 @@ def test_shared_lanes_kd(engine, oracle, rqm, terrain, n_rays):
     _kd_check(engine, oracle, rqm, oracle.TRIANGLES, engine.scene_triangles(v, f), prims, _grazing(n_rays, 80 + n_rays))
 
 
-def test_shared_lanes_kd_any_hit_over_the_shared_limit(engine, oracle, rqm, terrain):
-    """One ray a lane from 2^20 rays on: the same bits on both sides of the line."""
+def test_shared_lanes_kd_any_hit_million_rays(engine, oracle, rqm, terrain):
+    """A launch of more than 2^20 rays gives the bits of its parts."""
     v, f = terrain
     prims, _, _ = oracle.tri_prims(v, f)
     acc = engine.build(engine.scene_triangles(v, f), rqm.KDTREE)
@@ -115,6 +115,18 @@ def test_shared_lanes_kd_any_hit_over_the_shared_limit(engine, oracle, rqm, terr
     bits = rqm.unpack_bits(engine.trace_any(acc, rays), len(rays))
     below = rqm.unpack_bits(engine.trace_any(acc, rays[:1 << 20]), 1 << 20)
     assert np.array_equal(bits[:1 << 20], below)
+
+
+@pytest.mark.parametrize("depth", [1, 4, 9])
+@pytest.mark.parametrize("n_rays", [1, 33, 20_001])
+def test_shared_lanes_kd_long_leaves(engine, oracle, rqm, terrain, n_rays, depth):
+    """Leaves of dozens to thousands of primitives, each triangle there three times: equal distances within and across
+    batches of 32 go to the first of the leaf's list."""
+    v, f = terrain
+    f = np.concatenate([f[: len(f) // 8]] * 3)
+    engine.configure(kd_max_depth=depth)
+    prims, _, _ = oracle.tri_prims(v, f)
+    _kd_check(engine, oracle, rqm, oracle.TRIANGLES, engine.scene_triangles(v, f), prims, _grazing(n_rays, 90 + n_rays))
 
 
 @pytest.mark.parametrize("n_rays", [700, 100_003])
