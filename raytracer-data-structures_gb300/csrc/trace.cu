@@ -70,13 +70,13 @@ __global__ void __launch_bounds__(kThreads, 10) k_trace_fast(Bvh2View bvh, const
 // list[0]) for k_trace_exact, so this kernel carries only the fused walk.
 // UNIT: the LBVH's one-primitive leaves (4-byte stack entries).
 template <int KIND, bool ANY, bool UNIT>
-__global__ void __launch_bounds__(kThreads, kWalkBlocks) k_trace_warps(Bvh2View bvh, const float4* __restrict__ rays,
+__global__ void __launch_bounds__(kThreads, UNIT ? kWalkBlocks : kWalkBlocksWide) k_trace_warps(Bvh2View bvh, const float4* __restrict__ rays,
                                                           uint32_t n, float4* __restrict__ hits,
                                                           uint32_t* __restrict__ occ, uint32_t* err,
                                                           const uint32_t* __restrict__ perm,
                                                           uint32_t* __restrict__ list) {
-  __shared__ WarpShare<ANY, false> share[kThreads / 32];
-  WarpShare<ANY, false>& sh = share[threadIdx.x >> 5];
+  __shared__ WarpShare<ANY, false, UNIT> share[kThreads / 32];
+  WarpShare<ANY, false, UNIT>& sh = share[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31;
   for (;;) {
     uint32_t base = 0;
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kThreads) k_trace_once(Bvh2View bvh, const flo
                                                          float4* __restrict__ hits, uint32_t* __restrict__ occ,
                                                          uint32_t* err, const uint32_t* __restrict__ perm,
                                                          uint32_t grab, const uint32_t* __restrict__ n_dev) {
-  __shared__ WarpShare<ANY, false> share[kThreads / 32];
+  __shared__ WarpShare<ANY, false, UNIT> share[kThreads / 32];
   __shared__ uint32_t bits[kThreads / 32];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = gridDim.x * (kThreads / 32);
   if (n_dev) {

@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(BLOCK, W == 2 ? 1152 / BLOCK : 1) k_trace_batc
                                                          float4* __restrict__ hits, uint32_t* __restrict__ occ,
                                                          uint32_t* __restrict__ work, uint32_t* err,
                                                          const uint32_t* __restrict__ perm) {
-  __shared__ WarpShare<ANY, true> share[W == 2 ? BLOCK / 32 : 1];
+  __shared__ WarpShare<ANY, true, UNIT> share[W == 2 ? BLOCK / 32 : 1];
   const uint32_t lane = threadIdx.x & 31;
   for (;;) {
     uint32_t base = 0;

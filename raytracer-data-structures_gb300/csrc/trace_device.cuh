@@ -395,15 +395,15 @@ __device__ __forceinline__ bool walk_bvh8(const Bvh8View& bvh, const Ray& ray, C
 // What it is for: with one lane a ray the warp waits for its longest ray
 // (8.5 of 32 lanes busy on bounce rays), and a ray is one chain of dependent
 // fetches (a launch of few rays lasts as long as its longest chain).  With
-// shared lanes 17 of 32 are busy and the walk is bound by L1 wavefronts (77%
+// shared lanes 17 of 32 are busy and the walk is bound by L1 wavefronts (80%
 // of peak; the one-lane walk 48%).  Testing leaves once a round instead of
 // at every step matters as much: a tenth of the visits are leaves, so nearly
 // every step of a full warp paid for a leaf test of one or two lanes.
 // Measured on a GB300 against the one-lane walk (us): 8.3M bounce rays
-// 4371 -> 2631 (in octant order 3332 -> 2738), 1M random rays 620 -> 385
-// (any hit 417 -> 317), 2M bounce rays on a median BVH 1421 -> 768, 115k
-// scanner rays 250 -> 168, 1k random rays 82 -> 37; coherent rays gain
-// nothing: 8.3M camera rays 997 -> 1034, shadow rays 999 -> 1003.
+// 4371 -> 2535 (in octant order 3332 -> 2643), 1M random rays 620 -> 368
+// (any hit 417 -> 319), 2M bounce rays on a median BVH 1421 -> 696, 115k
+// scanner rays 250 -> 156, 1k random rays 82 -> 33; coherent rays gain
+// nothing: 8.3M camera rays 997 -> 1042, shadow rays 999 -> 1009.
 //
 // kWalkChunk: 2 / 3 / 4 / 6 / 8 node steps a round give 2915 / 2838 / 2853 /
 // 2922 / 3016 us on the ordered bounce rays, and camera rays want 4 or more
@@ -419,10 +419,24 @@ __device__ __forceinline__ bool walk_bvh8(const Bvh8View& bvh, const Ray& ray, C
 constexpr int kWalkChunk = 4;
 constexpr int kWalkIdle = 12;
 constexpr int kWalkIdleAny = 20;
-constexpr int kWalkBlocks = 10;  // blocks of 128 per SM (48 registers); 8 / 9 / 10: 2920 / 2817 / 2738 us (bounce)
+// Blocks of 128 an SM: 4-byte stack entries 8 / 9 / 10: 2920 / 2817 / 2738 us
+// (bounce rays in octant order), 8-byte ones 721 / 696 / 764 (2M bounce rays on
+// a median BVH; 10 spill).
+constexpr int kWalkBlocks = 10, kWalkBlocksWide = 9;
 
-template <bool ANY, bool MANY>
+// Stack entries of a closest-hit walk that sit in shared memory, the deeper
+// ones in local memory: the lanes' stack heights differ, so a push or pop of
+// the warp touches as many lines of local memory as there are heights, but
+// one line of banks here.  0 / 8 / 12 entries: 383 / 370 / 368 us on the
+// random rays, 2627 / 2547 / 2535 bounce, 745 / 696 / 696 on the median BVH
+// (8-byte entries), 1028 / 1042 / 1042 camera.  Any hit keeps its stack local:
+// 0 / 8 entries 1009 / 1024 us on the coherent shadow rays, 319 / 311 random.
+template <bool ANY>
+constexpr int kWalkTop = ANY ? 0 : 12;
+
+template <bool ANY, bool MANY, bool UNIT>
 struct WarpShare {
+  typename std::conditional<UNIT, int, int2>::type stack[kWalkTop<ANY> ? kWalkTop<ANY> : 1][32];
   uint32_t give[32];           // a meeting's donors, by rank
   const float4* prims[MANY ? 32 : 1];    // MANY: the structure of each ray
   const uint32_t* order[MANY ? 32 : 1];
@@ -466,10 +480,17 @@ __device__ __forceinline__ bool slab_pairs(const SlabRay& r, float lx, float hx,
 // to different structures (bvh is the lane's own).
 template <int KIND, bool ANY, bool UNIT, int STACK, bool MANY>
 __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay sr, bool walk, bool eager, Closest& c,
-                                          WarpShare<ANY, MANY>& sh, uint32_t* err) {
+                                          WarpShare<ANY, MANY, UNIT>& sh, uint32_t* err) {
   constexpr bool kShare = ANY || KIND == kTriangles;
   const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-  typename std::conditional<UNIT, int, int2>::type stack[STACK];
+  using Entry = typename std::conditional<UNIT, int, int2>::type;
+  constexpr int kTop = kWalkTop<ANY>;
+  Entry deep[STACK];
+  auto get = [&](int i) -> Entry {
+    if constexpr (kTop > 0)
+      if (i < kTop) return sh.stack[i][lane];
+    return deep[i];
+  };
   int sp = 0, bot = 0;  // entries [bot, sp): lanes that take over work take the entry at bot
   int cur = bvh.n_internal ? 0 : -1;
   int cnt = bvh.n_internal ? 0 : (int)bvh.n_slots;
@@ -498,9 +519,9 @@ __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay 
     if (sp == bot) {
       walk = false;
     } else if constexpr (UNIT) {
-      cur = stack[--sp];
+      cur = get(--sp);
     } else {
-      const int2 e = stack[--sp];
+      const int2 e = get(--sp);
       cur = e.x;
       cnt = e.y;
     }
@@ -520,13 +541,19 @@ __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay 
         cur = left ? l.x : l.y;
         if (!UNIT) cnt = left ? l.z : l.w;
         if (hl && hr) {
-          if (sp >= STACK) {
+          Entry e;
+          if constexpr (UNIT) e = left ? l.y : l.x;
+          else e = left ? make_int2(l.y, l.w) : make_int2(l.x, l.z);
+          if (kTop > 0 && sp < kTop) {
+            sh.stack[sp][lane] = e;
+          } else if (sp < STACK) {
+            deep[sp] = e;
+          } else {
             atomicOr(err, kErrStackOverflow);
             walk = false;
             break;
           }
-          if constexpr (UNIT) stack[sp++] = left ? l.y : l.x;
-          else stack[sp++] = left ? make_int2(l.y, l.w) : make_int2(l.x, l.z);
+          ++sp;
         }
       } else {
         pop();
@@ -582,9 +609,9 @@ __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay 
     int give = 0, give_cnt = 0;
     if (walk && sp > bot && rank < pairs) {
       if constexpr (UNIT) {
-        give = stack[bot++];
+        give = get(bot++);
       } else {
-        const int2 e = stack[bot++];
+        const int2 e = get(bot++);
         give = e.x;
         give_cnt = e.y;
       }
