@@ -661,11 +661,32 @@ rq_status_t rq_accel_export_kd(rq_ctx_t ctx, rq_accel_t a, int32_t* nodes, int32
 
 // ----------------------------------------------------------------- queries
 
+// Whether a host-buffer query goes chunk by chunk.  From pinned arrays the
+// copies overlap the traversals from half a million rays on (closest hits of
+// 0.6M / 1M / 3M / 6M bounce rays: 415 / 635 / 1730 / 2199 us whole or in the
+// former chunks, 349 / 486 / 1151 / 2120 now).  Copies of pageable arrays wait
+// for each other, so more chunks cost more there (2M any hit 736 us whole, 996
+// in chunks) until there are enough rays for full ones; a ray order pays off
+// over the whole batch.
+static bool pinned(const void* p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeHost;
+}
+static bool streams(const rq_settings_t& cfg, const void* rays, const void* out, uint32_t n) {
+  if (n >= 2 * kPipeChunk) return true;
+  return n >= kPipeMin && cfg.ray_sort == RQ_RAY_SORT_NONE && pinned(rays) && pinned(out);
+}
+
 // Streamed query over host buffers: per chunk, upload on pipe.up, trace on
 // the context's stream, download on pipe.down, with kPipeSlots device slots
 // in rotation (a slot is re-filled only after its previous download).
 static rq_status_t trace_streamed_enqueue(rq_ctx_t ctx, rq_accel_t a, const rq_ray_t* rays, uint32_t n,
-                                          void* out, bool any, const rq_settings_t& cfg, bool join_downloads = true) {
+                                          void* out, bool any, const rq_settings_t& cfg, bool join_downloads = true,
+                                          bool begins = true, bool ends = true) {
   HostPipe& p = ctx->pipe;
   RQ_TRY_CUDA(ctx, p.init());
   const size_t out_chunk = any ? kPipeChunk / 8 : (size_t)kPipeChunk * 16;
@@ -675,33 +696,30 @@ static rq_status_t trace_streamed_enqueue(rq_ctx_t ctx, rq_accel_t a, const rq_r
   }
   // Traversals start after everything already queued on the context's
   // stream (a rebuild, say); uploads start at once, overlapping that work,
-  // after only the previous call's use of each slot (events never recorded
-  // are complete).
+  // each after only the previous use of its slot (events never recorded are
+  // complete).
   RQ_TRY_CUDA(ctx, cudaEventRecord(p.start, ctx->stream));
   RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.down, p.start, 0));
   RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.lane2, p.start, 0));
-  for (int k = 0; k < kPipeSlots; ++k) RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.up, p.downloaded[k], 0));
   const SceneView sv = scene_view(a->scene);
-  // Chunk plan: a quarter and a half chunk first (a short first upload), full
-  // chunks, then halving chunks at the end (a short last traversal and
-  // download).  Every chunk but the last is a multiple of 32 rays, so
-  // occlusion words never straddle chunks.
+  // Chunk plan: doubling chunks while nothing is being traced yet (a short
+  // first upload), full chunks, then halving chunks where nothing follows (a
+  // short last traversal and download).  Every chunk but the last is a
+  // multiple of 32 rays, so occlusion words never straddle chunks.
   std::vector<uint32_t> plan;
-  for (uint64_t left = n; left > 0;) {
-    uint64_t size = plan.empty() ? kPipeChunk / 4 : plan.size() == 1 ? kPipeChunk / 2 : kPipeChunk;
-    if (left <= 2ull * kPipeChunk) {
-      uint64_t half = (left / 2) & ~uint64_t(31);
-      size = std::min<uint64_t>(size, std::max<uint64_t>(kPipeChunk / 4, half));
-    }
-    size = std::min<uint64_t>(size, left);
-    plan.push_back((uint32_t)size);
-    left -= size;
+  const uint64_t head = std::min<uint64_t>(n / 4, std::max<uint64_t>(kPipeHead, n / 16)) & ~uint64_t(31);
+  for (uint64_t left = n, size = begins ? head : kPipeChunk; left > 0; size *= 2) {
+    size = std::min<uint64_t>(size, kPipeChunk);
+    if (ends && left <= 2 * size) size = std::max(head, (left / 2) & ~uint64_t(31));
+    const uint64_t take = std::min(size, left);
+    plan.push_back((uint32_t)take);
+    left -= take;
   }
   uint64_t first = 0;
   for (uint32_t c = 0; c < (uint32_t)plan.size(); first += plan[c], ++c) {
-    const int sl = (int)(c % kPipeSlots);
+    const int sl = (int)(p.next++ % kPipeSlots);
     const uint32_t m = plan[c];
-    if (c >= (uint32_t)kPipeSlots) RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.up, p.downloaded[sl], 0));
+    RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.up, p.downloaded[sl], 0));
     RQ_TRY_CUDA(ctx, cudaMemcpyAsync(p.rays[sl].p, rays + first, (size_t)m * 32, cudaMemcpyHostToDevice, p.up));
     RQ_TRY_CUDA(ctx, cudaEventRecord(p.uploaded[sl], p.up));
     cudaStream_t lane = (c & 1) ? p.lane2 : ctx->stream;
@@ -760,7 +778,8 @@ static rq_status_t trace(rq_ctx_t ctx, rq_accel_t a, const rq_ray_t* rays, uint3
   if (n == 0) return RQ_SUCCESS;
   if (!rays || !out) return fail(ctx, RQ_ERROR_INVALID_ARGUMENT, "null ray or result buffer");
   const bool dev = flags & RQ_DEVICE_POINTERS;
-  if (!dev && n >= 2 * kPipeChunk) return trace_streamed(ctx, a, rays, n, out, any);
+  if (!dev && !ctx->debug.small_stack && streams(ctx->settings, rays, out, n))
+    return trace_streamed(ctx, a, rays, n, out, any);
   const float4* d_rays = nullptr;
   RQ_TRY(to_device(ctx, ctx->stage_in, reinterpret_cast<const float4*>(rays), (size_t)n * 32, flags, &d_rays));
   const size_t out_bytes = any ? (size_t)((n + 31) / 32) * 4 : (size_t)n * 16;
@@ -847,10 +866,12 @@ rq_status_t rq_trace_candidates(rq_ctx_t ctx, rq_accel_t a, const rq_ray_t* rays
   return collect_device_errors(ctx);
 }
 
-// Several host-buffer queries in one call: the first streams chunk by chunk,
-// the others upload whole (on the upload stream, behind the first's chunks)
-// while earlier queries trace, trace as full batches on the context's stream
-// and download while later ones trace.
+// Several host-buffer queries in one call, each streamed chunk by chunk
+// through the same slots or whole (uploaded behind the chunks before it, traced
+// as one batch on the context's stream, downloaded while later ones trace).
+// With the second query's upload waiting for the first's last chunk, 6M
+// closest-hit and 6M any-hit queries took 3745 us; as one train of chunks
+// 2878, where their traversals alone take 2738.
 static rq_status_t trace_queries_enqueue(rq_ctx_t ctx, rq_accel_t a, const rq_query_t* qs, uint32_t nq) {
   HostPipe& p = ctx->pipe;
   RQ_TRY_CUDA(ctx, p.init());
@@ -861,17 +882,14 @@ static rq_status_t trace_queries_enqueue(rq_ctx_t ctx, rq_accel_t a, const rq_qu
     if (q.scheduling >= 0) c.scheduling = q.scheduling;
     return c;
   };
-  // The first query streams in chunks unless it has a ray order: an order
-  // pays off over the whole batch (sorted chunks of 2M rays trace about as
-  // slowly as unsorted ones), so such a query uploads whole like the others.
-  uint32_t first = 0;
-  if (qs[0].n >= 2 * kPipeChunk && cfg_of(qs[0]).ray_sort == RQ_RAY_SORT_NONE) {
-    RQ_TRY(trace_streamed_enqueue(ctx, a, qs[0].rays, qs[0].n, qs[0].out, qs[0].any != 0, cfg_of(qs[0]), false));
-    first = 1;
-  } else {
-    RQ_TRY_CUDA(ctx, cudaEventRecord(p.start, ctx->stream));
-    RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.down, p.start, 0));
-  }
+  // whole: the queries that upload, trace and download as one batch (an
+  // order pays off over the whole batch: sorted chunks of 2M rays trace about
+  // as slowly as unsorted ones)
+  std::vector<bool> whole(nq);
+  for (uint32_t k = 0; k < nq; ++k)
+    whole[k] = cfg_of(qs[k]).ray_sort != RQ_RAY_SORT_NONE || !streams(cfg_of(qs[k]), qs[k].rays, qs[k].out, qs[k].n);
+  RQ_TRY_CUDA(ctx, cudaEventRecord(p.start, ctx->stream));
+  RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.down, p.start, 0));
   if (p.q_rays.size() < nq) {
     p.q_rays.resize(nq);
     p.q_out.resize(nq);
@@ -881,16 +899,25 @@ static rq_status_t trace_queries_enqueue(rq_ctx_t ctx, rq_accel_t a, const rq_qu
     RQ_TRY_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     p.q_events.push_back(e);
   }
-  for (uint32_t k = first; k < nq; ++k) {
+  for (uint32_t k = 0; k < nq; ++k) {
     const rq_query_t& q = qs[k];
     if (q.n == 0) continue;
+    if (!whole[k]) {
+      for (DevBuf& b : p.out) RQ_TRY_CUDA(ctx, b.ensure((size_t)kPipeChunk * (q.any ? 1 : 128) / 8));
+      continue;
+    }
     const size_t out_bytes = q.any ? (size_t)((q.n + 31) / 32) * 4 : (size_t)q.n * 16;
     RQ_TRY_CUDA(ctx, p.q_rays[k].ensure((size_t)q.n * 32));
     RQ_TRY_CUDA(ctx, p.q_out[k].ensure(out_bytes));
   }
-  for (uint32_t k = first; k < nq; ++k) {
+  for (uint32_t k = 0; k < nq; ++k) {
     const rq_query_t& q = qs[k];
     if (q.n == 0) continue;
+    if (!whole[k]) {
+      RQ_TRY(trace_streamed_enqueue(ctx, a, q.rays, q.n, q.out, q.any != 0, cfg_of(q), false, k == 0,
+                                    k + 1 == nq));
+      continue;
+    }
     cudaEvent_t up = p.q_events[2 * k], done = p.q_events[2 * k + 1];
     // the upload overwrites this query's buffer once the previous call's
     // traversal of it is done (uploads overlap work queued before the call)

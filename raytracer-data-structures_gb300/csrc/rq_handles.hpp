@@ -12,18 +12,21 @@
 
 using namespace rq;
 
-// Host-buffer queries of at least 2 chunks are streamed: chunk k+1 uploads
-// (one copy stream) and chunk k-1 downloads (another) while chunk k is traced.
-// Chunks alternate between two compute lanes (the context's stream and one
+// Host-buffer queries of at least 2 chunks, or kPipeMin rays in pinned arrays,
+// are streamed: chunk k+1 uploads (one copy stream) and chunk k-1 downloads
+// (another) while chunk k is traced.  Chunks alternate between two compute lanes (the context's stream and one
 // more, each with its own sort scratch) so that the slow tail of one chunk's
 // traversal overlaps the start of the next.
 constexpr uint32_t kPipeChunk = 1u << 21;  // rays per chunk: 64 MB up, 32 MB (or 256 KB of bits) down
-constexpr int kPipeSlots = 3;
+constexpr uint32_t kPipeMin = 1u << 19;
+constexpr uint32_t kPipeHead = 1u << 18;  // smallest first chunk, unless that is a quarter of the rays
+constexpr int kPipeSlots = 4;  // 3 / 4 / 5: 3062 / 2878 / 2886 us on 6M closest-hit and 6M any-hit rays
 struct HostPipe {
   cudaStream_t up = nullptr, down = nullptr, lane2 = nullptr;
   BuildScratch scratch2;
   cudaEvent_t start = nullptr, uploaded[kPipeSlots] = {}, traced[kPipeSlots] = {}, downloaded[kPipeSlots] = {};
   DevBuf rays[kPipeSlots], out[kPipeSlots];
+  uint32_t next = 0;                   // the next chunk's slot
   std::vector<DevBuf> q_rays, q_out;   // whole-query buffers of rq_trace_queries
   std::vector<cudaEvent_t> q_events;   // uploaded / traced per query
   bool ready = false;
