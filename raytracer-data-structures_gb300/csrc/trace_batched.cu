@@ -2,14 +2,15 @@
 //
 // Rays of all structures lie back to back; ray_off (n_views + 1 entries)
 // gives each structure's range.  The grid is sized to what the SMs hold at
-// once; each warp takes blocks of 256 consecutive rays from a global counter
+// once; each warp takes 32 consecutive rays at a time from a global counter
 // until none are left, so long and short structures, coherent and incoherent
 // rays share the GPU without a tail per structure.  Each ray finds its
 // structure by binary search over ray_off and walks it with the same FAST
 // walk as a one-structure query (identical results; the binary walk shares
 // the warp's lanes, walk_warp, whose rays may belong to different
-// structures).  64 scenes, 8M random rays: closest hit 2798 -> 2399 us, any
-// hit 2271 -> 1976 us; 8 / 9 / 10 blocks of 128 per SM 2409 / 2399 / 2451.
+// structures).  64 scenes, 8M random rays: closest hit 2798 us with one lane a
+// ray, 2171 now, any hit 2271 and 1869 (256 rays per counter access: 2377 and
+// 1982, 64: 2292 and 1882); 8 / 9 / 10 blocks of 128 per SM 2191 / 2171 / 2380.
 //
 // Launch shapes (block size, traversal stack depth) are template choices that
 // rq_plan_create times on the caller's rays; a stack too shallow for a tree
@@ -18,8 +19,6 @@
 
 namespace rq {
 namespace {
-
-constexpr uint32_t kGrab = 256;  // rays a warp takes per counter access (8 passes of 32)
 
 // UNIT: every structure of the launch has single-primitive leaves (batched
 // LBVH builds): 4-byte stack entries.
@@ -34,60 +33,57 @@ __global__ void __launch_bounds__(BLOCK, W == 2 ? 1152 / BLOCK : 1) k_trace_batc
   const uint32_t lane = threadIdx.x & 31;
   for (;;) {
     uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(work, kGrab);
+    if (lane == 0) base = atomicAdd(work, 32u);
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= n) return;  // the whole warp leaves together
-#pragma unroll 1
-    for (uint32_t sub = 0; sub < kGrab && base + sub < n; sub += 32) {
-      const uint32_t w = base + sub + lane;  // work index; the ray itself through perm
-      const uint32_t r = (perm && w < n) ? __ldg(perm + w) : w;
-      bool occluded = false;
-      if constexpr (W == 2) {
-        // the warp's rays share its lanes (walk_warp); rays that need the
-        // exact box test are walked on their own first
-        Bvh2View v{};
-        Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
-        SlabRay sr = {};
-        bool walk = w < n;
-        if (walk) {
-          v = views[segment_of(roff, n_views, r)];
-          ray = load_ray(rays, r);
-          sr = slab_ray(ray.o, ray.d);
-        }
-        Closest c = {ray.tmax, kMiss, 0.f, 0.f};
-        bool exact_hit = false;
-        if (walk && zero_dir(sr)) {
-          uint32_t visits = 0, tests = 0;
-          exact_hit = walk_bvh2_form<KIND, ANY, false, STACK, true, UNIT>(v, ray, sr, c, visits, tests, err);
-          if (!ANY) store_hit(hits, r, c);
-          walk = false;
-        }
-        __syncwarp();
-        const bool own = walk;
-        occluded = walk_warp<KIND, ANY, UNIT, STACK, true>(v, ray, sr, walk, false, c, share[threadIdx.x >> 5], err);
-        if (!ANY && own) store_hit(hits, r, c);
-        occluded = occluded || exact_hit;
-      } else if (w < n) {
-        const Bvh2View v = views[segment_of(roff, n_views, r)];
-        const Ray ray = load_ray(rays, r);
-        Closest c = {ray.tmax, kMiss, 0.f, 0.f};
-        uint32_t visits = 0, tests = 0;
-        if (W == 4) {
-          const Bvh4View v4{v.nodes, v.prims, v.order, v.root, v.n_internal, v.n_slots};
-          occluded = walk_bvh4<KIND, ANY, false, STACK>(v4, ray, c, visits, tests, err);
-        } else {
-          const Bvh8View v8{v.nodes, v.prims, v.order, v.root, v.n_internal, v.n_slots};
-          occluded = walk_bvh8<KIND, ANY, false, STACK>(v8, ray, c, visits, tests, err);
-        }
-        if (!ANY) store_hit(hits, r, c);
+    const uint32_t w = base + lane;  // work index; the ray itself through perm
+    const uint32_t r = (perm && w < n) ? __ldg(perm + w) : w;
+    bool occluded = false;
+    if constexpr (W == 2) {
+      // the warp's rays share its lanes (walk_warp); rays that need the
+      // exact box test are walked on their own first
+      Bvh2View v{};
+      Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
+      SlabRay sr = {};
+      bool walk = w < n;
+      if (walk) {
+        v = views[segment_of(roff, n_views, r)];
+        ray = load_ray(rays, r);
+        sr = slab_ray(ray.o, ray.d);
       }
-      if (ANY) {
-        if (perm) {  // bits of scattered rays: set one by one in the zeroed words
-          if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
-        } else {
-          const uint32_t bits = __ballot_sync(0xffffffffu, occluded);
-          if (lane == 0) occ[(base + sub) >> 5] = bits;
-        }
+      Closest c = {ray.tmax, kMiss, 0.f, 0.f};
+      bool exact_hit = false;
+      if (walk && zero_dir(sr)) {
+        uint32_t visits = 0, tests = 0;
+        exact_hit = walk_bvh2_form<KIND, ANY, false, STACK, true, UNIT>(v, ray, sr, c, visits, tests, err);
+        if (!ANY) store_hit(hits, r, c);
+        walk = false;
+      }
+      __syncwarp();
+      const bool own = walk;
+      occluded = walk_warp<KIND, ANY, UNIT, STACK, true>(v, ray, sr, walk, false, c, share[threadIdx.x >> 5], err);
+      if (!ANY && own) store_hit(hits, r, c);
+      occluded = occluded || exact_hit;
+    } else if (w < n) {
+      const Bvh2View v = views[segment_of(roff, n_views, r)];
+      const Ray ray = load_ray(rays, r);
+      Closest c = {ray.tmax, kMiss, 0.f, 0.f};
+      uint32_t visits = 0, tests = 0;
+      if (W == 4) {
+        const Bvh4View v4{v.nodes, v.prims, v.order, v.root, v.n_internal, v.n_slots};
+        occluded = walk_bvh4<KIND, ANY, false, STACK>(v4, ray, c, visits, tests, err);
+      } else {
+        const Bvh8View v8{v.nodes, v.prims, v.order, v.root, v.n_internal, v.n_slots};
+        occluded = walk_bvh8<KIND, ANY, false, STACK>(v8, ray, c, visits, tests, err);
+      }
+      if (!ANY) store_hit(hits, r, c);
+    }
+    if (ANY) {
+      if (perm) {  // bits of scattered rays: set one by one in the zeroed words
+        if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
+      } else {
+        const uint32_t bits = __ballot_sync(0xffffffffu, occluded);
+        if (lane == 0) occ[base >> 5] = bits;
       }
     }
   }
@@ -104,7 +100,7 @@ cudaError_t launch_shape(const BatchedTrace& t, cudaStream_t s) {
   int dev = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  const uint64_t want_warps = ((uint64_t)t.n + kGrab - 1) / kGrab;
+  const uint64_t want_warps = ((uint64_t)t.n + 31) / 32;
   uint64_t blocks = (uint64_t)(per_sm > 0 ? per_sm : 1) * sms;
   const uint64_t enough = (want_warps * 32 + BLOCK - 1) / BLOCK;  // no more warps than work blocks
   if (blocks > enough) blocks = enough;
