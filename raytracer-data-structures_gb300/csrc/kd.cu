@@ -1019,9 +1019,9 @@ __global__ void __launch_bounds__(128) k_trace_kd_warps(KdView kd, uint32_t n_no
 // is the smallest (t, place in the list), which is what testing them in turn
 // finds.
 // us, one lane a ray / lanes shared, own leaves / leaves spread: 1023 random
-// rays 194 / 60 / 46, 300k random rays 377 / 279 / 244 (any hit 347 / 209 /
-// 162), 307k camera rays 260 / 215 / 181, their shadow rays 348 / 257 / 212, 2M
-// bounce rays 2020 / 1950 / 1452, 2M coherent shadow rays 697 / 778 / 674.
+// rays 194 / 60 / 42, 300k random rays 377 / 279 / 237 (any hit 347 / 209 /
+// 162), 307k camera rays 260 / 215 / 174, their shadow rays 348 / 257 / 212, 2M
+// bounce rays 2020 / 1950 / 1400, 2M coherent shadow rays 697 / 778 / 674.
 constexpr int kKdChunk = 4;  // 2 / 3 / 4 / 5 / 8 / 16, 2M bounce rays: 1681 / 1569 / 1527 / 1518 / 1565 / 1733 us; 300k shadow rays: 176 / 174 / 172 / 175 / 186 / 212
 constexpr uint32_t kKdLeafMax = 1u << 26;  // primitives of a leaf tested at one meeting (32 lanes' fit 32 bits)
 constexpr int kKdIdle = 8;   // lanes idle before pieces move; 5 / 8 / 12: within 1%
@@ -1044,7 +1044,10 @@ struct KdShare {
 
 // Blocks an SM: closest hit 6 / 7 / 8: 1641 / 1452 / 1527 us on the bounce
 // rays (8 spill), any hit 8 / 9 / 10: 701 / 674 / 744 on the 2M shadow rays.
-template <int KIND, bool ANY>
+// PLACED: every warp has its rays by its place, far apart (k_trace_once,
+// trace.cu; 100k shadow rays 130 -> 95 us), instead of taking them from a
+// counter (one kernel for both: 1517 us on the bounce rays, 1400 apart).
+template <int KIND, bool ANY, bool PLACED>
 __global__ void __launch_bounds__(128, ANY ? 9 : 7) k_trace_kd_shared(KdView kd, uint32_t n_nodes,
                                                                    const float4* __restrict__ rays, uint32_t n,
                                                                    float4* __restrict__ hits,
@@ -1056,14 +1059,17 @@ __global__ void __launch_bounds__(128, ANY ? 9 : 7) k_trace_kd_shared(KdView kd,
   const uint32_t limit = 2u * n_nodes + 8u;  // meetings: a piece has a node of its ray behind it for every one
   int2 todo[kStackSize];                     // (node, bits of tMin)
   for (;;) {
-    // without a counter every warp has its rays by its place
-    uint32_t base = (blockIdx.x * 4 + (threadIdx.x >> 5)) * grab;
-    if (work) {
+    uint32_t base = 0, r;
+    if constexpr (!PLACED) {
       if (lane == 0) base = atomicAdd(work, grab);
       base = __shfl_sync(0xffffffffu, base, 0);
       if (base >= n) break;
+      r = base + lane;
+    } else if constexpr (ANY) {
+      r = ((lane >> 3) * gridDim.x + blockIdx.x) * 32u + ((lane & 7u) << 2 | threadIdx.x >> 5);
+    } else {
+      r = (lane * gridDim.x + blockIdx.x) * 4u + (threadIdx.x >> 5);
     }
-    const uint32_t r = base + lane;
     const bool own = lane < grab && r < n;
     float first = 0.f, last = 0.f;  // the ray's interval in the root box
     bool start = false;
@@ -1299,21 +1305,22 @@ __global__ void __launch_bounds__(128, ANY ? 9 : 7) k_trace_kd_shared(KdView kd,
       if (ANY || !__any_sync(0xffffffffu, open)) break;
     }
     if constexpr (ANY) {
-      if (work) {
+      if constexpr (!PLACED) {
         if (lane == 0) occ[base >> 5] = found;
       } else {  // the block's warps put their bits together (grab is 8 or more)
         __shared__ uint32_t bits[4];
         if (lane == 0) bits[threadIdx.x >> 5] = found;
         __syncthreads();
-        const uint32_t per = 32u / grab, word = blockIdx.x * grab / 8u + threadIdx.x;  // warps a word
+        const uint32_t word = threadIdx.x * gridDim.x + blockIdx.x;
         if (threadIdx.x < grab / 8u && word < (n + 31) / 32) {
           uint32_t w = 0;
-          for (uint32_t q = 0; q < per; ++q) w |= bits[threadIdx.x * per + q] << (q * grab);
+          for (uint32_t q = 0; q < 4; ++q)
+            for (uint32_t l = 0; l < 8; ++l) w |= ((bits[q] >> (threadIdx.x * 8 + l)) & 1u) << (l << 2 | q);
           occ[word] = w;
         }
       }
     }
-    if (!work) break;
+    if constexpr (PLACED) break;
   }
 }
 
@@ -1347,15 +1354,15 @@ void dispatch_kd(int traversal, const KdView& v, uint32_t n_nodes, const float4*
     }
     // fewer rays a warp when there are fewer rays than resident lanes, and no
     // counter when every warp's rays follow from its place, as for the BVH (trace.cu)
-    const uint32_t blocks = kd_resident_blocks<k_trace_kd_shared<KIND, ANY>>();
+    const uint32_t blocks = kd_resident_blocks<k_trace_kd_shared<KIND, ANY, false>>();
     uint32_t grab = 32u;
     while (grab > (ANY ? 8u : 1u) && (uint64_t)blocks * 4 * (grab / 2) >= n) grab /= 2;
     const uint32_t need = (n + 4 * grab - 1) / (4 * grab);
     if (need <= blocks) {
-      k_trace_kd_shared<KIND, ANY><<<need, 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, nullptr, grab);
+      k_trace_kd_shared<KIND, ANY, true><<<need, 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, nullptr, grab);
     } else {
       cudaMemsetAsync(work, 0, 4, s);
-      k_trace_kd_shared<KIND, ANY><<<blocks, 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work, grab);
+      k_trace_kd_shared<KIND, ANY, false><<<blocks, 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err, work, grab);
     }
   } else if (traversal == RQ_TRAVERSAL_REFERENCE) {
     k_trace_kd<KIND, ANY, true><<<g, 128, 0, s>>>(v, n_nodes, rays, n, hits, occ, err);

@@ -139,8 +139,18 @@ __global__ void __launch_bounds__(kThreads) k_trace_once(Bvh2View bvh, const flo
     n = __ldg(n_dev);
     grab = rays_a_warp(warps, n, 1u);
   }
-  for (uint32_t base = (blockIdx.x * (kThreads / 32) + warp) * grab;;) {
-    const uint32_t i = base + lane;
+  // Rays next to each other cost about the same, and here the launch lasts as
+  // long as its slowest warp, so a warp's rays lie `warps` apart; any hit: the
+  // block's words lie gridDim.x apart and its warps take every fourth ray of
+  // each.  Consecutive / 8 together / far apart: 115k scanner rays 158 / 117 /
+  // 91 us, 120k camera rays 138 / 91 / 68, their bounce rays 117 / 115 / 111,
+  // their shadow rays 91 / 64 / -, 65k rays down on a terrain 89 / 76 / 58.  In
+  // the last turns of a launch from the counter (k_trace_warps) it costs more
+  // than it gives: 1M random rays 368 -> 383, 8.3M camera rays 1048 -> 1159.
+  uint32_t slot = lane * warps + blockIdx.x * (kThreads / 32) + warp;
+  if (ANY && !perm) slot = ((lane >> 3) * gridDim.x + blockIdx.x) * 32u + ((lane & 7u) << 2 | warp);
+  for (uint32_t base = 0;;) {
+    const uint32_t i = base + slot;
     const bool live = lane < grab && i < n;
     Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
     SlabRay sr = {};
@@ -170,11 +180,12 @@ __global__ void __launch_bounds__(kThreads) k_trace_once(Bvh2View bvh, const flo
       const uint32_t mine = __ballot_sync(0xffffffffu, occluded);
       if (lane == 0) bits[warp] = mine;
       __syncthreads();
-      const uint32_t per = 32u / grab, word = blockIdx.x * grab / 8u + threadIdx.x;  // warps a word
+      const uint32_t word = threadIdx.x * gridDim.x + blockIdx.x;
       if (threadIdx.x < grab / 8u && word < (n + 31) / 32) {
-        uint32_t w = 0;
-        for (uint32_t q = 0; q < per; ++q) w |= bits[threadIdx.x * per + q] << (q * grab);
-        occ[word] = w;
+        uint32_t out = 0;
+        for (uint32_t q = 0; q < 4; ++q)
+          for (uint32_t l = 0; l < 8; ++l) out |= ((bits[q] >> (threadIdx.x * 8 + l)) & 1u) << (l << 2 | q);
+        occ[word] = out;
       }
     }
     if (!n_dev) break;

@@ -402,7 +402,7 @@ __device__ __forceinline__ bool walk_bvh8(const Bvh8View& bvh, const Ray& ray, C
 // Measured on a GB300 against the one-lane walk (us): 8.3M bounce rays
 // 4371 -> 2535 (in octant order 3332 -> 2643), 1M random rays 620 -> 368
 // (any hit 417 -> 319), 2M bounce rays on a median BVH 1421 -> 696, 115k
-// scanner rays 250 -> 156, 1k random rays 82 -> 33; coherent rays gain
+// scanner rays 250 -> 91, 1k random rays 82 -> 31; coherent rays gain
 // nothing: 8.3M camera rays 997 -> 1042, shadow rays 999 -> 1009.
 //
 // kWalkChunk: 2 / 3 / 4 / 6 / 8 node steps a round give 2915 / 2838 / 2853 /
