@@ -260,7 +260,7 @@ rq_status_t rq_accel_destroy(rq_accel_t accel);
 
 /* Build one structure per scene.  RQ_LBVH builds the whole batch in one pass
  * of batched kernels (scene boxes, Morton codes, one segmented radix sort by
- * (scene, code), Karras topology, refit), the arrays of all scenes back to
+ * (scene, code), the trees), the arrays of all scenes back to
  * back in one allocation that lives until the last of the returned
  * structures is destroyed; each structure equals the one rq_build would make
  * from its scene.  The scenes must all hold triangles or all spheres, with
@@ -369,15 +369,17 @@ typedef struct rq_query_t {
 } rq_query_t;
 /* Several host-buffer queries on one structure in one call, with copies
  * and traversals overlapped across queries: queries run in the given order;
- * the first streams chunk by chunk when it has no ray order, the others (and
- * a first query with a ray order, whose order pays off only over the whole
- * batch) upload whole while earlier ones trace, each traced as one batch,
+ * large queries without a ray order (4M rays, or half a million in pinned
+ * arrays) stream chunk by chunk, one after another, up to the first query that
+ * is not one; that one and those behind it (an order pays off only over the
+ * whole batch) upload whole while earlier ones trace, each traced as one batch,
  * and download while later ones trace.  Uploads begin at once, overlapping
  * work already queued on the context's stream such as a rebuild.  Put the
  * query with the longest traversal first.  Results equal
  * rq_trace_closest / rq_trace_any per query; returns when every result is in
- * host memory.  Device memory: each query after the first keeps a buffer of
- * its rays and results (grow-only, per context). */
+ * host memory.  Device memory: four slots of a chunk's rays and results, and
+ * for each query that uploads whole a buffer of its rays and results
+ * (grow-only, per context). */
 rq_status_t rq_trace_queries(rq_ctx_t ctx, rq_accel_t accel, const rq_query_t* queries, uint32_t n_queries);
 
 /* The FAST closest/any query of rq_trace_closest / rq_trace_any that also

@@ -882,12 +882,16 @@ static rq_status_t trace_queries_enqueue(rq_ctx_t ctx, rq_accel_t a, const rq_qu
     if (q.scheduling >= 0) c.scheduling = q.scheduling;
     return c;
   };
-  // whole: the queries that upload, trace and download as one batch (an
-  // order pays off over the whole batch: sorted chunks of 2M rays trace about
-  // as slowly as unsorted ones)
+  // whole: the queries that upload, trace and download as one batch: those
+  // with a ray order (it pays off over the whole batch: sorted chunks of 2M
+  // rays trace about as slowly as unsorted ones) and those behind one, whose
+  // upload has all of its traversal to hide under, not four slots' worth.
   std::vector<bool> whole(nq);
-  for (uint32_t k = 0; k < nq; ++k)
-    whole[k] = cfg_of(qs[k]).ray_sort != RQ_RAY_SORT_NONE || !streams(cfg_of(qs[k]), qs[k].rays, qs[k].out, qs[k].n);
+  for (uint32_t k = 0; k < nq; ++k) {
+    const rq_settings_t c = cfg_of(qs[k]);
+    whole[k] = k && whole[k - 1];
+    if (qs[k].n && (c.ray_sort != RQ_RAY_SORT_NONE || !streams(c, qs[k].rays, qs[k].out, qs[k].n))) whole[k] = true;
+  }
   RQ_TRY_CUDA(ctx, cudaEventRecord(p.start, ctx->stream));
   RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.down, p.start, 0));
   if (p.q_rays.size() < nq) {
