@@ -395,7 +395,7 @@ __device__ __forceinline__ bool walk_bvh8(const Bvh8View& bvh, const Ray& ray, C
 // What it is for: with one lane a ray the warp waits for its longest ray
 // (8.5 of 32 lanes busy on bounce rays), and a ray is one chain of dependent
 // fetches (a launch of few rays lasts as long as its longest chain).  With
-// shared lanes 17 of 32 are busy and the walk is bound by L1 wavefronts (80%
+// shared lanes 17 of 32 are busy and the walk is bound by L1 wavefronts (85%
 // of peak; the one-lane walk 48%).  Testing leaves once a round instead of
 // at every step matters as much: a tenth of the visits are leaves, so nearly
 // every step of a full warp paid for a leaf test of one or two lanes.
