@@ -825,14 +825,16 @@ cudaError_t launch_refill_kind(const Bvh2View& v, const float4* rays, uint32_t n
 // between them of more than 2^-20 of the larger decides; a smaller one, an
 // infinity or a NaN is left to box_ref.  plain: no direction component so small
 // or large that a reciprocal or a product loses bits other than by underflow,
-// which the constant in the margin covers.
+// which the constant in the margin covers, and a finite origin (fminf and fmaxf
+// pass over a NaN that box_ref's comparisons would not).
 struct RefRay {
   F3 inv;
   bool plain;
 };
-__device__ __forceinline__ RefRay ref_ray(F3 d) {
+__device__ __forceinline__ RefRay ref_ray(F3 o, F3 d) {
   auto mid = [](float x) { return fabsf(x) > 0x1p-60f && fabsf(x) < 0x1p60f; };
-  return {{__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z)}, mid(d.x) && mid(d.y) && mid(d.z)};
+  const bool finite = fabsf(o.x) < 0x1p60f && fabsf(o.y) < 0x1p60f && fabsf(o.z) < 0x1p60f;
+  return {{__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z)}, finite && mid(d.x) && mid(d.y) && mid(d.z)};
 }
 __device__ __noinline__ bool box_ref_exact(F3 o, F3 d, float lx, float hx, float ly, float hy, float lz, float hz) {
   float a0, a1;
@@ -872,7 +874,7 @@ __global__ void __launch_bounds__(kThreads) k_trace_ref(Bvh2View bvh, const floa
   Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
   if (walk) ray = load_ray(rays, r);
   Closest c = {ray.tmax, kMiss, 0.f, 0.f};
-  const RefRay rr = ref_ray(ray.d);
+  const RefRay rr = ref_ray(ray.o, ray.d);
   const float* rb = bvh.root;
   if (walk) walk = box_ref_hit(ray.o, ray.d, rr, rb[0], rb[3], rb[1], rb[4], rb[2], rb[5]);
   int2 stack[kStackSize];
