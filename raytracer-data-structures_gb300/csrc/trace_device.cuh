@@ -403,7 +403,7 @@ __device__ __forceinline__ bool walk_bvh8(const Bvh8View& bvh, const Ray& ray, C
 // 4371 -> 2535 (in octant order 3332 -> 2643), 1M random rays 620 -> 368
 // (any hit 417 -> 319), 2M bounce rays on a median BVH 1421 -> 696, 115k
 // scanner rays 250 -> 91, 1k random rays 82 -> 31; coherent rays gain
-// nothing: 8.3M camera rays 997 -> 1042, shadow rays 999 -> 1009.
+// nothing: 8.3M camera rays 997 -> 1032, shadow rays 999 -> 1009.
 //
 // kWalkChunk: 2 / 3 / 4 / 6 / 8 node steps a round give 2915 / 2838 / 2853 /
 // 2922 / 3016 us on the ordered bounce rays, and camera rays want 4 or more
@@ -562,11 +562,10 @@ __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay 
     bool hit = false;  // any hit: the ray is occluded; closest hit: c is a new one
     if (walk && cur < 0) {
       if (UNIT) cnt = 1;
-      const uint32_t had = c.prim;
-      const float had_t = c.t;
+      const uint32_t had = c.prim;  // a leaf is tested once: a new hit is another primitive
       hit = test_leaf<KIND, ANY, false>(MANY ? sh.prims[MANY ? home : 0] : bvh.prims,
                                         MANY ? sh.order[MANY ? home : 0] : bvh.order, (uint32_t)(~cur), cnt, ray, c);
-      if (!ANY) hit = c.prim != had || c.t != had_t;
+      if (!ANY) hit = c.prim != had;
       pop();
     }
     __syncwarp();

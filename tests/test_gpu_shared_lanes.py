@@ -68,6 +68,22 @@ def test_shared_lanes_rays_with_a_zero_direction_component(engine, oracle, rqm, 
     assert np.array_equal(rqm.unpack_bits(engine.trace_any(acc, rays), len(rays)), occ)
 
 
+def test_shared_lanes_rays_without_an_end(engine, oracle, rqm, terrain):
+    """tmax infinite or not a number, tmin above tmax, among rays that share lanes: the oracle's bits."""
+    v, f = terrain
+    prims, _, _ = oracle.tri_prims(v, f)
+    acc = engine.build(engine.scene_triangles(v, f), rqm.LBVH)
+    tree = _oracle_tree(engine, oracle, acc)
+    rays = _grazing(5000, 13)
+    rays["tmax"][::5] = np.nan
+    rays["tmax"][1::7] = np.inf
+    rays["tmax"][2::11] = -1.0
+    want = oracle.trace_bvh2(oracle.TRIANGLES, oracle.FAST, oracle.CLOSEST, tree, prims, rays)
+    occ = oracle.trace_bvh2(oracle.TRIANGLES, oracle.FAST, oracle.ANY, tree, prims, rays)
+    assert np.array_equal(_u32(engine.trace_closest(acc, rays)), _u32(want))
+    assert np.array_equal(rqm.unpack_bits(engine.trace_any(acc, rays), len(rays)), occ)
+
+
 def test_shared_lanes_many_structures(engine, oracle, rqm, terrain):
     """Warps whose rays belong to several structures of different sizes."""
     meshes = [terrain, scenes.displaced_icosphere(2, seed=4), scenes.heightfield(9, 7, seed=6), terrain]
