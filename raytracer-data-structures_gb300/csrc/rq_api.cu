@@ -702,19 +702,7 @@ static rq_status_t trace_streamed_enqueue(rq_ctx_t ctx, rq_accel_t a, const rq_r
   RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.down, p.start, 0));
   RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.lane2, p.start, 0));
   const SceneView sv = scene_view(a->scene);
-  // Chunk plan: doubling chunks while nothing is being traced yet (a short
-  // first upload), full chunks, then halving chunks where nothing follows (a
-  // short last traversal and download).  Every chunk but the last is a
-  // multiple of 32 rays, so occlusion words never straddle chunks.
-  std::vector<uint32_t> plan;
-  const uint64_t head = std::min<uint64_t>(n / 4, std::max<uint64_t>(kPipeHead, n / 16)) & ~uint64_t(31);
-  for (uint64_t left = n, size = begins ? head : kPipeChunk; left > 0; size *= 2) {
-    size = std::min<uint64_t>(size, kPipeChunk);
-    if (ends && left <= 2 * size) size = std::max(head, (left / 2) & ~uint64_t(31));
-    const uint64_t take = std::min(size, left);
-    plan.push_back((uint32_t)take);
-    left -= take;
-  }
+  const std::vector<uint32_t> plan = chunk_plan(n, begins, ends);
   uint64_t first = 0;
   for (uint32_t c = 0; c < (uint32_t)plan.size(); first += plan[c], ++c) {
     const int sl = (int)(p.next++ % kPipeSlots);

@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 
+#include "host_chunks.hpp"
 #include "rq_build.hpp"
 #include "rq_internal.hpp"
 
@@ -17,9 +18,6 @@ using namespace rq;
 // (another) while chunk k is traced.  Chunks alternate between two compute lanes (the context's stream and one
 // more, each with its own sort scratch) so that the slow tail of one chunk's
 // traversal overlaps the start of the next.
-constexpr uint32_t kPipeChunk = 1u << 21;  // rays per chunk: 64 MB up, 32 MB (or 256 KB of bits) down
-constexpr uint32_t kPipeMin = 1u << 19;
-constexpr uint32_t kPipeHead = 1u << 18;  // smallest first chunk, unless that is a quarter of the rays
 constexpr int kPipeSlots = 4;  // 3 / 4 / 5: 3062 / 2878 / 2886 us on 6M closest-hit and 6M any-hit rays
 struct HostPipe {
   cudaStream_t up = nullptr, down = nullptr, lane2 = nullptr;
