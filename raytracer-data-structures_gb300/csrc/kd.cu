@@ -1292,7 +1292,8 @@ __global__ void __launch_bounds__(128, ANY ? 9 : 7) k_trace_kd_shared(KdView kd,
       if constexpr (!ANY) {
         bool again = false;
         if (shared) {
-          const float2 uv = sh.uv[lane];  // written before the last meeting's ballot
+          __syncwarp();  // the last round's stores; a ballot does not order memory
+          const float2 uv = sh.uv[lane];
           best = sh.t[lane];
           bprim = sh.prim[lane];
           bu = uv.x;

@@ -647,7 +647,8 @@ __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay 
   }
   if constexpr (!ANY) {
     if (shared) {
-      const float2 uv = sh.uv[lane];  // written before the last meeting's ballot
+      __syncwarp();  // the last round's stores; a ballot does not order memory
+      const float2 uv = sh.uv[lane];
       c = {sh.t[lane], (uint32_t)sh.key[lane], uv.x, uv.y};
       __syncwarp();
     }
