@@ -78,13 +78,15 @@ __global__ void __launch_bounds__(kThreads, UNIT ? kWalkBlocks : kWalkBlocksWide
   __shared__ WarpShare<ANY, false, UNIT> share[kThreads / 32];
   WarpShare<ANY, false, UNIT>& sh = share[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31;
+  uint32_t base = 0, again = 0;  // again: closest hits in doubt, walked once more without sharing
   for (;;) {
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(list + 1, 32u);
-    base = __shfl_sync(0xffffffffu, base, 0);
+    if (ANY || again == 0u) {
+      if (lane == 0) base = atomicAdd(list + 1, 32u);
+      base = __shfl_sync(0xffffffffu, base, 0);
+    }
     if (base >= n) break;
     const uint32_t i = base + lane;
-    const bool live = i < n;
+    const bool live = i < n && (ANY || again == 0u || (again >> lane & 1u));
     Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
     SlabRay sr = {};
     bool walk = live;
@@ -99,10 +101,11 @@ __global__ void __launch_bounds__(kThreads, UNIT ? kWalkBlocks : kWalkBlocksWide
     }
     const bool own = walk;  // this lane's ray is walked here
     Closest c = {ray.tmax, kMiss, 0.f, 0.f};
-    const bool occluded = walk_warp<KIND, ANY, UNIT, kStackSize, false>(bvh, ray, sr, walk, false, c, sh, err);
+    const bool occluded = walk_warp<KIND, ANY, UNIT, kStackSize, false, false>(bvh, ray, sr, walk, false, again != 0u, c, sh, err);
     const uint32_t r = (perm && live) ? __ldg(perm + i) : i;
     if (!ANY) {
       if (own) store_hit(hits, r, c);
+      again = __ballot_sync(0xffffffffu, own && occluded);
     } else if (perm) {
       if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
     } else {
@@ -149,9 +152,10 @@ __global__ void __launch_bounds__(kThreads) k_trace_once(Bvh2View bvh, const flo
   // than it gives: 1M random rays 368 -> 383, 8.3M camera rays 1048 -> 1159.
   uint32_t slot = lane * warps + blockIdx.x * (kThreads / 32) + warp;
   if (ANY && !perm) slot = ((lane >> 3) * gridDim.x + blockIdx.x) * 32u + ((lane & 7u) << 2 | warp);
+  uint32_t again = 0;  // closest hits in doubt, walked once more without sharing
   for (uint32_t base = 0;;) {
     const uint32_t i = base + slot;
-    const bool live = lane < grab && i < n;
+    const bool live = lane < grab && i < n && (ANY || again == 0u || (again >> lane & 1u));
     Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
     SlabRay sr = {};
     bool walk = live, exact_hit = false;
@@ -171,9 +175,12 @@ __global__ void __launch_bounds__(kThreads) k_trace_once(Bvh2View bvh, const flo
     __syncwarp();
     const bool own = walk;
     const bool occluded =
-        walk_warp<KIND, ANY, UNIT, kStackSize, false>(bvh, ray, sr, walk, grab < 32u, c, share[warp], err) || exact_hit;
+        walk_warp<KIND, ANY, UNIT, kStackSize, false, true>(bvh, ray, sr, walk, grab < 32u, again != 0u, c, share[warp], err) ||
+        exact_hit;
     if (!ANY) {
       if (own) store_hit(hits, r, c);
+      again = __ballot_sync(0xffffffffu, own && occluded);
+      if (again) continue;
     } else if (perm) {
       if (occluded) atomicOr(occ + (r >> 5), 1u << (r & 31));
     } else {  // one round: every warp of the block is here

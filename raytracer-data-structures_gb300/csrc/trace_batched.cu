@@ -9,8 +9,9 @@
 // walk as a one-structure query (identical results; the binary walk shares
 // the warp's lanes, walk_warp, whose rays may belong to different
 // structures).  64 scenes, 8M random rays: closest hit 2798 us with one lane a
-// ray, 2171 now, any hit 2271 and 1869 (256 rays per counter access: 2377 and
-// 1982, 64: 2292 and 1882); 8 / 9 / 10 blocks of 128 per SM 2191 / 2171 / 2380.
+// ray, 2230 now, any hit 2271 and 1870 (256 rays per counter access were 9 and
+// 6% slower than 32, 64: 6 and 1%); 7 / 8 / 9 blocks of 128 per SM 2327 / 2230 /
+// 2359 (closest hit: 9 spill), 1872 at 8 and 1870 at 9 (any hit).
 //
 // Launch shapes (block size, traversal stack depth) are template choices that
 // rq_plan_create times on the caller's rays; a stack too shallow for a tree
@@ -23,7 +24,7 @@ namespace {
 // UNIT: every structure of the launch has single-primitive leaves (batched
 // LBVH builds): 4-byte stack entries.
 template <int KIND, bool ANY, int W, int STACK, int BLOCK, bool UNIT = false>
-__global__ void __launch_bounds__(BLOCK, W == 2 ? 1152 / BLOCK : 1) k_trace_batched(const Bvh2View* __restrict__ views,
+__global__ void __launch_bounds__(BLOCK, W == 2 ? (ANY ? 1152 : 1024) / BLOCK : 1) k_trace_batched(const Bvh2View* __restrict__ views,
                                                          const uint32_t* __restrict__ roff, uint32_t n_views,
                                                          const float4* __restrict__ rays, uint32_t n,
                                                          float4* __restrict__ hits, uint32_t* __restrict__ occ,
@@ -31,10 +32,12 @@ __global__ void __launch_bounds__(BLOCK, W == 2 ? 1152 / BLOCK : 1) k_trace_batc
                                                          const uint32_t* __restrict__ perm) {
   __shared__ WarpShare<ANY, true, UNIT> share[W == 2 ? BLOCK / 32 : 1];
   const uint32_t lane = threadIdx.x & 31;
+  uint32_t base = 0, again = 0;  // again: closest hits in doubt, walked once more without sharing
   for (;;) {
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(work, 32u);
-    base = __shfl_sync(0xffffffffu, base, 0);
+    if (ANY || again == 0u) {
+      if (lane == 0) base = atomicAdd(work, 32u);
+      base = __shfl_sync(0xffffffffu, base, 0);
+    }
     if (base >= n) return;  // the whole warp leaves together
     const uint32_t w = base + lane;  // work index; the ray itself through perm
     const uint32_t r = (perm && w < n) ? __ldg(perm + w) : w;
@@ -45,7 +48,7 @@ __global__ void __launch_bounds__(BLOCK, W == 2 ? 1152 / BLOCK : 1) k_trace_batc
       Bvh2View v{};
       Ray ray = {{0.f, 0.f, 0.f}, {0.f, 0.f, 1.f}, 0.f, 0.f};
       SlabRay sr = {};
-      bool walk = w < n;
+      bool walk = w < n && (ANY || again == 0u || (again >> lane & 1u));
       if (walk) {
         v = views[segment_of(roff, n_views, r)];
         ray = load_ray(rays, r);
@@ -61,8 +64,10 @@ __global__ void __launch_bounds__(BLOCK, W == 2 ? 1152 / BLOCK : 1) k_trace_batc
       }
       __syncwarp();
       const bool own = walk;
-      occluded = walk_warp<KIND, ANY, UNIT, STACK, true>(v, ray, sr, walk, false, c, share[threadIdx.x >> 5], err);
+      occluded = walk_warp<KIND, ANY, UNIT, STACK, true, true>(v, ray, sr, walk, false, again != 0u, c,
+                                                               share[threadIdx.x >> 5], err);
       if (!ANY && own) store_hit(hits, r, c);
+      if (!ANY) again = __ballot_sync(0xffffffffu, own && occluded);
       occluded = occluded || exact_hit;
     } else if (w < n) {
       const Bvh2View v = views[segment_of(roff, n_views, r)];

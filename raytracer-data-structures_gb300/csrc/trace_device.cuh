@@ -382,15 +382,37 @@ __device__ __forceinline__ bool walk_bvh8(const Bvh8View& bvh, const Ray& ray, C
 // ray; a round is at most kWalkChunk node steps a lane, then one leaf test
 // for the lanes that reached a leaf, then a meeting of the warp: lanes whose
 // ray is finished take over the oldest (largest) stacked subtree of lanes
-// that still have some, with a copy of the ray.  The closest-hit rule
-// (smallest t, ties to the smallest id) makes a ray's result independent of
-// which lane tests which subtree and when, so the results are those of the
-// one-lane walk, as long as no box is culled whose primitive is hit at a
-// smaller t than the box is entered at: the slab test's widening covers the
-// rounding of a triangle's t (113M bounce, camera, scanner and random rays
-// walked without any culling gave the culled walk's hits, bit for bit), not
-// that of a small distant sphere's, whose t cancels.  So closest hits on
-// spheres stay with their lane; its order is the one-lane walk's.
+// that still have some, with a copy of the ray.
+//
+// A ray's result is that of the one-lane walk, whichever lanes walk it and
+// when.  An any-hit walk culls by the ray's own interval alone, so no order
+// matters.  A closest hit is the smallest (t, id) of the primitives tested, so
+// what could differ is which boxes are culled.  Call a hit early when its box
+// would be culled with that very hit as the bound: a triangle's t is off by
+// about |e1||e2||o - v0| 2^-24 / det, and for a long triangle seen edge-on (det
+// is 1e-6 or more) that can be far outside the slab test's widening.  Where no
+// hit is early no bound that is itself a hit culls the answer, and every order
+// gives it; an early hit is the one-lane walk's answer or not by what was found
+// before.  So, once lanes are shared,
+//  * pieces carry their place in the one-lane order (as in the KD walk), and a
+//    lane's bound comes only from hits that the one-lane walk comes to before:
+//    its own, those it got with its piece, and the ray's best one if that is
+//    from an earlier piece;
+//  * an early hit is no bound and no answer, it is noted (the smallest t a
+//    ray), and a ray whose noted t is not behind its answer is walked again by
+//    its own lane alone.  A ray's first piece needs no such care: what it has
+//    found is what the one-lane walk has found by then.
+// Every box that the one-lane walk visits is visited then: what culls it here
+// is a hit from before it whose box the one-lane walk visited too, or culled by
+// a nearer hit.  So an early hit that the one-lane walk may have taken is noted.
+// Boxes are taken to hold what is below them, as those of every build do.
+// Long edge-on triangles among ordinary ones: one ray in eight had another hit
+// in another batch without this.  It costs 1% on 1M random rays, 2% on 8.3M
+// bounce rays, 4% on a median BVH (test beside the vote on hits; inside the
+// leaf test 7, 10 and 7%).
+//
+// Closest hits on spheres stay with their lane: a small distant sphere's t
+// cancels, so early hits are common there.
 //
 // What it is for: with one lane a ray the warp waits for its longest ray
 // (8.5 of 32 lanes busy on bounce rays), and a ray is one chain of dependent
@@ -400,10 +422,10 @@ __device__ __forceinline__ bool walk_bvh8(const Bvh8View& bvh, const Ray& ray, C
 // at every step matters as much: a tenth of the visits are leaves, so nearly
 // every step of a full warp paid for a leaf test of one or two lanes.
 // Measured on a GB300 against the one-lane walk (us): 8.3M bounce rays
-// 4371 -> 2535 (in octant order 3332 -> 2643), 1M random rays 620 -> 368
-// (any hit 417 -> 319), 2M bounce rays on a median BVH 1421 -> 696, 115k
+// 4371 -> 2590 (in octant order 3332 -> 2673), 1M random rays 620 -> 374
+// (any hit 417 -> 319), 2M bounce rays on a median BVH 1421 -> 721, 115k
 // scanner rays 250 -> 91, 1k random rays 82 -> 31; coherent rays gain
-// nothing: 8.3M camera rays 997 -> 1032, shadow rays 999 -> 1009.
+// nothing: 8.3M camera rays 997 -> 1020, shadow rays 999 -> 1009.
 //
 // kWalkChunk: 2 / 3 / 4 / 6 / 8 node steps a round give 2915 / 2838 / 2853 /
 // 2922 / 3016 us on the ordered bounce rays, and camera rays want 4 or more
@@ -420,7 +442,7 @@ constexpr int kWalkChunk = 4;
 constexpr int kWalkIdle = 12;
 constexpr int kWalkIdleAny = 20;
 // Blocks of 128 an SM: 4-byte stack entries 8 / 9 / 10: 2920 / 2817 / 2738 us
-// (bounce rays in octant order), 8-byte ones 721 / 696 / 764 (2M bounce rays on
+// (bounce rays in octant order), 8-byte ones 747 / 721 / 798 (2M bounce rays on
 // a median BVH; 10 spill).
 constexpr int kWalkBlocks = 10, kWalkBlocksWide = 9;
 
@@ -443,7 +465,11 @@ struct WarpShare {
   unsigned long long key[ANY ? 1 : 32];  // best hit per ray: (order-preserving bits of t + 0, prim)
   float t[ANY ? 1 : 32];
   float2 uv[ANY ? 1 : 32];
+  uint32_t place[ANY ? 1 : 32];  // the best hit's place in the one-lane order
+  uint32_t doubt[ANY ? 1 : 32];  // smallest t of an early hit, order-preserving bits
+  uint32_t piece[ANY || MANY ? 1 : 32];  // what a lane walks: places lo .. lo + 2^k - 1 of its ray's order, as lo << 5 | k
 };
+constexpr uint32_t kWholeRay = 27u;  // a piece's size in places is halved at each give; lo has 27 bits
 
 __device__ __forceinline__ float from_order_key(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
@@ -472,15 +498,36 @@ __device__ __forceinline__ bool slab_pairs(const SlabRay& r, float lx, float hx,
   return tnear <= __fmaf_rn(tf, kWiden, r.eps);
 }
 
+// Whether a triangle's hit at t is early: its box, entered with the hit as the
+// bound, may fail the slab test.  The box is the triangle's own from its
+// payload (v0, v1 - v0, v2 - v0), each entry plane moved inwards by more than
+// what the two roundings of a vertex can have moved it; any larger box is
+// entered no later, and its exit has passed the test already.  A NaN is early.
+__device__ __forceinline__ bool early_hit(const float4* __restrict__ tri, const SlabRay& r, float tmin, float t) {
+  const float4 v = __ldg(tri), e1 = __ldg(tri + 1), e2 = __ldg(tri + 2);
+  const float far = __fmaf_rn(t, kWiden, r.eps);
+  auto entered = [&](float p0, float d1, float d2, float inv, float noi) {
+    const float p1 = __fadd_rn(p0, d1), p2 = __fadd_rn(p0, d2);
+    const float p = inv > 0.f ? fminf(fminf(p0, p1), p2) : fmaxf(fmaxf(p0, p1), p2);
+    const float pad = __fmul_rn(__fadd_rn(fabsf(p), fmaxf(fabsf(d1), fabsf(d2))), 0x3p-24f);
+    return __fmaf_rn(__fadd_rn(p, inv > 0.f ? pad : -pad), inv, noi) <= far;
+  };
+  return !(tmin <= far && entered(v.x, e1.x, e2.x, r.inv.x, r.noi.x) && entered(v.y, e1.y, e2.y, r.inv.y, r.noi.y) &&
+           entered(v.z, e1.z, e2.z, r.inv.z, r.noi.z));
+}
+
 // The warp's 32 lanes call it together, each with its ray (walk: it has one,
 // and not one for the exact box test).  c starts as the ray's (tmax, miss)
 // and returns its closest hit; any hit returns whether the lane's ray is
-// occluded.  eager: lanes start without a ray (fewer than 32 rays), so
-// subtrees move as soon as a lane is idle.  MANY: the lanes' rays may belong
-// to different structures (bvh is the lane's own).
-template <int KIND, bool ANY, bool UNIT, int STACK, bool MANY>
-__device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay sr, bool walk, bool eager, Closest& c,
-                                          WarpShare<ANY, MANY, UNIT>& sh, uint32_t* err) {
+// occluded, closest hit whether it is in doubt: the caller walks it again with
+// alone, where no lane takes over another's work.  eager: lanes start without a
+// ray (fewer than 32 rays), so subtrees move as soon as a lane is idle.  MANY:
+// the lanes' rays may belong to different structures (bvh is the lane's own).
+// KEEP: a lane's piece is in a register, not in shared memory: 1-3% faster where
+// registers do not bound the kernel, 1-2% slower where they do (k_trace_warps).
+template <int KIND, bool ANY, bool UNIT, int STACK, bool MANY, bool KEEP>
+__device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay sr, bool walk, bool eager, bool alone,
+                                          Closest& c, WarpShare<ANY, MANY, UNIT>& sh, uint32_t* err) {
   constexpr bool kShare = ANY || KIND == kTriangles;
   const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
   using Entry = typename std::conditional<UNIT, int, int2>::type;
@@ -502,14 +549,19 @@ __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay 
   // takes over a subtree continues its donor's walk: whatever lane is busy at
   // a meeting, at least one node or leaf of its ray lies behind it for every
   // meeting so far.
-  uint32_t max_meetings = 2u * (bvh.n_internal + bvh.n_slots) + 8u;
+  uint32_t meetings = 2u * (bvh.n_internal + bvh.n_slots) + 8u;  // that are left
+  uint32_t piece_reg = kWholeRay;  // KEEP: sh.piece of this lane
+  auto piece = [&]() -> uint32_t& {
+    if constexpr (KEEP) return piece_reg;
+    else return sh.piece[lane];
+  };
+  if constexpr (!ANY && kShare) piece() = kWholeRay;
   if (MANY) {
-    max_meetings = __reduce_max_sync(0xffffffffu, walk ? max_meetings : 0u);
+    meetings = __reduce_max_sync(0xffffffffu, walk ? meetings : 0u);
     sh.prims[MANY ? lane : 0] = bvh.prims;
     sh.order[MANY ? lane : 0] = bvh.order;
     __syncwarp();
   }
-  uint32_t meetings = 0;
   if (walk) {
     float tn;
     const float* rb = bvh.root;
@@ -560,9 +612,11 @@ __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay 
       }
     }
     bool hit = false;  // any hit: the ray is occluded; closest hit: c is a new one
+    const uint32_t had = c.prim;  // a leaf is tested once: a new hit is another primitive
+    const float had_t = c.t;
+    const int leaf = cur;
     if (walk && cur < 0) {
       if (UNIT) cnt = 1;
-      const uint32_t had = c.prim;  // a leaf is tested once: a new hit is another primitive
       hit = test_leaf<KIND, ANY, false>(MANY ? sh.prims[MANY ? home : 0] : bvh.prims,
                                         MANY ? sh.order[MANY ? home : 0] : bvh.order, (uint32_t)(~cur), cnt, ray, c);
       if (!ANY) hit = c.prim != had;
@@ -574,6 +628,17 @@ __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay 
         found |= __reduce_or_sync(0xffffffffu, hit ? 1u << home : 0u);
         if ((found >> home) & 1u) walk = false;
       } else if (shared) {
+        if (hit && piece() >= 32u) {  // not the ray's first piece
+          const float4* tri = (MANY ? sh.prims[MANY ? home : 0] : bvh.prims) + 3 * (size_t)(uint32_t)(~leaf);
+          if (!UNIT)
+            while (__float_as_uint(__ldg(&tri->w)) != c.prim) tri += 3;  // the hit is one of this leaf's
+          if (early_hit(tri, sr, ray.tmin, c.t)) {
+            atomicMin(&sh.doubt[home], order_key(__fadd_rn(c.t, 0.f)));
+            c.t = had_t;
+            c.prim = had;
+            hit = false;
+          }
+        }
         const unsigned long long mine = hit_key(c);
         if (hit) atomicMin(&sh.key[home], mine);
         __syncwarp();
@@ -581,32 +646,40 @@ __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay 
         if (hit && best == mine) {  // equal keys: the same primitive, so the same t, u, v
           sh.t[home] = c.t;
           sh.uv[home] = make_float2(c.u, c.v);
+          sh.place[home] = piece() >> 5;
         }
-        c.t = from_order_key((uint32_t)(best >> 32));
-        c.prim = (uint32_t)best;
+        __syncwarp();
+        if (sh.place[home] <= piece() >> 5) {
+          c.t = from_order_key((uint32_t)(best >> 32));
+          c.prim = (uint32_t)best;
+        }
       }
     }
     const uint32_t busy = __ballot_sync(0xffffffffu, walk);
     if (busy == 0u) break;
-    if (++meetings > max_meetings) {
+    if (meetings-- == 0u) {
       if (lane == 0) atomicOr(err, kErrCorrupt);
       break;
     }
-    if (!kShare || 32 - __popc(busy) < (eager ? 1 : ANY ? kWalkIdleAny : kWalkIdle)) continue;
-    const uint32_t donors = __ballot_sync(0xffffffffu, walk && sp > bot);
+    if (!kShare || (!ANY && alone) || 32 - __popc(busy) < (eager ? 1 : ANY ? kWalkIdleAny : kWalkIdle)) continue;
+    const bool can = walk && sp > bot && (ANY || !kShare || (piece() & 31u));
+    const uint32_t donors = __ballot_sync(0xffffffffu, can);
     if (donors == 0u) continue;
     if constexpr (!ANY) {
       if (!shared) {  // every lane still holds its own ray
         sh.key[lane] = hit_key(c);
         sh.t[lane] = c.t;
         sh.uv[lane] = make_float2(c.u, c.v);
+        sh.place[lane] = 0u;
+        sh.doubt[lane] = 0xFFFFFFFFu;
       }
     }
     shared = true;
     const int pairs = min(__popc(donors), 32 - __popc(busy));
     const int rank = __popc((walk ? donors : ~busy) & below);
     int give = 0, give_cnt = 0;
-    if (walk && sp > bot && rank < pairs) {
+    if (can && rank < pairs) {
+      if constexpr (!ANY) --piece();  // the lower half stays here
       if constexpr (UNIT) {
         give = get(bot++);
       } else {
@@ -636,8 +709,11 @@ __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay 
     if (MANY)
       nodes = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(nodes), src));
     give = __shfl_sync(0xffffffffu, give, src);
+    uint32_t half = 0;
+    if constexpr (!ANY) half = KEEP ? __shfl_sync(0xffffffffu, piece_reg, src) : sh.piece[src];
     if (!UNIT) give_cnt = __shfl_sync(0xffffffffu, give_cnt, src);
     if (take) {
+      if constexpr (!ANY) piece() = half + (32u << (half & 31u));  // the upper half of what the donor had
       walk = true;
       cur = give;
       cnt = give_cnt;
@@ -649,7 +725,10 @@ __device__ __forceinline__ bool walk_warp(const Bvh2View& bvh, Ray ray, SlabRay 
     if (shared) {
       __syncwarp();  // the last round's stores; a ballot does not order memory
       const float2 uv = sh.uv[lane];
-      c = {sh.t[lane], (uint32_t)sh.key[lane], uv.x, uv.y};
+      const unsigned long long best = sh.key[lane];
+      const uint32_t doubt = sh.doubt[lane];
+      c = {sh.t[lane], (uint32_t)best, uv.x, uv.y};
+      found = doubt != 0xFFFFFFFFu && doubt <= (uint32_t)(best >> 32) ? 1u << lane : 0u;
       __syncwarp();
     }
   }
