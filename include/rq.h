@@ -306,8 +306,9 @@ rq_status_t rq_accel_export_bvh4(rq_ctx_t ctx, rq_accel_t accel, float* nodes, u
  * itself is not checked: a cycle makes queries end with
  * RQ_ERROR_INVALID_ARGUMENT ("malformed acceleration structure") once a walk
  * exceeds the steps a valid tree allows, and boxes that miss their primitives
- * lose those hits.  The structure reports type RQ_BVH, is walked with binary
- * nodes whatever settings.node_width says, and cannot be rebuilt
+ * lose those hits (closest-hit queries of triangles then run one lane a ray).
+ * The structure reports type RQ_BVH, is walked with binary nodes whatever
+ * settings.node_width says, and cannot be rebuilt
  * (rq_accel_rebuild: RQ_ERROR_UNSUPPORTED).  No reference counterpart: the
  * reference builds its trees in process (constructBVHNew, accelerators.h:246). */
 rq_status_t rq_accel_import_bvh2(rq_ctx_t ctx, rq_scene_t scene, const float* nodes, uint32_t n_nodes,

@@ -72,7 +72,49 @@ __global__ void __launch_bounds__(256) k_update(const float* __restrict__ verts,
   if (bad) atomicOr(err, kErrBadInput);
 }
 
+// Whether every box of a BVH2 holds what is below it: the boxes of a child
+// node's children, a leaf's triangles.  *loose becomes 1 otherwise.
+__global__ void __launch_bounds__(256) k_check_boxes(const float4* __restrict__ nodes, uint32_t n_nodes,
+                                                     const uint32_t* __restrict__ order, const float* __restrict__ verts,
+                                                     const uint32_t* __restrict__ idx, uint32_t* loose) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> 1, side = t & 1u;
+  if (i >= n_nodes) return;
+  auto child = [&](uint32_t node, uint32_t s, float* b) {  // lo, hi per axis
+    const float4 xy = __ldg(nodes + 4 * (size_t)node + s), z = __ldg(nodes + 4 * (size_t)node + 2);
+    b[0] = xy.x; b[1] = xy.y; b[2] = xy.z; b[3] = xy.w;
+    b[4] = s ? z.z : z.x; b[5] = s ? z.w : z.y;
+  };
+  float b[6];
+  child(i, side, b);
+  const int4 l = __ldg(reinterpret_cast<const int4*>(nodes + 4 * (size_t)i + 3));
+  const int link = side ? l.y : l.x, count = side ? l.w : l.z;
+  bool in = true;
+  if (link >= 0) {
+    for (uint32_t s = 0; s < 2; ++s) {
+      float c[6];
+      child((uint32_t)link, s, c);
+      for (int a = 0; a < 3; ++a) in = in && b[2 * a] <= c[2 * a] && c[2 * a + 1] <= b[2 * a + 1];
+    }
+  } else {
+    for (int k = 0; k < count; ++k) {
+      const uint32_t p = __ldg(order + (uint32_t)(~link) + (uint32_t)k);
+      for (int q = 0; q < 3; ++q) {
+        const float* v = verts + 3 * (size_t)__ldg(idx + 3 * (size_t)p + q);
+        for (int a = 0; a < 3; ++a) in = in && b[2 * a] <= __ldg(v + a) && __ldg(v + a) <= b[2 * a + 1];
+      }
+    }
+  }
+  if (!in) *loose = 1u;
+}
+
 }  // namespace
+
+void launch_check_boxes(const float4* nodes, uint32_t n_nodes, const uint32_t* order, const float* verts,
+                        const uint32_t* idx, uint32_t* loose, cudaStream_t st) {
+  if (n_nodes == 0) return;
+  count_launch();
+  k_check_boxes<<<(unsigned)((2ull * n_nodes + 255) / 256), 256, 0, st>>>(nodes, n_nodes, order, verts, idx, loose);
+}
 
 void launch_update(const float* verts, uint32_t nv, float* to_verts, float4* verts4, const uint32_t* idx, uint32_t nt,
                    uint32_t* to_idx, uint4* idx4, const float* sph, uint32_t n, float4* to_sph, uint32_t* err,
@@ -277,7 +319,7 @@ void launch_query(int type, const SceneView& s, const AccelBuffers& a, int trave
     launch_trace_bvh8(s.kind, any, bvh8_view(a), q.rays, q.n, q.hits, q.occ, err, st);
   } else {
     Bvh2View v{a.nodes.as<const float4>(), a.prims.as<const float4>(), a.order.as<const uint32_t>(),
-               a.root.as<const float>(), a.n_nodes, a.n_slots, a.unit_leaves ? 1u : 0u};
+               a.root.as<const float>(), a.n_nodes, a.n_slots, a.unit_leaves ? 1u : 0u, a.loose ? 1u : 0u};
     launch_trace_bvh2(s.kind, traversal, any, v, q.rays, q.n, q.hits, q.occ, err, st, nullptr, q.small_stack,
                       q.exact);
   }
@@ -331,7 +373,7 @@ BuildResult launch_query_sorted(int type, const SceneView& s, const AccelBuffers
     }
   }
   Bvh2View v{a.nodes.as<const float4>(), a.prims.as<const float4>(), a.order.as<const uint32_t>(),
-             a.root.as<const float>(), a.n_nodes, a.n_slots, a.unit_leaves ? 1u : 0u};
+             a.root.as<const float>(), a.n_nodes, a.n_slots, a.unit_leaves ? 1u : 0u, a.loose ? 1u : 0u};
   if (top) {
     RQ_B(sc.top.ensure(64 * 64), "top-level copy");
     launch_trace_bvh2_top(s.kind, any, v, sc.top.as<float4>(), q.rays, q.n, q.hits, q.occ, err, perm, st);

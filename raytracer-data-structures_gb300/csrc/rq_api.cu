@@ -450,9 +450,15 @@ rq_status_t rq_accel_import_bvh2(rq_ctx_t ctx, rq_scene_t scene, const float* no
     const SceneView sv = scene_view(scene);
     launch_prims_gather(sv.kind, sv.verts, sv.idx, sv.sph, b.order.as<const uint32_t>(), n_slots,
                         b.prims.as<float4>(), ctx->stream);
+    // closest hits on triangles share lanes only where boxes hold what is below them (root word 7)
+    if (sv.kind == kTriangles)
+      launch_check_boxes(b.nodes.as<const float4>(), n_nodes, b.order.as<const uint32_t>(), sv.verts, sv.idx,
+                         b.root.as<uint32_t>() + 7, ctx->stream);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // root8 lives on this stack frame
+  uint32_t loose = 0;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&loose, b.root.as<uint32_t>() + 7, 4, cudaMemcpyDeviceToHost, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);  // root8 and loose live on this stack frame
   if (e != cudaSuccess) {
     b.release();
     delete a;
@@ -462,6 +468,7 @@ rq_status_t rq_accel_import_bvh2(rq_ctx_t ctx, rq_scene_t scene, const float* no
   b.n_slots = n_slots;
   b.node_width = 2;
   b.unit_leaves = unit;
+  b.loose = loose != 0;
   *out = a;
   return RQ_SUCCESS;
 }
@@ -990,7 +997,10 @@ static rq_status_t batch_tables(rq_ctx_t ctx, const rq_accel_t* accels, uint32_t
   t.any = any;
   t.width = (int)accels[0]->buf.node_width;
   t.unit = true;
-  for (uint32_t k = 0; k < n; ++k) t.unit = t.unit && accels[k]->buf.unit_leaves;
+  for (uint32_t k = 0; k < n; ++k) {
+    t.unit = t.unit && accels[k]->buf.unit_leaves;
+    t.loose = t.loose || accels[k]->buf.loose;
+  }
   t.views = reinterpret_cast<const Bvh2View*>(base);
   t.roff = reinterpret_cast<const uint32_t*>(base + vbytes);
   t.n_views = n;

@@ -34,12 +34,13 @@ struct AccelBuffers {
   uint32_t node_width = 2;  // BVH2 structures: 2, or 4 / 8 when nodes4 holds a wide copy
   uint32_t n4_cap = 0;      // bound of the 4-wide node count (exact count: root word 6)
   bool unit_leaves = false; // every BVH2 leaf holds one primitive (LBVH builds)
+  bool loose = false;       // imported boxes that do not hold what is below them
   void release() {
     nodes.release(); prims.release(); order.release(); codes.release(); root.release();
     kd_nodes.release(); kd_idx.release(); nodes4.release();
     n_nodes = n_slots = max_depth = n4_cap = 0;
     node_width = 2;
-    unit_leaves = false;
+    unit_leaves = loose = false;
   }
   size_t device_bytes() const {
     return nodes.cap + prims.cap + order.cap + codes.cap + root.cap + kd_nodes.cap + kd_idx.cap + nodes4.cap;
@@ -222,6 +223,10 @@ BuildResult trace_counted(int type, const SceneView& s, const AccelBuffers& a, b
 void launch_update(const float* verts, uint32_t nv, float* to_verts, float4* verts4, const uint32_t* idx, uint32_t nt,
                    uint32_t* to_idx, uint4* idx4, const float* sph, uint32_t n, float4* to_sph, uint32_t* err,
                    cudaStream_t st);
+// *loose (zeroed by the caller) becomes 1 when a box of the nodes does not
+// hold its child's boxes or its leaf's triangles.
+void launch_check_boxes(const float4* nodes, uint32_t n_nodes, const uint32_t* order, const float* verts,
+                        const uint32_t* idx, uint32_t* loose, cudaStream_t st);
 void launch_validate(const float* verts, uint32_t nv, const uint32_t* idx, uint32_t nt,
                      const float4* sph, uint32_t n, uint32_t* err, cudaStream_t st);
 

@@ -144,6 +144,7 @@ struct Bvh2View {
   uint32_t n_internal;
   uint32_t n_slots;
   uint32_t unit_leaves = 0;  // 1: every leaf holds one primitive (LBVH): 4-byte stack entries
+  uint32_t loose = 0;        // 1: boxes may not hold what is below them: closest hits keep their lane
 };
 // perm (optional): trace ray perm[i] in thread i (results stay in caller order).
 // small_stack (a test hook): the FAST walk's stack holds kDebugStack entries,
@@ -247,6 +248,7 @@ struct BatchedTrace {
   uint32_t* err = nullptr;
   const uint32_t* perm = nullptr;  // optional ray order: work index -> ray index
   bool unit = false;               // every structure's leaves hold one primitive (LBVH)
+  bool loose = false;              // some structure's boxes may not hold what is below them
 };
 // block: 128 or 256 threads; deep: the deeper of the two stack sizes.
 cudaError_t launch_trace_batched(const BatchedTrace& t, int block, int deep, cudaStream_t s);

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kThreads, UNIT ? kWalkBlocks : kWalkBlocksWide
     }
     const bool own = walk;  // this lane's ray is walked here
     Closest c = {ray.tmax, kMiss, 0.f, 0.f};
-    const bool occluded = walk_warp<KIND, ANY, UNIT, kStackSize, false, false>(bvh, ray, sr, walk, false, again != 0u, c, sh, err);
+    const bool occluded = walk_warp<KIND, ANY, UNIT, kStackSize, false, false>(bvh, ray, sr, walk, false, again != 0u || bvh.loose, c, sh, err);
     const uint32_t r = (perm && live) ? __ldg(perm + i) : i;
     if (!ANY) {
       if (own) store_hit(hits, r, c);
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kThreads) k_trace_once(Bvh2View bvh, const flo
     __syncwarp();
     const bool own = walk;
     const bool occluded =
-        walk_warp<KIND, ANY, UNIT, kStackSize, false, true>(bvh, ray, sr, walk, grab < 32u, again != 0u, c, share[warp], err) ||
+        walk_warp<KIND, ANY, UNIT, kStackSize, false, true>(bvh, ray, sr, walk, grab < 32u, again != 0u || bvh.loose, c, share[warp], err) ||
         exact_hit;
     if (!ANY) {
       if (own) store_hit(hits, r, c);

@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(BLOCK, W == 2 ? (ANY ? 1152 : 1024) / BLOCK : 
                                                          const float4* __restrict__ rays, uint32_t n,
                                                          float4* __restrict__ hits, uint32_t* __restrict__ occ,
                                                          uint32_t* __restrict__ work, uint32_t* err,
-                                                         const uint32_t* __restrict__ perm) {
+                                                         const uint32_t* __restrict__ perm, bool loose) {
   __shared__ WarpShare<ANY, true, UNIT> share[W == 2 ? BLOCK / 32 : 1];
   const uint32_t lane = threadIdx.x & 31;
   uint32_t base = 0, again = 0;  // again: closest hits in doubt, walked once more without sharing
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(BLOCK, W == 2 ? (ANY ? 1152 : 1024) / BLOCK : 
       }
       __syncwarp();
       const bool own = walk;
-      occluded = walk_warp<KIND, ANY, UNIT, STACK, true, true>(v, ray, sr, walk, false, again != 0u, c,
+      occluded = walk_warp<KIND, ANY, UNIT, STACK, true, true>(v, ray, sr, walk, false, again != 0u || loose, c,
                                                                share[threadIdx.x >> 5], err);
       if (!ANY && own) store_hit(hits, r, c);
       if (!ANY) again = __ballot_sync(0xffffffffu, own && occluded);
@@ -114,7 +114,7 @@ cudaError_t launch_shape(const BatchedTrace& t, cudaStream_t s) {
   if (ANY && t.perm && (e = cudaMemsetAsync(t.occ, 0, (size_t)((t.n + 31) / 32) * 4, s)) != cudaSuccess) return e;
   count_launch();
   k<<<(unsigned)blocks, BLOCK, 0, s>>>(t.views, t.roff, t.n_views, t.rays, t.n, t.hits, t.occ, t.work, t.err,
-                                       t.perm);
+                                       t.perm, t.loose);
   return cudaGetLastError();
 }
 

@@ -405,7 +405,8 @@ __device__ __forceinline__ bool walk_bvh8(const Bvh8View& bvh, const Ray& ray, C
 // Every box that the one-lane walk visits is visited then: what culls it here
 // is a hit from before it whose box the one-lane walk visited too, or culled by
 // a nearer hit.  So an early hit that the one-lane walk may have taken is noted.
-// Boxes are taken to hold what is below them, as those of every build do.
+// Boxes have to hold what is below them, as those of every build do; an imported
+// tree is checked, and without that its closest hits keep their lanes (alone).
 // Long edge-on triangles among ordinary ones: one ray in eight had another hit
 // in another batch without this.  It costs 1% on 1M random rays, 2% on 8.3M
 // bounce rays, 4% on a median BVH (test beside the vote on hits; inside the
