@@ -294,11 +294,18 @@ __global__ void __launch_bounds__(1024) k_seg_level(Segs g, uint32_t* ctl, int l
 // the split list's order (centroid, primitive), so its side needs no table.
 // k_part_count takes the sides of a tile of one list (ballot words and the
 // tile's left count), k_partition the tile's left elements before it (the
-// earlier tiles' counts, and the counts inside the tile) and scatters.
+// earlier tiles' counts, or their prefix sum, and the counts inside the tile)
+// and scatters.
 // (Six launches before: marks, flags, three of a 3n scan, scatter.)
 constexpr int kPartItems = 4;  // 8 / 4 / 2: 303 / 301 / 281 us (36k spheres), 2314 / 2303 / 2481 (2.7M triangles)
 constexpr uint32_t kPartRun = 32 * kPartItems;               // positions per warp
 constexpr uint32_t kPartTile = kPartRun * (kThreads / 32);  // positions per block
+// Up to here every block of k_partition adds up its list's earlier tiles
+// itself, above a prefix sum of the counts (three launches) does, or the reads
+// grow with the square of the primitives.  Rebuild with sums in the blocks /
+// with the prefix sum: 2.7M spheres 2765 / 2922 us, 8M 8851 / 8946, 14M 18539 /
+// 18470, 30M 48520 / 47380, 60M 114960 / 105740.
+constexpr uint32_t kPartSelf = 8192;  // tiles
 
 __global__ void __launch_bounds__(kThreads) k_part_count(Segs g, const int32_t* __restrict__ seg_id,
                                                          const uint32_t* __restrict__ lists, uint32_t n,
@@ -355,6 +362,7 @@ __global__ void __launch_bounds__(kThreads) k_partition(Segs g, const int32_t* _
                                                         const uint32_t* __restrict__ in, uint32_t n, uint32_t tiles,
                                                         const uint32_t* __restrict__ sides,
                                                         const uint32_t* __restrict__ counts,
+                                                        const uint32_t* __restrict__ offs,
                                                         uint32_t* __restrict__ out, int32_t* __restrict__ next_seg) {
   __shared__ uint32_t wsum[kThreads / 32], wleft[kThreads / 32];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
@@ -367,7 +375,11 @@ __global__ void __launch_bounds__(kThreads) k_partition(Segs g, const int32_t* _
     side[j] = w < words ? __ldg(sides + (size_t)a * words + w) : 0u;
     mine += __popc(side[j]);
   }
-  for (uint32_t t = threadIdx.x; t < tile; t += kThreads) before += __ldg(counts + a * tiles + t);
+  if (offs) {  // the counts' prefix sum over all three lists
+    if (threadIdx.x == 0) before = __ldg(offs + blockIdx.x) - __ldg(offs + a * tiles);
+  } else {
+    for (uint32_t t = threadIdx.x; t < tile; t += kThreads) before += __ldg(counts + a * tiles + t);
+  }
   before = __reduce_add_sync(0xffffffffu, before);
   if (lane == 0) {
     wsum[warp] = before;
@@ -712,7 +724,8 @@ BuildResult build_median_bvh(const SceneView& s, AccelBuffers& a, BuildScratch& 
   MB_TRY(sc.m0.ensure((size_t)n * 9 * 4), "BVH scratch");              // aabb (6) + centroid (3)
   MB_TRY(sc.m1.ensure((size_t)n * 6 * 4), "BVH scratch");              // lists, double buffered
   MB_TRY(sc.m2.ensure((size_t)n * 3 * 4), "BVH scratch");              // sort keys
-  MB_TRY(sc.m3.ensure(((size_t)((n + 31) / 32) * 3 + 3 * (size_t)tiles) * 4), "BVH scratch");  // sides, tile counts
+  const uint64_t cells = 3 * (uint64_t)tiles;
+  MB_TRY(sc.m3.ensure(((size_t)((n + 31) / 32) * 3 + 2 * cells + scan_tmp_words(cells) + 8) * 4), "BVH scratch");  // sides, tile counts and their prefix
   MB_TRY(sc.m4.ensure((size_t)n * 8), "BVH scratch");                  // segment of every position, double buffered
   MB_TRY(sc.m5.ensure((size_t)cap * kSegWords * 4), "BVH scratch");    // segments, this level
   MB_TRY(sc.m6.ensure((size_t)cap * kSegWords * 4), "BVH scratch");    // segments, next level
@@ -724,6 +737,8 @@ BuildResult build_median_bvh(const SceneView& s, AccelBuffers& a, BuildScratch& 
   uint32_t* keys = sc.m2.as<uint32_t>();
   uint32_t* sides = sc.m3.as<uint32_t>();
   uint32_t* tile_counts = sides + 3 * (size_t)((n + 31) / 32);
+  uint32_t* tile_offs = tiles > kPartSelf ? tile_counts + cells : nullptr;
+  uint32_t* tile_tmp = tile_counts + 2 * cells;
   int32_t* seg_id = sc.m4.as<int32_t>();
   int32_t* next_seg = seg_id + n;
   Segs cur = segs_at(sc.m5.as<uint32_t>(), cap), nxt = segs_at(sc.m6.as<uint32_t>(), cap);
@@ -753,7 +768,9 @@ BuildResult build_median_bvh(const SceneView& s, AccelBuffers& a, BuildScratch& 
     k_seg_level<<<1, S < 1024u ? (S + 31) / 32 * 32 : 1024u, 0, st>>>(cur, ctl, level, lists, n, cen, nxt,
                                                                       a.nodes.as<float4>(), a.root.as<float>());
     k_part_count<<<3 * tiles, kThreads, 0, st>>>(cur, seg_id, lists, n, tiles, cen, sides, tile_counts);
-    k_partition<<<3 * tiles, kThreads, 0, st>>>(cur, seg_id, lists, n, tiles, sides, tile_counts, lists_alt, next_seg);
+    if (tile_offs) launch_scan_excl(tile_counts, tile_offs, cells, tile_tmp, tile_tmp + scan_tmp_words(cells) + 4, st);
+    k_partition<<<3 * tiles, kThreads, 0, st>>>(cur, seg_id, lists, n, tiles, sides, tile_counts, tile_offs, lists_alt,
+                                                next_seg);
     MB_TRY(cudaGetLastError(), "BVH level");
     std::swap(lists, lists_alt);
     std::swap(seg_id, next_seg);
@@ -773,7 +790,7 @@ BuildResult build_median_bvh(const SceneView& s, AccelBuffers& a, BuildScratch& 
              "BVH finish");
       attr_set.fetch_or(bit);
     }
-    const uint64_t cells = (uint64_t)kFinishDepth * S;
+    const uint64_t cells = (uint64_t)kFinishDepth * S;  // levels x subtrees
     MB_TRY(sc.keys.ensure((2 * cells + scan_tmp_words(cells) + 8) * 4), "BVH scratch");
     uint32_t* counts = sc.keys.as<uint32_t>();
     uint32_t* offs = counts + cells;
