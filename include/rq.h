@@ -378,7 +378,8 @@ typedef struct rq_query_t {
  * work already queued on the context's stream such as a rebuild.  Put the
  * query with the longest traversal first.  Results equal
  * rq_trace_closest / rq_trace_any per query; returns when every result is in
- * host memory.  Device memory: four slots of a chunk's rays and results, and
+ * host memory.  Device memory: four slots of the largest chunk's rays and results
+ * (at most 2M rays, at most half of a query that is first or last), and
  * for each query that uploads whole a buffer of its rays and results
  * (grow-only, per context). */
 rq_status_t rq_trace_queries(rq_ctx_t ctx, rq_accel_t accel, const rq_query_t* queries, uint32_t n_queries);

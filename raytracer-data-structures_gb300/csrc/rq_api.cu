@@ -688,6 +688,18 @@ static bool streams(const rq_settings_t& cfg, const void* rays, const void* out,
   return n >= kPipeMin && cfg.ray_sort == RQ_RAY_SORT_NONE && pinned(rays) && pinned(out);
 }
 
+// The slots of a call's streamed queries: as large as the largest chunk of them
+// (grown while nothing of the call is queued yet, so no slot moves under it).
+static rq_status_t ensure_slots(rq_ctx_t ctx, const std::vector<uint32_t>& plan, bool any) {
+  size_t rays = 0;
+  for (uint32_t m : plan) rays = std::max<size_t>(rays, m);
+  for (int k = 0; k < kPipeSlots; ++k) {
+    RQ_TRY_CUDA(ctx, ctx->pipe.rays[k].ensure(rays * 32));
+    RQ_TRY_CUDA(ctx, ctx->pipe.out[k].ensure(any ? (rays + 31) / 32 * 4 : rays * 16));
+  }
+  return RQ_SUCCESS;
+}
+
 // Streamed query over host buffers: per chunk, upload on pipe.up, trace on
 // the context's stream, download on pipe.down, with kPipeSlots device slots
 // in rotation (a slot is re-filled only after its previous download).
@@ -696,11 +708,8 @@ static rq_status_t trace_streamed_enqueue(rq_ctx_t ctx, rq_accel_t a, const rq_r
                                           bool begins = true, bool ends = true) {
   HostPipe& p = ctx->pipe;
   RQ_TRY_CUDA(ctx, p.init());
-  const size_t out_chunk = any ? kPipeChunk / 8 : (size_t)kPipeChunk * 16;
-  for (int k = 0; k < kPipeSlots; ++k) {
-    RQ_TRY_CUDA(ctx, p.rays[k].ensure((size_t)kPipeChunk * 32));
-    RQ_TRY_CUDA(ctx, p.out[k].ensure(out_chunk));
-  }
+  const std::vector<uint32_t> plan = chunk_plan(n, begins, ends);
+  RQ_TRY(ensure_slots(ctx, plan, any));
   // Traversals start after everything already queued on the context's
   // stream (a rebuild, say); uploads start at once, overlapping that work,
   // each after only the previous use of its slot (events never recorded are
@@ -709,7 +718,6 @@ static rq_status_t trace_streamed_enqueue(rq_ctx_t ctx, rq_accel_t a, const rq_r
   RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.down, p.start, 0));
   RQ_TRY_CUDA(ctx, cudaStreamWaitEvent(p.lane2, p.start, 0));
   const SceneView sv = scene_view(a->scene);
-  const std::vector<uint32_t> plan = chunk_plan(n, begins, ends);
   uint64_t first = 0;
   for (uint32_t c = 0; c < (uint32_t)plan.size(); first += plan[c], ++c) {
     const int sl = (int)(p.next++ % kPipeSlots);
@@ -902,7 +910,7 @@ static rq_status_t trace_queries_enqueue(rq_ctx_t ctx, rq_accel_t a, const rq_qu
     const rq_query_t& q = qs[k];
     if (q.n == 0) continue;
     if (!whole[k]) {
-      for (DevBuf& b : p.out) RQ_TRY_CUDA(ctx, b.ensure((size_t)kPipeChunk * (q.any ? 1 : 128) / 8));
+      RQ_TRY(ensure_slots(ctx, chunk_plan(q.n, k == 0, k + 1 == nq), q.any != 0));
       continue;
     }
     const size_t out_bytes = q.any ? (size_t)((q.n + 31) / 32) * 4 : (size_t)q.n * 16;
