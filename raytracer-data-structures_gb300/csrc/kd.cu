@@ -96,7 +96,7 @@ struct EdgeLists {
 // bounded, and a tile that gives up marks itself so later tiles do too.
 constexpr unsigned long long kTileAgg = 1ull << 62, kTilePrefix = 2ull << 62, kTileAbort = 3ull << 62;
 constexpr unsigned long long kTileValue = (1ull << 62) - 1;
-constexpr uint32_t kTilePolls = 1u << 20;
+constexpr uint32_t kTilePolls = 1u << 20;  // polls of the same 32 tiles before giving up
 
 __device__ __forceinline__ unsigned long long tile_load(const unsigned long long* p) {
   unsigned long long v;
@@ -166,6 +166,7 @@ __device__ __forceinline__ unsigned long long grid_prefix(unsigned long long v, 
           break;
         }
         j -= 32;
+        polls = 0;  // the limit is for the same 32 tiles
       }
     }
     if (lane == 0) {

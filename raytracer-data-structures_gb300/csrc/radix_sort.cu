@@ -31,7 +31,7 @@ constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagPrefix = 2u << 30;
 constexpr uint32_t kFlagAbort = 3u << 30;
 constexpr uint32_t kValueMask = (1u << 30) - 1;
-constexpr uint32_t kSpinLimit = 1u << 20;  // polls of one predecessor word before giving up
+constexpr uint32_t kSpinLimit = 1u << 20;  // polls of the same eight predecessors' words before giving up
 constexpr int kThreads32 = 512, kItems32 = 8;      // 32-bit keys: tiles of 4,096
 constexpr int kThreadsSmall = 256, kItemsSmall = 8;  // short 32-bit sorts: tiles of 2,048
 constexpr int kThreads64 = 512, kItems64 = 6;      // 64-bit keys: tiles of 3,072
@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(T) k_onesweep(const K* __restrict__ kin, const
         excl += sum;
         if (stop) break;
         j -= kWin;
+        polls = 0;  // the limit is for one window's words
       }
       if (failed) {
         store_status(st + (size_t)tile * 256, kFlagAbort);
