@@ -101,7 +101,17 @@ __global__ void __launch_bounds__(kThreads, UNIT ? kWalkBlocks : kWalkBlocksWide
     }
     const bool own = walk;  // this lane's ray is walked here
     Closest c = {ray.tmax, kMiss, 0.f, 0.f};
-    const bool occluded = walk_warp<KIND, ANY, UNIT, kStackSize, false, false>(bvh, ray, sr, walk, false, again != 0u || bvh.loose, c, sh, err);
+    bool occluded = false;
+    // closest hits on spheres keep their lanes, and rounds only cost them (2M random
+    // rays on a median BVH 111 us in rounds, 105 without, camera rays 86 and 81)
+    if constexpr (!ANY && KIND == kSpheres) {
+      uint32_t visits = 0, tests = 0;
+      if (walk) walk_bvh2_form<KIND, ANY, false, kStackSize, false, UNIT>(bvh, ray, sr, c, visits, tests, err);
+      __syncwarp();
+    } else {
+      occluded = walk_warp<KIND, ANY, UNIT, kStackSize, false, false>(bvh, ray, sr, walk, false, again != 0u || bvh.loose,
+                                                                      c, sh, err);
+    }
     const uint32_t r = (perm && live) ? __ldg(perm + i) : i;
     if (!ANY) {
       if (own) store_hit(hits, r, c);

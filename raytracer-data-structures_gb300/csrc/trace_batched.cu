@@ -2,8 +2,8 @@
 //
 // Rays of all structures lie back to back; ray_off (n_views + 1 entries)
 // gives each structure's range.  The grid is sized to what the SMs hold at
-// once; each warp takes 32 consecutive rays at a time from a global counter
-// until none are left, so long and short structures, coherent and incoherent
+// once; each warp takes 32 consecutive rays (spheres: 64) at a time from a
+// global counter until none are left, so long and short structures, coherent and incoherent
 // rays share the GPU without a tail per structure.  Each ray finds its
 // structure by binary search over ray_off and walks it with the same FAST
 // walk as a one-structure query (identical results; the binary walk shares
@@ -11,7 +11,9 @@
 // structures).  64 scenes, 8M random rays: closest hit 2798 us with one lane a
 // ray, 2230 now, any hit 2271 and 1870 (256 rays per counter access were 9 and
 // 6% slower than 32, 64: 6 and 1%); 7 / 8 / 9 blocks of 128 per SM 2327 / 2230 /
-// 2359 (closest hit: 9 spill), 1872 at 8 and 1870 at 9 (any hit).
+// 2359 (closest hit: 9 spill), 1872 at 8 and 1870 at 9 (any hit).  32 scenes of
+// 5k spheres, 3.2M random rays, whose walks are short: 32 / 64 / 128 / 256 rays
+// a turn 127 / 115 / 116 / 119 us, any hit 118 / 102 / 107 / 109.
 //
 // Launch shapes (block size, traversal stack depth) are template choices that
 // rq_plan_create times on the caller's rays; a stack too shallow for a tree
@@ -32,11 +34,19 @@ __global__ void __launch_bounds__(BLOCK, W == 2 ? (ANY ? 1152 : 1024) / BLOCK : 
                                                          const uint32_t* __restrict__ perm, bool loose) {
   __shared__ WarpShare<ANY, true, UNIT> share[W == 2 ? BLOCK / 32 : 1];
   const uint32_t lane = threadIdx.x & 31;
-  uint32_t base = 0, again = 0;  // again: closest hits in doubt, walked once more without sharing
+  constexpr uint32_t kGrab = KIND == kSpheres ? 64u : 32u;  // rays a warp takes at a time
+  uint32_t base = 0, taken = kGrab;                         // taken: how many of them it has begun
+  uint32_t again = 0;  // closest hits in doubt, walked once more without sharing
   for (;;) {
     if (ANY || again == 0u) {
-      if (lane == 0) base = atomicAdd(work, 32u);
-      base = __shfl_sync(0xffffffffu, base, 0);
+      if (taken == kGrab) {
+        if (lane == 0) base = atomicAdd(work, kGrab);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        taken = 32u;
+      } else {
+        base += 32u;
+        taken += 32u;
+      }
     }
     if (base >= n) return;  // the whole warp leaves together
     const uint32_t w = base + lane;  // work index; the ray itself through perm
@@ -64,8 +74,14 @@ __global__ void __launch_bounds__(BLOCK, W == 2 ? (ANY ? 1152 : 1024) / BLOCK : 
       }
       __syncwarp();
       const bool own = walk;
-      occluded = walk_warp<KIND, ANY, UNIT, STACK, true, true>(v, ray, sr, walk, false, again != 0u || loose, c,
-                                                               share[threadIdx.x >> 5], err);
+      if constexpr (!ANY && KIND == kSpheres) {  // their lanes are their own, and rounds only cost them
+        uint32_t visits = 0, tests = 0;
+        if (walk) walk_bvh2_form<KIND, ANY, false, STACK, false, UNIT>(v, ray, sr, c, visits, tests, err);
+        __syncwarp();
+      } else {
+        occluded = walk_warp<KIND, ANY, UNIT, STACK, true, true>(v, ray, sr, walk, false, again != 0u || loose, c,
+                                                                 share[threadIdx.x >> 5], err);
+      }
       if (!ANY && own) store_hit(hits, r, c);
       if (!ANY) again = __ballot_sync(0xffffffffu, own && occluded);
       occluded = occluded || exact_hit;
