@@ -1023,6 +1023,11 @@ __global__ void __launch_bounds__(128) k_trace_kd_warps(KdView kd, uint32_t n_no
 // rays 194 / 60 / 42, 300k random rays 377 / 279 / 237 (any hit 347 / 209 /
 // 162), 307k camera rays 260 / 215 / 174, their shadow rays 348 / 257 / 212, 2M
 // bounce rays 2020 / 1950 / 1400, 2M coherent shadow rays 697 / 778 / 674.
+// Coherent rays by the million lose on small trees, the more the smaller: 3M
+// parallel rays 86 -> 166 on 12 triangles, 180 -> 210 on 3,468, 966 -> 1028 on
+// 998k (one lane a ray / now); random rays on the same trees gain from 48
+// triangles on (296 -> 241, 701 -> 510, 1958 -> 1358), and no size tells the two
+// apart.
 constexpr int kKdChunk = 4;  // 2 / 3 / 4 / 5 / 8 / 16, 2M bounce rays: 1681 / 1569 / 1527 / 1518 / 1565 / 1733 us; 300k shadow rays: 176 / 174 / 172 / 175 / 186 / 212
 constexpr uint32_t kKdLeafMax = 1u << 26;  // primitives of a leaf tested at one meeting (32 lanes' fit 32 bits)
 constexpr int kKdIdle = 8;   // lanes idle before pieces move; 5 / 8 / 12: within 1%

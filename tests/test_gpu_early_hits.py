@@ -83,3 +83,17 @@ def test_imported_boxes_that_do_not_hold_their_primitives(engine, oracle, rqm):
     plain = engine.build(scene, rqm.LBVH)
     offs = np.array([0, len(rays), len(rays) + 900])
     assert np.array_equal(_u32(engine.trace_batched([acc, plain], np.concatenate([rays, rays[:900]]), offs))[:len(rays)], want)
+
+
+def test_early_hits_kd(engine, oracle, rqm):
+    v, f, rays = early_hits.scene_and_rays(1500, 1)
+    prims, _, _ = oracle.tri_prims(v, f)
+    acc = engine.build(engine.scene_triangles(v, f), rqm.KDTREE)
+    nodes, pidx, root, _ = engine.export_kd(acc)
+    want = _u32(oracle.trace_kd(oracle.TRIANGLES, oracle.FAST, oracle.CLOSEST, oracle.Kd(nodes, pidx, root), prims, rays))
+    for k in range(20):
+        assert np.array_equal(_u32(engine.trace_closest(acc, rays[k:k + 1])), want[k:k + 1])
+    rng = np.random.default_rng(2)
+    for n in (33, 700, 1500, 40_000, 300_003):
+        pick = rng.integers(0, len(rays), n)
+        assert np.array_equal(_u32(engine.trace_closest(acc, rays[pick])), want[pick]), n
