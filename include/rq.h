@@ -85,9 +85,9 @@ typedef struct rq_settings_t {
 } rq_settings_t;
 
 /* How FAST queries on binary BVH structures map rays to GPU threads.  Speed
- * only: every ray walks the same nodes in the same order either way. */
+ * only: hits and occlusion bits are those of one lane walking the ray alone. */
 typedef enum rq_scheduling_t {
-  RQ_SCHEDULING_THREAD_PER_RAY = 0, /* each thread walks one ray at a time; warps take 32 rays at a time from a counter */
+  RQ_SCHEDULING_THREAD_PER_RAY = 0, /* a lane starts with one ray; idle lanes take over parts of their warp's other rays */
   RQ_SCHEDULING_LANE_REFILL = 1,    /* persistent warps refill finished lanes with new rays */
   RQ_SCHEDULING_SPECULATIVE = 2,    /* while-while walk that postpones leaves until the warp has one each */
   RQ_SCHEDULING_WARP_PACKET = 3,    /* the warp walks one shared stack (lane masks per entry): coherent rays */
@@ -126,7 +126,11 @@ typedef enum rq_lbvh_quality_t {
 
 /* Ray reordering before FAST BVH2 traversal of batches of at least 65,536
  * rays.  Results are written in the caller's order either way and do not
- * change; only the speed does. */
+ * change; only the speed does.  An order pays for rays in no order on large
+ * meshes (shuffled bounce rays on a 10M-triangle terrain: 10.0 ms unordered, 9.3
+ * by octant, 5.5 by octant and origin); rays that come in order of their origin,
+ * as a renderer's do, are faster without one (8.3M bounce rays: 2.59 ms, 2.67 by
+ * octant). */
 typedef enum rq_ray_sort_t {
   RQ_RAY_SORT_NONE = 0,
   RQ_RAY_SORT_OCTANT_MORTON = 1,    /* direction octant, then 27-bit Morton code of the origin */
@@ -142,9 +146,12 @@ typedef enum rq_traversal_t {
   /* Reciprocal-direction slab test clipped to [tmin, closest hit], widened by
    * 1 + 2*gamma(3) so no box is lost to rounding; near child first; hits
    * limited to (tmin, tmax).  BVH and brute-force closest hit is the smallest
-   * t and, among primitives hit at exactly that t, the smallest primitive id:
-   * a result independent of the order of the walk (node width, scheduling,
-   * ray reordering). */
+   * t and, among primitives hit at exactly that t, the smallest primitive id,
+   * so that the result does not depend on the order of the walk, with one
+   * exception: a hit whose computed t lies before the primitive's own box (a
+   * long triangle seen edge-on) is taken or not by what the walk found before.
+   * Even that is one answer per structure and node width, whatever the batch,
+   * the scheduling or a ray order. */
   RQ_TRAVERSAL_FAST = 0,
   /* The reference's semantics: division slab test with no clipping
    * (accelerators.h:588-626), boxIntersect's pre-order candidate walk
