@@ -85,7 +85,8 @@ typedef struct rq_settings_t {
 } rq_settings_t;
 
 /* How FAST queries on binary BVH structures map rays to GPU threads.  Speed
- * only: hits and occlusion bits are those of one lane walking the ray alone. */
+ * only: hits and occlusion bits do not change (for hits before their own box see
+ * RQ_TRAVERSAL_FAST). */
 typedef enum rq_scheduling_t {
   RQ_SCHEDULING_THREAD_PER_RAY = 0, /* a lane starts with one ray; idle lanes take over parts of their warp's other rays */
   RQ_SCHEDULING_LANE_REFILL = 1,    /* persistent warps refill finished lanes with new rays */
@@ -150,8 +151,9 @@ typedef enum rq_traversal_t {
    * so that the result does not depend on the order of the walk, with one
    * exception: a hit whose computed t lies before the primitive's own box (a
    * long triangle seen edge-on) is taken or not by what the walk found before.
-   * Even that is one answer per structure and node width, whatever the batch,
-   * the scheduling or a ray order. */
+   * Even that is one answer per structure and node width, whatever the batch or
+   * a ray order, except in SPECULATIVE and WARP_PACKET scheduling, where a ray's
+   * walk waits for its warp's. */
   RQ_TRAVERSAL_FAST = 0,
   /* The reference's semantics: division slab test with no clipping
    * (accelerators.h:588-626), boxIntersect's pre-order candidate walk
